@@ -496,18 +496,23 @@ int DevGeom::upload(const RadB200Geom *G, bool tensor_coeffs, bool mesh)
   RB_TRY(bkg.upload(G->bkg, (size_t)G->n_bkg * 3 * sizeof(double)));
   // unit table: one entry per (source, image); cuboids, polyhedra, arcs, backgrounds
   std::vector<int4> u;
+  std::vector<char> diag(G->n_trf);
+  for (int t = 0; t < G->n_trf; t++) {
+    const double *T = G->trf + (size_t)t * RADB200_TRF_STRIDE;
+    diag[t] = T[1] == 0.0 && T[2] == 0.0 && T[3] == 0.0 && T[5] == 0.0 && T[6] == 0.0 && T[7] == 0.0;
+  }
   ustart[0] = 0;
   for (int i = 0; i < G->n_rec; i++)
-    for (int t = 0; t < G->rec_img[2 * i + 1]; t++) u.push_back(make_int4(0, i, G->rec_img[2 * i] + t, 0));
+    for (int t = 0; t < G->rec_img[2 * i + 1]; t++) u.push_back(make_int4(0, i, G->rec_img[2 * i] + t, diag[G->rec_img[2 * i] + t]));
   ustart[1] = (int)u.size();
   for (int i = 0; i < G->n_poly; i++)
-    for (int t = 0; t < G->poly_info[4 * i + 3]; t++) u.push_back(make_int4(1, i, G->poly_info[4 * i + 2] + t, 0));
+    for (int t = 0; t < G->poly_info[4 * i + 3]; t++) u.push_back(make_int4(1, i, G->poly_info[4 * i + 2] + t, diag[G->poly_info[4 * i + 2] + t]));
   ustart[2] = (int)u.size();
   for (int i = 0; i < G->n_arc; i++)
-    for (int t = 0; t < G->arc_img[2 * i + 1]; t++) u.push_back(make_int4(2, i, G->arc_img[2 * i] + t, 0));
+    for (int t = 0; t < G->arc_img[2 * i + 1]; t++) u.push_back(make_int4(2, i, G->arc_img[2 * i] + t, diag[G->arc_img[2 * i] + t]));
   ustart[3] = (int)u.size();
   for (int i = 0; i < G->n_bkg; i++)
-    for (int t = 0; t < G->bkg_img[2 * i + 1]; t++) u.push_back(make_int4(3, i, G->bkg_img[2 * i] + t, 0));
+    for (int t = 0; t < G->bkg_img[2 * i + 1]; t++) u.push_back(make_int4(3, i, G->bkg_img[2 * i] + t, diag[G->bkg_img[2 * i] + t]));
   ustart[4] = (int)u.size();
   n_units = (int)u.size();
   RB_TRY(units.upload(u.data(), u.size() * sizeof(int4)));

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "elem64.cuh"
+
 namespace rb {
 
 template <typename T> struct V3 { T x, y, z; };
@@ -59,78 +61,163 @@ template <typename T> __device__ __forceinline__ T atan4(T a, T b, T c, T d)
   return atanT(w) + Pi * (p1 + p2 + p3);
 }
 
-// Cuboid: q = observation point RELATIVE TO THE CUBOID CENTRE (object frame),
-// hd = half dimensions.  Returns 1 if strictly inside.  Writes the symmetric
-// tensor entries T = (Txx,Tyy,Tzz) and S = (Sx,Sy,Sz) scaled by 1/(4 pi):
-//   Q = [[Tx,-Sz,-Sy],[-Sz,Ty,-Sx],[-Sy,-Sx,Tz]]    (radrec.cpp:265-283)
-template <typename T>
-__device__ __forceinline__ int cuboid_TS(V3<double> q, V3<double> hd, const Guard &g, V3<T> &Tt, V3<T> &Ss)
+// ---- cuboid -------------------------------------------------------------------
+// Q of a uniformly magnetized cuboid (radrec.cpp:115-283) at q from its centre:
+//   4 pi Tx = sum of 8 arctan(+-y_j z_k / (x_i D_ijk)),
+//   4 pi Sz = -log of a product of 8 factors (z_k + D_ijk)^+-1,  and cyclic.
+// Evaluated term by term as the reference does, a pair costs 24 quotients
+// inside the arctangents, 18 in their addition formulas, 12 in the logarithms,
+// and 6 arctangents: about 2,000 FP64 issue slots.  Here:
+//   - each arctangent is the argument of x D + i (+-y z); the arguments of a
+//     face add up in the product of its four numbers, both faces of an axis in
+//     one more product, so an axis costs no quotients and one arctangent.  The
+//     product knows its angle modulo 2 pi.  The turns come from the quadrants
+//     of the two face products: seen from the point a face has a solid angle
+//     in (0, pi), or in (0, 2 pi) when the point projects into it (then all
+//     four arguments are positive and the product's quadrant cannot be
+//     mistaken by rounding).  Quadrant centres are within pi/4 of the angles,
+//     two faces and their product within 3 pi/4 of a multiple of 2 pi;
+//   - z + D with z < 0 cancels; there it is rho^2 / (|z| + D), rho^2 =
+//     x^2 + y^2.  For z_0 and z_1 of one sign the rho^2 cancel between the two
+//     ends and only the logarithm's sign changes; otherwise they stay as a
+//     factor.  No quotient, no cancellation, one logarithm of a ratio per axis.
+//   - the third diagonal entry is what the trace leaves: 0 outside, -1 inside.
+// elem64.cuh has the square root, arctangent and logarithm.
+
+// one axis: T of the faces at a0 and a1 (offsets along the axis), p_jk the
+// products of the other two offsets, D_jk the distances of the corners;
+// inner: the point projects into the faces
+RB_HD double cuboid_axis_T(double a0, double a1, double p00, double p01, double p10, double p11, double D000,
+                           double D001, double D010, double D011, double D100, double D101, double D110, double D111,
+                           bool inner)
 {
-  // corner offsets in FP64 (exact zeros and guards decided before any rounding to T)
-  double dx0 = -q.x - hd.x, dx1 = -q.x + hd.x;
-  double dy0 = -q.y - hd.y, dy1 = -q.y + hd.y;
-  double dz0 = -q.z - hd.z, dz1 = -q.z + hd.z;
-  if (dx0 == 0.0) dx0 = abs_rand(g, hd.x);
-  if (dx1 == 0.0) dx1 = abs_rand(g, hd.x);
-  if (dy0 == 0.0) dy0 = abs_rand(g, hd.y);
-  if (dy1 == 0.0) dy1 = abs_rand(g, hd.y);
-  if (dz0 == 0.0) dz0 = abs_rand(g, hd.z);
-  if (dz1 == 0.0) dz1 = abs_rand(g, hd.z);
-  T x0 = T(dx0), x1 = T(dx1), y0 = T(dy0), y1 = T(dy1), z0 = T(dz0), z1 = T(dz1);
-  int inside = (x0 * x1 < T(0)) && (y0 * y1 < T(0)) && (z0 * z1 < T(0));
-  T x0e2 = x0 * x0, x1e2 = x1 * x1, y0e2 = y0 * y0, y1e2 = y1 * y1, z0e2 = z0 * z0, z1e2 = z1 * z1;
-  T D000 = sqrtT(x0e2 + y0e2 + z0e2), D100 = sqrtT(x1e2 + y0e2 + z0e2);
-  T D010 = sqrtT(x0e2 + y1e2 + z0e2), D110 = sqrtT(x1e2 + y1e2 + z0e2);
-  T D001 = sqrtT(x0e2 + y0e2 + z1e2), D101 = sqrtT(x1e2 + y0e2 + z1e2);
-  T D011 = sqrtT(x0e2 + y1e2 + z1e2), D111 = sqrtT(x1e2 + y1e2 + z1e2);
+  const double u = p00 * p01, v = p10 * p11;
+  const double r0 = a0 * D000, r1 = a0 * D001, r2 = a0 * D010, r3 = a0 * D011;
+  const double e0 = fma(r0, r1, u), f0 = fma(p00, r1, -(r0 * p01));
+  const double e1 = fma(r2, r3, v), f1 = fma(r2, p11, -(p10 * r3));
+  const double re0 = fma(e0, e1, -(f0 * f1)), im0 = fma(e0, f1, f0 * e1);
+  const double t0 = a1 * D100, t1 = a1 * D101, t2 = a1 * D110, t3 = a1 * D111;
+  const double g0 = fma(t0, t1, u), h0 = fma(p00, t1, -(t0 * p01));
+  const double g1 = fma(t2, t3, v), h1 = fma(t2, p11, -(p10 * t3));
+  const double re1 = fma(g0, g1, -(h0 * h1)), im1 = fma(g0, h1, h0 * g1);
+  const double re = fma(re0, re1, im0 * im1), im = fma(im0, re1, -(re0 * im1));
+  // quadrant centres in units of pi/4; s: sign of the offset, which the products carry
+  const int s0 = hi32(a0), s1 = hi32(a1);
+  const int last = inner ? 7 : -1;
+  const int c0 = hi32(re0) < 0 ? ((hi32(im0) ^ s0) < 0 ? 5 : 3) : ((hi32(im0) ^ s0) < 0 ? last : 1);
+  const int c1 = hi32(re1) < 0 ? ((hi32(im1) ^ s1) < 0 ? 5 : 3) : ((hi32(im1) ^ s1) < 0 ? last : 1);
+  const int c = hi32(re) < 0 ? (hi32(im) < 0 ? -3 : 3) : (hi32(im) < 0 ? -1 : 1);
+  const int turns = ((s0 < 0 ? -c0 : c0) - (s1 < 0 ? -c1 : c1) - c + 4) >> 3;
+  return angle64(im, re, turns);
+}
 
-  T T0x = atan4(y0 * z0 / (x0 * D000), -y0 * z1 / (x0 * D001), -y1 * z0 / (x0 * D010), y1 * z1 / (x0 * D011));
-  T T1x = atan4(-y0 * z0 / (x1 * D100), y0 * z1 / (x1 * D101), y1 * z0 / (x1 * D110), -y1 * z1 / (x1 * D111));
-  T T0y = atan4(x0 * z0 / (y0 * D000), -x0 * z1 / (y0 * D001), -x1 * z0 / (y0 * D100), x1 * z1 / (y0 * D101));
-  T T1y = atan4(-x0 * z0 / (y1 * D010), x0 * z1 / (y1 * D011), x1 * z0 / (y1 * D110), -x1 * z1 / (y1 * D111));
-  T T0z = atan4(x0 * y0 / (z0 * D000), -x1 * y0 / (z0 * D100), -x0 * y1 / (z0 * D010), x1 * y1 / (z0 * D110));
-  T T1z = atan4(-x0 * y0 / (z1 * D001), x1 * y0 / (z1 * D101), x0 * y1 / (z1 * D011), -x1 * y1 / (z1 * D111));
+// one axis: the logarithm of S.  b_ijk = |a_k| + D of the corners, the axis's
+// own index last; n2, d2 the rho^2 products that replace the cancelling sums
+// when the two offsets have opposite signs (mixed); neg: the first one is negative
+RB_HD double cuboid_axis_L(double b000, double b001, double b010, double b011, double b100, double b101, double b110,
+                           double b111, double n2, double d2, bool mixed, bool neg)
+{
+  const double e = b001 * b111, f = b101 * b011, g = b100 * b010, h = b000 * b110;
+  const double n = mixed ? (e * h) * n2 : e * g, d = mixed ? (f * g) * d2 : f * h;
+  const double L = log_ratio64(n, d);
+  return neg && !mixed ? -L : L;
+}
 
-  T R000 = T(10) * abs_rand(g, D000), R010 = T(10) * abs_rand(g, D010);
-  T R001 = T(10) * abs_rand(g, D001), R011 = T(10) * abs_rand(g, D011);
-  T R100 = T(10) * abs_rand(g, D100), R110 = T(10) * abs_rand(g, D110);
-  T R101 = T(10) * abs_rand(g, D101), R111 = T(10) * abs_rand(g, D111);
-  const T h = T(0.5);
-  T z0pD100 = z0 + D100; if (z0pD100 < R100) z0pD100 = h * (x1e2 + y0e2) / fabsT(z0);
-  T z1pD101 = z1 + D101; if (z1pD101 < R101) z1pD101 = h * (x1e2 + y0e2) / fabsT(z1);
-  T z1pD001 = z1 + D001; if (z1pD001 < R001) z1pD001 = h * (x0e2 + y0e2) / fabsT(z1);
-  T z0pD000 = z0 + D000; if (z0pD000 < R000) z0pD000 = h * (x0e2 + y0e2) / fabsT(z0);
-  T z0pD010 = z0 + D010; if (z0pD010 < R010) z0pD010 = h * (x0e2 + y1e2) / fabsT(z0);
-  T z1pD011 = z1 + D011; if (z1pD011 < R011) z1pD011 = h * (x0e2 + y1e2) / fabsT(z1);
-  T z1pD111 = z1 + D111; if (z1pD111 < R111) z1pD111 = h * (x1e2 + y1e2) / fabsT(z1);
-  T z0pD110 = z0 + D110; if (z0pD110 < R110) z0pD110 = h * (x1e2 + y1e2) / fabsT(z0);
+// Replacement near a corner with the length guards on (radrec.cpp:131-156):
+// z + D below 10 times the guard of D becomes rho^2 / (2 |z|).  b = |z| + D.
+__device__ __forceinline__ double cuboid_guard_b(const Guard &g, double z, double D, double rho2)
+{
+  const double b = fabs(z) + D, R = 10.0 * abs_rand(g, D);
+  if (z < 0.0) return rho2 < R * b ? 2.0 * fabs(z) : b;
+  return b < R ? 0.5 * rho2 / fabs(z) : b;
+}
 
-  T y0pD100 = y0 + D100; if (y0pD100 < R100) y0pD100 = h * (x1e2 + z0e2) / fabsT(y0);
-  T y1pD110 = y1 + D110; if (y1pD110 < R110) y1pD110 = h * (x1e2 + z0e2) / fabsT(y1);
-  T y1pD010 = y1 + D010; if (y1pD010 < R010) y1pD010 = h * (x0e2 + z0e2) / fabsT(y1);
-  T y0pD000 = y0 + D000; if (y0pD000 < R000) y0pD000 = h * (x0e2 + z0e2) / fabsT(y0);
-  T y0pD001 = y0 + D001; if (y0pD001 < R001) y0pD001 = h * (x0e2 + z1e2) / fabsT(y0);
-  T y1pD011 = y1 + D011; if (y1pD011 < R011) y1pD011 = h * (x0e2 + z1e2) / fabsT(y1);
-  T y1pD111 = y1 + D111; if (y1pD111 < R111) y1pD111 = h * (x1e2 + z1e2) / fabsT(y1);
-  T y0pD101 = y0 + D101; if (y0pD101 < R101) y0pD101 = h * (x1e2 + z1e2) / fabsT(y0);
-
-  T x0pD010 = x0 + D010; if (x0pD010 < R010) x0pD010 = h * (y1e2 + z0e2) / fabsT(x0);
-  T x1pD110 = x1 + D110; if (x1pD110 < R110) x1pD110 = h * (y1e2 + z0e2) / fabsT(x1);
-  T x1pD100 = x1 + D100; if (x1pD100 < R100) x1pD100 = h * (y0e2 + z0e2) / fabsT(x1);
-  T x0pD000 = x0 + D000; if (x0pD000 < R000) x0pD000 = h * (y0e2 + z0e2) / fabsT(x0);
-  T x0pD001 = x0 + D001; if (x0pD001 < R001) x0pD001 = h * (y0e2 + z1e2) / fabsT(x0);
-  T x1pD101 = x1 + D101; if (x1pD101 < R101) x1pD101 = h * (y0e2 + z1e2) / fabsT(x1);
-  T x1pD111 = x1 + D111; if (x1pD111 < R111) x1pD111 = h * (y1e2 + z1e2) / fabsT(x1);
-  T x0pD011 = x0 + D011; if (x0pD011 < R011) x0pD011 = h * (y1e2 + z1e2) / fabsT(x0);
-
-  const T C = T(1.0 / (4.0 * 3.141592653589793238));
-  // S = -log(product of 4 ratios)  (radrec.cpp:257-260)
-  T Sx = -logT((x0pD010 / x1pD110) * (x1pD100 / x0pD000) * (x0pD001 / x1pD101) * (x1pD111 / x0pD011));
-  T Sy = -logT((y0pD100 / y1pD110) * (y1pD010 / y0pD000) * (y0pD001 / y1pD011) * (y1pD111 / y0pD101));
-  T Sz = -logT((z0pD100 / z1pD101) * (z1pD001 / z0pD000) * (z0pD010 / z1pD011) * (z1pD111 / z0pD110));
-  Tt = mk3<T>(C * (T0x + T1x), C * (T0y + T1y), C * (T0z + T1z));
-  Ss = mk3<T>(C * Sx, C * Sy, C * Sz);
-  return inside;
+// q = observation point RELATIVE TO THE CUBOID CENTRE (object frame), hd =
+// half dimensions.  Returns 1 if strictly inside.  Writes the symmetric tensor
+// entries T = (Txx,Tyy,Tzz) and S = (Sx,Sy,Sz) times 4 pi (the caller scales
+// by CUBOID_C):
+//   Q = [[Tx,-Sz,-Sy],[-Sz,Ty,-Sx],[-Sy,-Sx,Tz]]    (radrec.cpp:265-283)
+constexpr double CUBOID_C = 1.0 / (4.0 * 3.141592653589793238);
+__device__ __forceinline__ int cuboid_TS(V3<double> q, V3<double> hd, const Guard &g, V3<double> &Tt, V3<double> &Ss)
+{
+  // the signs of the widths, if negative, turn the sign of the whole tensor
+  const int ws = hi32(hd.x) ^ hi32(hd.y) ^ hi32(hd.z);
+  const double hx = fabs(hd.x), hy = fabs(hd.y), hz = fabs(hd.z);
+  double x0 = -q.x - hx, x1 = -q.x + hx;
+  double y0 = -q.y - hy, y1 = -q.y + hy;
+  double z0 = -q.z - hz, z1 = -q.z + hz;
+  // on a face plane the guards step off it; without guards the normal entry
+  // of the tensor is undefined there (0/0 in the reference), NaN
+  int nan = 0;
+  if (x0 == 0.0 || x1 == 0.0) {
+    const double r = abs_rand(g, hx);
+    if (x0 == 0.0) x0 = r;
+    if (x1 == 0.0) x1 = r;
+    nan |= (r == 0.0);
+  }
+  if (y0 == 0.0 || y1 == 0.0) {
+    const double r = abs_rand(g, hy);
+    if (y0 == 0.0) y0 = r;
+    if (y1 == 0.0) y1 = r;
+    nan |= (r == 0.0) << 1;
+  }
+  if (z0 == 0.0 || z1 == 0.0) {
+    const double r = abs_rand(g, hz);
+    if (z0 == 0.0) z0 = r;
+    if (z1 == 0.0) z1 = r;
+    nan |= (r == 0.0) << 2;
+  }
+  // Q has no dimension: bring extreme units (products of 16 lengths occur) to
+  // around 1 by a power of two
+  {
+    const int top = max(max(hi32(fabs(x0)), max(hi32(fabs(x1)), hi32(fabs(y0)))),
+                        max(hi32(fabs(y1)), max(hi32(fabs(z0)), hi32(fabs(z1)))));
+    const int e = (top >> 20) - 1023;
+    if (e > 40 || e < -40) {
+      const double sc = scalbn(1.0, e > 1000 ? -1000 : -e);
+      x0 *= sc; x1 *= sc; y0 *= sc; y1 *= sc; z0 *= sc; z1 *= sc;
+    }
+  }
+  const bool mx = (hi32(x0) & ~hi32(x1)) < 0, my = (hi32(y0) & ~hi32(y1)) < 0, mz = (hi32(z0) & ~hi32(z1)) < 0;
+  const double xx0 = x0 * x0, xx1 = x1 * x1, yy0 = y0 * y0, yy1 = y1 * y1, zz0 = z0 * z0, zz1 = z1 * z1;
+  const double xy00 = xx0 + yy0, xy01 = xx0 + yy1, xy10 = xx1 + yy0, xy11 = xx1 + yy1;
+  const double D000 = sqrt64(xy00 + zz0), D001 = sqrt64(xy00 + zz1), D010 = sqrt64(xy01 + zz0), D011 = sqrt64(xy01 + zz1);
+  const double D100 = sqrt64(xy10 + zz0), D101 = sqrt64(xy10 + zz1), D110 = sqrt64(xy11 + zz0), D111 = sqrt64(xy11 + zz1);
+  Tt.x = cuboid_axis_T(x0, x1, y0 * z0, y0 * z1, y1 * z0, y1 * z1, D000, D001, D010, D011, D100, D101, D110, D111, my && mz);
+  Tt.y = cuboid_axis_T(y0, y1, x0 * z0, x0 * z1, x1 * z0, x1 * z1, D000, D001, D100, D101, D010, D011, D110, D111, mx && mz);
+  const bool in = mx && my && mz;
+  Tt.z = (in ? -4.0 * 3.141592653589793238 : 0.0) - (Tt.x + Tt.y);
+  const double xz00 = xx0 + zz0, xz01 = xx0 + zz1, xz10 = xx1 + zz0, xz11 = xx1 + zz1;
+  const double yz00 = yy0 + zz0, yz01 = yy0 + zz1, yz10 = yy1 + zz0, yz11 = yy1 + zz1;
+  const double ax0 = fabs(x0), ax1 = fabs(x1), ay0 = fabs(y0), ay1 = fabs(y1), az0 = fabs(z0), az1 = fabs(z1);
+  if (g.absr > 0.0 && fmin(fmin(fmin(D000, D001), fmin(D010, D011)), fmin(fmin(D100, D101), fmin(D110, D111))) < 10.0 * g.absr) {
+    Ss.z = cuboid_axis_L(cuboid_guard_b(g, z0, D000, xy00), cuboid_guard_b(g, z1, D001, xy00), cuboid_guard_b(g, z0, D010, xy01),
+                         cuboid_guard_b(g, z1, D011, xy01), cuboid_guard_b(g, z0, D100, xy10), cuboid_guard_b(g, z1, D101, xy10),
+                         cuboid_guard_b(g, z0, D110, xy11), cuboid_guard_b(g, z1, D111, xy11), xy10 * xy01, xy00 * xy11, mz, hi32(z0) < 0);
+    Ss.y = cuboid_axis_L(cuboid_guard_b(g, y0, D000, xz00), cuboid_guard_b(g, y1, D010, xz00), cuboid_guard_b(g, y0, D001, xz01),
+                         cuboid_guard_b(g, y1, D011, xz01), cuboid_guard_b(g, y0, D100, xz10), cuboid_guard_b(g, y1, D110, xz10),
+                         cuboid_guard_b(g, y0, D101, xz11), cuboid_guard_b(g, y1, D111, xz11), xz10 * xz01, xz00 * xz11, my, hi32(y0) < 0);
+    Ss.x = cuboid_axis_L(cuboid_guard_b(g, x0, D000, yz00), cuboid_guard_b(g, x1, D100, yz00), cuboid_guard_b(g, x0, D001, yz01),
+                         cuboid_guard_b(g, x1, D101, yz01), cuboid_guard_b(g, x0, D010, yz10), cuboid_guard_b(g, x1, D110, yz10),
+                         cuboid_guard_b(g, x0, D011, yz11), cuboid_guard_b(g, x1, D111, yz11), yz10 * yz01, yz00 * yz11, mx, hi32(x0) < 0);
+  } else {
+    Ss.z = cuboid_axis_L(az0 + D000, az1 + D001, az0 + D010, az1 + D011, az0 + D100, az1 + D101, az0 + D110, az1 + D111,
+                         xy10 * xy01, xy00 * xy11, mz, hi32(z0) < 0);
+    Ss.y = cuboid_axis_L(ay0 + D000, ay1 + D010, ay0 + D001, ay1 + D011, ay0 + D100, ay1 + D110, ay0 + D101, ay1 + D111,
+                         xz10 * xz01, xz00 * xz11, my, hi32(y0) < 0);
+    Ss.x = cuboid_axis_L(ax0 + D000, ax1 + D100, ax0 + D001, ax1 + D101, ax0 + D010, ax1 + D110, ax0 + D011, ax1 + D111,
+                         yz10 * yz01, yz00 * yz11, mx, hi32(x0) < 0);
+  }
+  // S is minus the logarithm
+  Ss = mk3<double>(flip_sign(Ss.x, ~ws), flip_sign(Ss.y, ~ws), flip_sign(Ss.z, ~ws));
+  Tt = mk3<double>(flip_sign(Tt.x, ws), flip_sign(Tt.y, ws), flip_sign(Tt.z, ws));
+  if (nan) {
+    const double bad = __longlong_as_double(0x7ff8000000000000LL);
+    if (nan & 1) Tt.x = bad;
+    if (nan & 2) Tt.y = bad;
+    if (nan & 4) Tt.z = bad;
+  }
+  return in;
 }
 
 // Field of a current-carrying cuboid (radrec.cpp:183-249, J branch), q

@@ -141,7 +141,7 @@ struct GeomView {
   const double *vtx2d;
   const double *arc;
   const double *bkg;
-  const int4 *units;  // {kind, source, transform, 0}, ordered by kind
+  const int4 *units;  // {kind, source, transform, 1 if its point map is diagonal}, ordered by kind
   int n_units;
   int ustart[5];      // first unit of each kind (cuboid, polyhedron, arc, background), end
   Guard g;

@@ -63,9 +63,10 @@ __device__ V3<double> noalloc_source(const RadB200Geom &G, const Guard &gd, int 
         if (fabs(qc.x) < hd.x && fabs(qc.y) < hd.y && fabs(qc.z) < hd.z) f = mk3<double>(r[6], r[7], r[8]);
       } else {
         V3<double> Tt, Ss;
-        int in = cuboid_TS<double>(qc, hd, gd, Tt, Ss);
-        f = mk3<double>(Tt.x * r[6] - Ss.z * r[7] - Ss.y * r[8], -Ss.z * r[6] + Tt.y * r[7] - Ss.x * r[8],
-                        -Ss.y * r[6] - Ss.x * r[7] + Tt.z * r[8]);
+        int in = cuboid_TS(qc, hd, gd, Tt, Ss);
+        const double cx = CUBOID_C * r[6], cy = CUBOID_C * r[7], cz = CUBOID_C * r[8];
+        f = mk3<double>(Tt.x * cx - Ss.z * cy - Ss.y * cz, -Ss.z * cx + Tt.y * cy - Ss.x * cz,
+                        -Ss.y * cx - Ss.x * cy + Tt.z * cz);
         if (what == 0 && in) { f.x += r[6]; f.y += r[7]; f.z += r[8]; }
       }
     } else if (kind == 1) {

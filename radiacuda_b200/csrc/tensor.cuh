@@ -16,23 +16,19 @@ __device__ __forceinline__ void cuboid_tensor(const GeomView &g, int idx, V3<dou
   V3<double> qc = mk3<double>(q.x - __ldg(r + 0), q.y - __ldg(r + 1), q.z - __ldg(r + 2));
   V3<double> hd = mk3<double>(0.5 * __ldg(r + 3), 0.5 * __ldg(r + 4), 0.5 * __ldg(r + 5));
   V3<double> Tt, Ss;
-  cuboid_TS<double>(qc, hd, g.g, Tt, Ss);
-  Q[0] = Tt.x;  Q[1] = -Ss.z; Q[2] = -Ss.y;
-  Q[3] = -Ss.z; Q[4] = Tt.y;  Q[5] = -Ss.x;
-  Q[6] = -Ss.y; Q[7] = -Ss.x; Q[8] = Tt.z;
+  cuboid_TS(qc, hd, g.g, Tt, Ss);
+  Q[0] = CUBOID_C * Tt.x;
+  Q[4] = CUBOID_C * Tt.y;
+  Q[8] = CUBOID_C * Tt.z;
+  Q[1] = Q[3] = -CUBOID_C * Ss.z;
+  Q[2] = Q[6] = -CUBOID_C * Ss.y;
+  Q[5] = Q[7] = -CUBOID_C * Ss.x;
 }
 
 __device__ __forceinline__ void elem_tensor(const GeomView &g, int kind, int idx, V3<double> q, double *Q)
 {
   if (kind == 0) {
-    const double *r = g.rec + (size_t)idx * RADB200_REC_STRIDE;
-    V3<double> qc = mk3<double>(q.x - __ldg(r + 0), q.y - __ldg(r + 1), q.z - __ldg(r + 2));
-    V3<double> hd = mk3<double>(0.5 * __ldg(r + 3), 0.5 * __ldg(r + 4), 0.5 * __ldg(r + 5));
-    V3<double> Tt, Ss;
-    cuboid_TS<double>(qc, hd, g.g, Tt, Ss);  // (q relative to the centre, FP64)
-    Q[0] = Tt.x;  Q[1] = -Ss.z; Q[2] = -Ss.y;
-    Q[3] = -Ss.z; Q[4] = Tt.y;  Q[5] = -Ss.x;
-    Q[6] = -Ss.y; Q[7] = -Ss.x; Q[8] = Tt.z;
+    cuboid_tensor(g, idx, q, Q);
     return;
   }
   if (g.fast && __ldg(&g.tp.tinfo[idx].y) >= 0) {  // vertex/edge form

@@ -280,8 +280,8 @@ static void build_tet_record(const std::vector<double> &V, const std::vector<std
       double nu[3] = {t[1] * n[2] - t[2] * n[1], t[2] * n[0] - t[0] * n[2], t[0] * n[1] - t[1] * n[0]};
       int e = tet_pair(std::min(a, b), std::max(a, b));
       if (tensor) {
-        for (int r = 0; r < 3; r++)
-          for (int c = 0; c < 3; c++) rec[42 + 9 * e + 3 * r + c] += nu[r] * n[c];
+        for (int r = 0, k = 0; r < 3; r++)
+          for (int c = r; c < 3; c++, k++) rec[42 + 6 * e + k] += 0.5 * (nu[r] * n[c] + nu[c] * n[r]);
       } else {
         for (int c = 0; c < 3; c++) rec[42 + 3 * e + c] += sigma * nu[c];
       }
@@ -450,12 +450,16 @@ static void build_topo(const RadB200Geom *G, bool tensor, HostTopo &h)
   }
 }
 
-int DevGeom::upload(const RadB200Geom *G, bool tensor_coeffs, bool mesh)
+int DevGeom::upload(const RadB200Geom *G, Form form)
 {
   RB_TRY(validate_geom(G));
+  g.absr = G->abs_rand; g.relr = G->rel_rand; g.zeror = G->zero_rand;
   all_tets = 0;
   tet_single = 0;
-  if (G->n_poly > 0) {
+  has_topo = 0;
+  m_tiles = m_groups = 0;
+  if (G->n_poly > 0 && form != FACES) {
+    const bool tensor_coeffs = form == TENSOR;
     HostTopo h;
     PhaseClock pc;
     build_topo(G, tensor_coeffs, h);
@@ -476,13 +480,11 @@ int DevGeom::upload(const RadB200Geom *G, bool tensor_coeffs, bool mesh)
     all_tets = std::all_of(h.tetidx.begin(), h.tetidx.end(), [](int t) { return t >= 0; }) ? 1 : 0;
     tet_single = all_tets && G->n_rec == 0 && G->n_arc == 0 && G->n_bkg == 0;
     for (int i = 0; i < G->n_poly && tet_single; i++) tet_single = G->poly_info[4 * i + 3] == 1;
-    m_tiles = m_groups = 0;
+    has_topo = 1;
     // field geometry of an all-tetrahedron model: the mesh form (unique edges and faces)
     pc.mark("geometry: topology upload");
-    if (all_tets && !tensor_coeffs && mesh) RB_TRY(build_mesh(G, h.tetidx, h.tetrec, *this));
+    if (all_tets && form == MESH) RB_TRY(build_mesh(G, h.tetidx, h.tetrec, *this));
     pc.mark("geometry: mesh form");
-  } else {
-    m_tiles = m_groups = 0;
   }
   RB_TRY(trf.upload(G->trf, (size_t)G->n_trf * RADB200_TRF_STRIDE * sizeof(double)));
   RB_TRY(rec.upload(G->rec, (size_t)G->n_rec * RADB200_REC_STRIDE * sizeof(double)));
@@ -492,6 +494,15 @@ int DevGeom::upload(const RadB200Geom *G, bool tensor_coeffs, bool mesh)
   RB_TRY(face.upload(G->face, (size_t)G->n_face * RADB200_FACE_STRIDE * sizeof(double)));
   RB_TRY(face_vtx.upload(G->face_vtx, (size_t)G->n_face * 2 * sizeof(int)));
   RB_TRY(vtx2d.upload(G->vtx2d, (size_t)G->n_vtx * 2 * sizeof(double)));
+  RB_TRY(edge.alloc((size_t)G->n_vtx * EDGE_REC * sizeof(double)));
+  RB_TRY(launch_edge_records(face_vtx.as<int>(), vtx2d.as<double>(), G->n_face, edge.as<double>(), 0));
+  all_tri = form == FACES && G->n_poly > 0;
+  for (int f = 0; f < G->n_face && all_tri; f++) all_tri = G->face_vtx[2 * f + 1] == 3;
+  for (int i = 0; i < G->n_poly && all_tri; i++) all_tri = G->poly_info[4 * i + 1] <= TRI_TILE;
+  if (all_tri) {
+    RB_TRY(tri.alloc((size_t)G->n_face * TRI_REC * sizeof(double)));
+    RB_TRY(launch_tri_records(view(0), G->n_poly, tri.as<double>(), 0));
+  }
   RB_TRY(arc.upload(G->arc, (size_t)G->n_arc * RADB200_ARC_STRIDE * sizeof(double)));
   RB_TRY(bkg.upload(G->bkg, (size_t)G->n_bkg * 3 * sizeof(double)));
   // unit table: one entry per (source, image); cuboids, polyhedra, arcs, backgrounds
@@ -518,7 +529,6 @@ int DevGeom::upload(const RadB200Geom *G, bool tensor_coeffs, bool mesh)
   RB_TRY(units.upload(u.data(), u.size() * sizeof(int4)));
   n_rec = G->n_rec;
   n_poly = G->n_poly;
-  g.absr = G->abs_rand; g.relr = G->rel_rand; g.zeror = G->zero_rand;
   return 0;
 }
 
@@ -527,13 +537,14 @@ GeomView DevGeom::view(int fast) const
   GeomView v;
   v.trf = trf.as<double>(); v.rec = rec.as<double>(); v.rec_img = rec_img.as<int>();
   v.poly = poly.as<double>(); v.poly_info = poly_info.as<int>(); v.face = face.as<double>();
-  v.face_vtx = face_vtx.as<int>(); v.vtx2d = vtx2d.as<double>(); v.arc = arc.as<double>();
+  v.face_vtx = face_vtx.as<int>(); v.vtx2d = vtx2d.as<double>(); v.edge = edge.as<double>(); v.arc = arc.as<double>();
   v.bkg = bkg.as<double>(); v.units = units.as<int4>(); v.n_units = n_units; v.g = g;
   for (int k = 0; k < 5; k++) v.ustart[k] = ustart[k];
   v.tp.tinfo = tinfo.as<int4>(); v.tp.tinfo2 = tinfo2.as<int4>(); v.tp.tv = tv.as<double>();
   v.tp.te = te.as<int2>(); v.tp.tel = tel.as<double>(); v.tp.teg = teg.as<double>(); v.tp.teG = teG.as<double>();
   v.tp.tt = tt.as<int4>(); v.tp.ttm = ttm.as<double>(); v.tp.tfn = tfn.as<double>(); v.tp.tfa = tfa.as<double>();
-  v.fast = (fast && tinfo.p) ? 1 : 0;
+  v.fast = (fast && has_topo) ? 1 : 0;
+  v.tri = all_tri ? tri.as<double>() : nullptr;
   v.tetidx = tetidx.as<int>();
   v.tetrec = tetrec.as<double>();
   v.all_tets = all_tets;
@@ -639,7 +650,7 @@ int radb200_field_dev(const RadB200Geom *g, const double *d_pts, int64_t npts, i
   if (npts < 0 || what < 0 || what > 2 || precision < 0 || precision > 2) { set_error("bad field arguments"); return RADB200_E_ARG; }
   PhaseClock pc;
   // the mesh form serves FP64 B / H only
-  RB_TRY(g_fld_geom.upload(g, false, precision != 1 && what != 2));
+  RB_TRY(g_fld_geom.upload(g, precision == 0 ? DevGeom::FACES : precision == 2 && what != 2 ? DevGeom::MESH : DevGeom::FIELD));
   pc.mark("field: geometry upload");
   RB_TRY(launch_field(g_fld_geom.view(precision != 0), d_pts, npts, what, precision == 1 ? 1 : 0, d_out, g_fld_scratch, 0));
   RB_CUDA(cudaStreamSynchronize(0));
@@ -738,7 +749,7 @@ static int intrc_create_impl(const RadB200Geom *elems, const RadB200Relax *r, co
   if (I->nr != n && storage == RADB200_STORE_MIXED) { set_error("row blocks are stored FP32 or FP64"); return RADB200_E_ARG; }
   const int nr = I->nr;
   PhaseClock pc;
-  RB_TRY(I->geom.upload(elems, fast != 0));
+  RB_TRY(I->geom.upload(elems, fast ? DevGeom::TENSOR : DevGeom::FACES));
   I->fast = fast;
   pc.mark("create: geometry upload");
   // observation points and row transforms from each element's main image
@@ -796,7 +807,7 @@ static int intrc_create_impl(const RadB200Geom *elems, const RadB200Relax *r, co
   RB_CUDA(cudaMemset(I->hext.p, 0, vb));
   if (ext && (ext->n_rec + ext->n_poly + ext->n_arc + ext->n_bkg) > 0) {
     DevGeom &xg = I->xgeom;
-    RB_TRY(xg.upload(ext));
+    RB_TRY(xg.upload(ext, fast ? DevGeom::MESH : DevGeom::FACES));
     I->has_ext = 1;
     DBuf tmp, scratch;
     RB_TRY(tmp.alloc(3 * (size_t)nr * sizeof(double)));

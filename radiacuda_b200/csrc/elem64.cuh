@@ -123,17 +123,11 @@ RB_HD double angle64(double y, double x, int turns)
   return fma(dj, 0.78539816339744828, fma(dj, 3.0616169978683830e-17, flip_sign(a, neg)));
 }
 
-// log(n / d), n and d positive.  k: the power of two that brings n 2^-k / d
-// into [0.66, 1.5], read off the upper words; |s| <= 0.203.
-RB_HD double log_ratio64(double n, double d)
+// 2 artanh(s) = log((1 + s) / (1 - s)) for |s| <= 0.203: relative error of the
+// polynomial 1.8e-17
+RB_HD double artanh2_poly(double s)
 {
-  const int hn = hi32(n), hd = hi32(d);
-  // both normal, and the quotient's exponent in range; anything else (a point
-  // on an edge line: 0, infinity or NaN) takes the library's functions
-  if ((unsigned)(hn - 0x04000000) > 0x78000000u || (unsigned)(hd - 0x04000000) > 0x78000000u) return log(n / d);
-  const int k = (hn - hd + 0x80000) >> 20;
-  const double m = add_hi32(n, -(k << 20));
-  const double s = (m - d) * rcp64(m + d), z = s * s;
+  const double z = s * s;
   double p = 0x1.3c89e0ccdadebp-4;
   p = fma(p, z, 0x1.38143e890ab4dp-4);
   p = fma(p, z, 0x1.74783f2c7e313p-4);
@@ -141,8 +135,91 @@ RB_HD double log_ratio64(double n, double d)
   p = fma(p, z, 0x1.249249db9161bp-3);
   p = fma(p, z, 0x1.99999998a73b4p-3);
   p = fma(p, z, 0x1.5555555555927p-2);
-  const double t = s + s, dk = (double)k;
-  return fma(dk, 0.69314718055994529, fma(dk, 2.3190468138462996e-17, fma(t * z, p, t)));
+  const double t = s + s;
+  return fma(t * z, p, t);
 }
+// k log(2) + L
+RB_HD double add_klog2(int k, double L)
+{
+  const double dk = (double)k;
+  return fma(dk, 0.69314718055994529, fma(dk, 2.3190468138462996e-17, L));
+}
+// both upper words those of normal numbers well inside the range
+RB_HD bool plain_ratio(int hn, int hd)
+{
+  return (unsigned)(hn - 0x04000000) <= 0x78000000u && (unsigned)(hd - 0x04000000) <= 0x78000000u;
+}
+
+// log(n / d), n and d positive.  k: the power of two that brings n 2^-k / d
+// into [0.66, 1.5], read off the upper words.  log_plain64: both of ordinary
+// size (plain_ratio); log_ratio64 also takes zero, infinity and NaN (a point on
+// an edge line), by the library's function.
+RB_HD double log_plain64(double n, double d)
+{
+  const int k = (hi32(n) - hi32(d) + 0x80000) >> 20;
+  const double m = add_hi32(n, -(k << 20));
+  return add_klog2(k, artanh2_poly((m - d) * rcp64(m + d)));
+}
+RB_HD double log_ratio64(double n, double d) { return plain_ratio(hi32(n), hi32(d)) ? log_plain64(n, d) : log(n / d); }
+
+// L = int dl / |q - r'| along an edge of length l, S = Ra + Rb the sum of its
+// ends' distances from the point: log((S + l) / (S - l)) = 2 artanh(l / S),
+// whose relative accuracy a distant point needs (the terms of a body cancel to
+// third order there).  edge_log_far64: S - l not below S / 8.  Closer to the
+// edge S - l cancels and is 2 D / (S + l), D = Ra Rb + a.b (edge_D64).  The
+// two are apart so that a kernel can form several edges' far values without a
+// branch between them and mend the rare near ones after.
+RB_HD double edge_log_far64(double S, double l)
+{
+  const double n = S + l, d = S - l;
+  const int k = (hi32(n) - hi32(d) + 0x80000) >> 20;
+  const double m = add_hi32(n, -(k << 20));
+  const double u = k ? m - d : l, v = k ? m + d : S;
+  return add_klog2(k, artanh2_poly(u * rcp64(v)));
+}
+RB_HD bool edge_near64(double S, double l) { return hi32(S - l) < hi32(0.125 * S); }
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ static
+#else
+static
+#endif
+double edge_log_near64(double S, double l, double D)
+{
+  const double n = S + l;
+  return log_ratio64(n * n, 2.0 * D);
+}
+// D = Ra Rb + a.b of two offsets, |a x b|^2 / (Ra Rb - a.b) when a.b < 0
+#ifdef __CUDACC__
+__host__ __device__ __noinline__ static
+#else
+static
+#endif
+double edge_D64(double ax, double ay, double az, double Ra, double bx, double by, double bz, double Rb)
+{
+  const double s = fma(ax, bx, fma(ay, by, az * bz)), p = Ra * Rb;
+  if (!(s < 0.0)) return p + s;
+  const double cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
+  return (cx * cx + cy * cy + cz * cz) / (p - s);
+}
+
+// L of N edges, ends' distance sums S and lengths l: all far values first,
+// then the near ones again; nearD(e) gives D of edge e
+template <int N, typename F> RB_HD void edge_logs64(const double *S, const double *l, double *L, F nearD)
+{
+  bool near = false;
+#pragma unroll
+  for (int e = 0; e < N; e++) {
+    L[e] = edge_log_far64(S[e], l[e]);
+    near |= edge_near64(S[e], l[e]);
+  }
+  if (near) {
+#pragma unroll
+    for (int e = 0; e < N; e++)
+      if (edge_near64(S[e], l[e])) L[e] = edge_log_near64(S[e], l[e], nearD(e));
+  }
+}
+
+// arctan2(y, x)
+RB_HD double atan2_64(double y, double x) { return angle64(y, x, 0); }
 
 }  // namespace rb

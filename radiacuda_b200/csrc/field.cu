@@ -22,7 +22,7 @@ namespace rb {
 // KIND: 0 cuboid, 1 polyhedron (face-by-face form), 2 polyhedron (vertex/edge
 // form where available), 3 arc current, 4 background.  One kernel is compiled
 // per kind so each gets the register budget of its own formula.
-enum { UK_REC = 0, UK_POLY = 1, UK_POLY_FAST = 2, UK_ARC = 3, UK_BKG = 4, UK_TET = 5 };
+enum { UK_REC = 0, UK_POLY = 1, UK_POLY_FAST = 2, UK_ARC = 3, UK_BKG = 4, UK_TET = 5, UK_TRI = 6 };
 
 template <typename T, int KIND>
 __device__ __forceinline__ V3<double> eval_unit(const GeomView &g, int4 u, V3<double> P, int what)
@@ -97,16 +97,9 @@ __device__ __forceinline__ V3<double> eval_unit(const GeomView &g, int4 u, V3<do
       double mloc = r6 * mx + r7 * my + r8 * mz;
       int v0 = __ldg(g.face_vtx + 2 * fi), nv = __ldg(g.face_vtx + 2 * fi + 1);
       const double *vt = g.vtx2d + 2 * (size_t)v0;
-      double cx = 0, cy = 0;
-      if (g.g.absr != 0.0 || g.g.relr != 0.0 || g.g.zeror != 0.0) {
-        for (int k = 0; k < nv; k++) { cx += __ldg(vt + 2 * k); cy += __ldg(vt + 2 * k + 1); }
-        cx /= nv; cy /= nv;
-      }
       double plx = r0 * q.x + r1 * q.y + r2 * q.z, ply = r3 * q.x + r4 * q.y + r5 * q.z, plz = r6 * q.x + r7 * q.y + r8 * q.z;
-      // the face-by-face form stays in FP64: its products of powers of the edge
-      // slope overflow the FP32 range for near-vertical edges
       double s0, s1, s2;
-      int in = polygon_S<double, double>(vt, nv, cz, cx, cy, mk3<double>(plx, ply, plz), g.g, s0, s1, s2);
+      int in = polygon_S(vt, g.edge + EDGE_REC * (size_t)v0, nv, cz, mk3<double>(plx, ply, plz), g.g, s0, s1, s2);
       if (!in) inside = 0;
       if (what != 2) {
         double w = -CH * mloc;
@@ -138,12 +131,12 @@ __device__ __forceinline__ V3<double> eval_unit(const GeomView &g, int4 u, V3<do
 // Units [ub, ue) of one kind; gridDim.y splits them into chunks.  With one
 // chunk the result goes to out directly (accumulate: out += result), else to
 // the chunk's slice of the partial buffer.
-template <typename T, int KIND>
 //
 // Cuboids: bound by the FP64 pipe (about 430 operations a pair, 65-70% of its
 // rate) and the latency between them.  4 CTAs per SM (128 registers): 3.94e9
 // pairs in 136 ms, 2.9e10 pairs/s; 143 ms at 3 CTAs (158 registers); 490 ms
 // with the term-by-term formula.
+template <typename T, int KIND>
 __global__ void __launch_bounds__(128, KIND == UK_REC ? 4 : 1) field_kernel(GeomView g, const double *__restrict__ pts, int64_t npts, int what,
                                                     double *__restrict__ out, int ub, int ue, int chunk, int accumulate)
 {
@@ -311,6 +304,133 @@ static int launch_tet(const GeomView &g, const double *d_pts, int64_t npts, int 
   return launch_tet_ppt<T, 1>(g, d_pts, npts, what, d_out, ub, ue, accumulate, scratch, st);
 }
 
+// Triangle-face records (TRI_REC): a thread per polyhedron.
+__global__ void tri_record_kernel(GeomView g, int n_poly, double *__restrict__ tri)
+{
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n_poly) return;
+  // the reference's polygon face form uses this 15-digit pi (radplnr2.cpp:32)
+  const double CH = 1.0 / (4.0 * 3.14159265358979);
+  const double *pr = g.poly + (size_t)p * RADB200_POLY_STRIDE;
+  const int f0 = g.poly_info[4 * p], nf = g.poly_info[4 * p + 1];
+  for (int f = f0; f < f0 + nf; f++) {
+    const double *R = g.face + (size_t)f * RADB200_FACE_STRIDE;
+    const double *vt = g.vtx2d + 2 * (size_t)g.face_vtx[2 * f];
+    double *o = tri + (size_t)f * TRI_REC;
+    const double n[3] = {R[6], R[7], R[8]}, c = CH * (n[0] * pr[3] + n[1] * pr[4] + n[2] * pr[5]);
+    double a2 = 0.0, cx = 0.0, cy = 0.0;
+    for (int k = 0; k < 3; k++) {
+      const double x = vt[2 * k], y = vt[2 * k + 1];
+      double e[EDGE_REC];
+      edge_record(vt, 3, k, e);
+      if (k == 1) a2 = e[3];
+      cx += x;
+      cy += y;
+      o[9 + k] = e[2];
+      for (int d = 0; d < 3; d++) {
+        o[3 * k + d] = x * R[d] + y * R[3 + d] + R[9] * R[6 + d];
+        o[18 + 3 * k + d] = c * (e[1] * R[d] - e[0] * R[3 + d]);  // outward: direction turned by -90 degrees
+      }
+    }
+    for (int d = 0; d < 3; d++) {
+      o[12 + d] = a2 * n[d];
+      o[15 + d] = -c * n[d];
+    }
+    o[27] = fmax(abs_rand(g.g, R[9]), fmax(abs_rand(g.g, vt[0] - cx / 3), abs_rand(g.g, vt[1] - cy / 3)));
+  }
+}
+
+int launch_tri_records(const GeomView &g, int n_poly, double *tri, cudaStream_t st)
+{
+  tri_record_kernel<<<(n_poly + 127) / 128, 128, 0, st>>>(g, n_poly, tri);
+  return check_launch("tri_record_kernel");
+}
+
+// Face-by-face field of polyhedra with triangle faces.  The general kernel
+// above reads a face through a chain of dependent loads (polyhedron, face,
+// vertices) and waits on it: FP64 pipe 25% busy, 6e7 tetrahedron pairs in 8.4
+// ms.  Here a block stages the records of up to TRI_TILE faces of up to 16
+// units in shared memory: FP64 pipe 62% busy, 3.7 ms (1.6e10 pairs/s); the
+// reference's polygon formula took 28 ms.
+constexpr int TRI_UNITS = 16;
+__global__ void __launch_bounds__(128) field_tri_kernel(GeomView g, const double *__restrict__ pts, int64_t npts, int what,
+                                                        double *__restrict__ out, int ub, int ue, int chunk, int accumulate)
+{
+  __shared__ double sf[TRI_TILE * TRI_REC];
+  __shared__ double su[TRI_UNITS * 24];  // point map (12), field map (9), magnetization (3)
+  __shared__ int s_face[TRI_UNITS], s_end[TRI_UNITS + 1], s_unit[TRI_UNITS], s_trf[TRI_UNITS], s_n;
+  const int tid = threadIdx.x;
+  const int64_t i = (int64_t)blockIdx.x * 128 + tid;
+  const int u0 = ub + blockIdx.y * chunk, u1 = min(ue, u0 + chunk);
+  V3<double> P = mk3<double>(0, 0, 0);
+  if (i < npts) P = mk3<double>(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]);
+  double acc[3] = {0, 0, 0};
+  for (int base = u0; base < u1;) {
+    __syncthreads();  // the previous tile's readers are done
+    if (tid < 32) {
+      // the units that fit: a running sum of their faces
+      int4 un = make_int4(0, 0, 0, 0);
+      int nf = 0, f0 = 0;
+      const bool has = tid < TRI_UNITS && base + tid < u1;
+      if (has) {
+        un = __ldg(g.units + base + tid);
+        f0 = __ldg(g.poly_info + 4 * un.y);
+        nf = __ldg(g.poly_info + 4 * un.y + 1);
+      }
+      int sum = nf;
+#pragma unroll
+      for (int o = 1; o < TRI_UNITS; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (tid >= o) sum += v;
+      }
+      const unsigned fit = __ballot_sync(0xffffffffu, has && sum <= TRI_TILE);
+      if (has) {
+        s_face[tid] = f0;
+        s_end[tid + 1] = sum;
+        s_unit[tid] = un.y;
+        s_trf[tid] = un.z;
+      }
+      if (tid == 0) {
+        s_end[0] = 0;
+        s_n = __popc(fit);
+      }
+    }
+    __syncthreads();
+    const int nu = s_n;
+    for (int k = 0; k < nu; k++) {
+      const int e0 = s_end[k] * TRI_REC, ne = (s_end[k + 1] - s_end[k]) * TRI_REC;
+      const double *src = g.tri + (size_t)s_face[k] * TRI_REC;
+      for (int e = tid; e < ne; e += 128) sf[e0 + e] = __ldg(src + e);
+    }
+    for (int e = tid; e < nu * 24; e += 128) {
+      const int k = e / 24, f = e - 24 * k;
+      su[e] = f < 21 ? __ldg(g.trf + (size_t)s_trf[k] * RADB200_TRF_STRIDE + f)
+                     : __ldg(g.poly + (size_t)s_unit[k] * RADB200_POLY_STRIDE + 3 + (f - 21));
+    }
+    __syncthreads();
+    for (int k = 0; k < nu; k++) {
+      const double *Tr = su + 24 * k, *F = Tr + 12, *M = Tr + 21;
+      const double dx = P.x - Tr[9], dy = P.y - Tr[10], dz = P.z - Tr[11];
+      const V3<double> q = mk3<double>(Tr[0] * dx + Tr[1] * dy + Tr[2] * dz, Tr[3] * dx + Tr[4] * dy + Tr[5] * dz,
+                                       Tr[6] * dx + Tr[7] * dy + Tr[8] * dz);
+      double h[3] = {0, 0, 0};
+      int inside = 1;
+      for (int f = s_end[k]; f < s_end[k + 1]; f++) inside &= tri_face(sf + f * TRI_REC, q, h);
+      if (what == 2) h[0] = h[1] = h[2] = 0.0;
+      if (what != 1 && inside) { h[0] += M[0]; h[1] += M[1]; h[2] += M[2]; }
+      acc[0] += F[0] * h[0] + F[1] * h[1] + F[2] * h[2];
+      acc[1] += F[3] * h[0] + F[4] * h[1] + F[5] * h[2];
+      acc[2] += F[6] * h[0] + F[7] * h[1] + F[8] * h[2];
+    }
+    base += nu;
+  }
+  if (i < npts) {
+    double *o = out + ((size_t)blockIdx.y * npts + i) * 3;
+    if (accumulate) { o[0] += acc[0]; o[1] += acc[1]; o[2] += acc[2]; }
+    else { o[0] = acc[0]; o[1] = acc[1]; o[2] = acc[2]; }
+  }
+}
+
 template <typename T, int KIND>
 static int launch_kind(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int ub, int ue,
                        int accumulate, DBuf &scratch, cudaStream_t st)
@@ -327,13 +447,16 @@ static int launch_kind(const GeomView &g, const double *d_pts, int64_t npts, int
   int chunk = (nu + nchunk - 1) / nchunk;
   nchunk = (nu + chunk - 1) / chunk;
   dim3 grid((unsigned)nblk, (unsigned)nchunk);
-  if (nchunk == 1) {
-    field_kernel<T, KIND><<<grid, TPB, 0, st>>>(g, d_pts, npts, what, d_out, ub, ue, chunk, accumulate);
-    return check_launch("field_kernel");
+  double *dst = d_out;
+  if (nchunk > 1) {
+    RB_TRY(scratch.alloc((size_t)nchunk * npts * 3 * sizeof(double)));
+    dst = scratch.as<double>();
   }
-  RB_TRY(scratch.alloc((size_t)nchunk * npts * 3 * sizeof(double)));
-  field_kernel<T, KIND><<<grid, TPB, 0, st>>>(g, d_pts, npts, what, scratch.as<double>(), ub, ue, chunk, 0);
+  const int acc = nchunk > 1 ? 0 : accumulate;
+  if constexpr (KIND == UK_TRI) field_tri_kernel<<<grid, TPB, 0, st>>>(g, d_pts, npts, what, dst, ub, ue, chunk, acc);
+  else field_kernel<T, KIND><<<grid, TPB, 0, st>>>(g, d_pts, npts, what, dst, ub, ue, chunk, acc);
   RB_TRY(check_launch("field_kernel"));
+  if (nchunk == 1) return 0;
   int64_t n3 = npts * 3;
   chunk_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(scratch.as<double>(), nchunk, n3, d_out, accumulate);
   return check_launch("chunk_reduce_kernel");
@@ -373,13 +496,15 @@ int launch_field(const GeomView &g, const double *d_pts, int64_t npts, int what,
     // tetrahedra one by one, at a 1.25x speed-up (1.42x in FP64)
     else if (kind == 1 && g.fast && g.all_tets && g.mesh.n_tiles > 0 && what != 2 && precision != 1 &&
              mesh_form_enabled())
-      rc = launch_mesh_field(g, d_pts, npts, what, precision, d_out, acc, scratch, st);
+      rc = launch_mesh_field(g, d_pts, npts, what, d_out, acc, scratch, st);
     else if (kind == 1 && g.fast && g.all_tets)
       rc = (precision == 1) ? launch_tet<float>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st)
                             : launch_tet<double>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st);
     else if (kind == 1 && g.fast)
       rc = (precision == 1) ? launch_kind<float, UK_POLY_FAST>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st)
                             : launch_kind<double, UK_POLY_FAST>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st);
+    else if (kind == 1 && g.tri)
+      rc = launch_kind<double, UK_TRI>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st);
     else if (kind == 1)
       rc = launch_kind<double, UK_POLY>(g, d_pts, npts, what, d_out, ub, ue, acc, scratch, st);
     else if (kind == 2)
@@ -390,6 +515,22 @@ int launch_field(const GeomView &g, const double *d_pts, int64_t npts, int what,
     acc = 1;
   }
   return 0;
+}
+
+__global__ void edge_record_kernel(const int *__restrict__ face_vtx, const double *__restrict__ vtx2d, int n_face,
+                                   double *__restrict__ edge)
+{
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= n_face) return;
+  const int v0 = face_vtx[2 * f], nv = face_vtx[2 * f + 1];
+  for (int j = 0; j < nv; j++) edge_record(vtx2d + 2 * (size_t)v0, nv, j, edge + EDGE_REC * ((size_t)v0 + j));
+}
+
+int launch_edge_records(const int *face_vtx, const double *vtx2d, int n_face, double *edge, cudaStream_t st)
+{
+  if (n_face <= 0) return 0;
+  edge_record_kernel<<<(n_face + 127) / 128, 128, 0, st>>>(face_vtx, vtx2d, n_face, edge);
+  return check_launch("edge_record_kernel");
 }
 
 // out_i = rowT_i * in_i  (3x3 per element)

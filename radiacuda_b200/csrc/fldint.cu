@@ -586,7 +586,7 @@ int radb200_field_int(const RadB200Geom *g, const double *P1, const double *P2, 
   GeomView view{};
   PointField fld = [&](const RadB200Geom *gg, const double *pts, int64_t n, int w, double *res) -> int {
     if (up != gg) {
-      RB_TRY(g_int_geom.upload(gg));
+      RB_TRY(g_int_geom.upload(gg, precision != 0 ? DevGeom::MESH : DevGeom::FACES));
       view = g_int_geom.view(precision != 0);
       up = gg;
     }
@@ -638,7 +638,7 @@ int radb200_trajectories(const RadB200Geom *g, double energy_gev, int n_traj, co
   }
   if (n_traj == 0) return 0;
   if ((size_t)n_traj * (size_t)np * 5 > ((size_t)1 << 31)) { set_error("too many trajectory points"); return RADB200_E_ARG; }
-  RB_TRY(g_trj_geom.upload(g));
+  RB_TRY(g_trj_geom.upload(g, DevGeom::FACES));
   RB_TRY(g_trj_init.upload(init, (size_t)n_traj * 4 * sizeof(double)));
   size_t ob = (size_t)n_traj * np * 5 * sizeof(double);
   RB_TRY(g_trj_out.alloc(ob));

@@ -280,9 +280,13 @@ __device__ __forceinline__ V3<double> cuboid_J(V3<double> q, V3<double> hd, V3<d
 // Planar polygon face integrals (Sx,Sy,Sz) at a point given in the face frame
 // (px,py,pz), vertices (counter-clockwise) in shared or global memory.
 // Returns 1 when the point is on the inner side of the face plane (z > 0).
-// radTPolygon::B_comp, radplnr2.cpp:29-388 (B/H/PreRelax paths).
+// radTPolygon::B_comp, radplnr2.cpp:29-388 (B/H/PreRelax paths), term by term.
+// Used where blocks of the interaction matrix must follow the reference's own
+// rounding: close to slivers its terms lose 1e-12 of a block and more, which
+// chi = 1000 amplifies, and relaxed magnetizations are compared at 1e-9.
+// Fields use polygon_S below (2,500 against about 170 issue slots a face).
 template <typename T, typename VP>
-__device__ __forceinline__ int polygon_S(const VP *vtx, int nv, T coordz, T cx, T cy, V3<T> P,
+__device__ __forceinline__ int polygon_S_terms(const VP *vtx, int nv, T coordz, T cx, T cy, V3<T> P,
                                           const Guard &g, T &Sx_o, T &Sy_o, T &Sz_o)
 {
   const T Max_k = T(1.E+09);
@@ -366,6 +370,146 @@ __device__ __forceinline__ int polygon_S(const VP *vtx, int nv, T coordz, T cx, 
   Sx += logT(arg_logs2);
   Sx_o = Sx; Sy_o = Sy; Sz_o = sum_atan;
   return z > T(0);
+}
+
+// ---- polygon face ---------------------------------------------------------------
+// Face integrals (Sx, Sy, Sz) of a planar polygon at a point given in the face
+// frame (radTPolygon::B_comp, radplnr2.cpp:29-388; B/H/PreRelax paths):
+//   (Sx, Sy) = sum over edges of (-ty, tx) L,   Sz = solid angle, > 0 below,
+// with (tx, ty) the edge's direction and L = edge_log64.  The reference writes
+// each edge as y = k x + b: its log(L2/L1)/sqrt(k^2+1) is this L, the
+// remaining product of its logarithm telescopes to the vertical edges' share,
+// and its arctangents of one edge each sum to the solid angle of the polygon.
+// Here an edge costs one logarithm and no quotient (directions and lengths
+// are kept per vertex, EdgeRec), neighbouring edges share a distance, and a
+// triangle of the fan takes one arctangent (Van Oosterom-Strackee), its
+// numerator z times twice its area: a triangle face about 170 FP64 operations
+// against 2,500 issue slots.
+constexpr int EDGE_REC = 4;
+// of polygon vertex j: direction (2) and length of the edge to the next
+// vertex, twice the area of the fan triangle (0, j, j + 1)
+RB_HD void edge_record(const double *vtx, int nv, int j, double *e)
+{
+  const int k = j + 1 < nv ? j + 1 : 0;
+  const double ex = vtx[2 * k] - vtx[2 * j], ey = vtx[2 * k + 1] - vtx[2 * j + 1];
+  const double l = sqrt(ex * ex + ey * ey);
+  const double fx = vtx[2 * j] - vtx[0], fy = vtx[2 * j + 1] - vtx[1];
+  e[0] = ex / l;
+  e[1] = ey / l;
+  e[2] = l;
+  e[3] = fx * ey - fy * ex;
+}
+
+// half the solid angle of a triangle whose plane is at height z: a2 twice its
+// area, offsets (x, y, z) and distances of its vertices
+__device__ __forceinline__ double half_solid_angle(double z, double zz, double a2, double x0, double y0, double R0,
+                                                   double x1, double y1, double R1, double x2, double y2, double R2)
+{
+  const double d01 = fma(x0, x1, fma(y0, y1, zz)), d02 = fma(x0, x2, fma(y0, y2, zz)), d12 = fma(x1, x2, fma(y1, y2, zz));
+  return atan2_64(z * a2, fma(fma(R0, R1, d01), R2, fma(d02, R1, d12 * R0)));
+}
+
+// vtx: nv counter-clockwise vertices in the face frame; er: their edge records
+// (null: formed here); z == 0 steps off the plane by the length guard.
+// Returns 1 when the point is on the inner side of the face plane (z > 0).
+__device__ __forceinline__ int polygon_S(const double *vtx, const double *er, int nv, double coordz, V3<double> P,
+                                         const Guard &g, double &Sx, double &Sy, double &Sz)
+{
+  double z = coordz - P.z;
+  if (z == 0.0 && (g.absr != 0.0 || g.relr != 0.0 || g.zeror != 0.0)) {
+    double cx = 0, cy = 0;
+    for (int k = 0; k < nv; k++) { cx += vtx[2 * k]; cy += vtx[2 * k + 1]; }
+    z = fmax(abs_rand(g, coordz), fmax(abs_rand(g, vtx[0] - cx / nv), abs_rand(g, vtx[1] - cy / nv)));
+  }
+  const double zz = z * z;
+  auto edge = [&](int j, double *e) {
+    if (er) {
+      const double2 a = __ldg(reinterpret_cast<const double2 *>(er + EDGE_REC * j)),
+                    b = __ldg(reinterpret_cast<const double2 *>(er + EDGE_REC * j) + 1);
+      e[0] = a.x; e[1] = a.y; e[2] = b.x; e[3] = b.y;
+    } else edge_record(vtx, nv, j, e);
+  };
+  auto edge_L = [&](double ax, double ay, double Ra, double bx, double by, double Rb, double l) {
+    const double S = Ra + Rb;
+    double L;
+    edge_logs64<1>(&S, &l, &L, [&](int) { return edge_D64(ax, ay, z, Ra, bx, by, z, Rb); });
+    return L;
+  };
+  const double x0 = vtx[0] - P.x, y0 = vtx[1] - P.y, R0 = sqrt64(fma(x0, x0, fma(y0, y0, zz)));
+  double e[EDGE_REC];
+  if (nv == 3) {
+    const double x1 = vtx[2] - P.x, y1 = vtx[3] - P.y, R1 = sqrt64(fma(x1, x1, fma(y1, y1, zz)));
+    const double x2 = vtx[4] - P.x, y2 = vtx[5] - P.y, R2 = sqrt64(fma(x2, x2, fma(y2, y2, zz)));
+    edge(0, e);
+    double L = edge_L(x0, y0, R0, x1, y1, R1, e[2]);
+    Sx = -e[1] * L;
+    Sy = e[0] * L;
+    edge(2, e);
+    L = edge_L(x2, y2, R2, x0, y0, R0, e[2]);
+    Sx = fma(-e[1], L, Sx);
+    Sy = fma(e[0], L, Sy);
+    edge(1, e);
+    L = edge_L(x1, y1, R1, x2, y2, R2, e[2]);
+    Sx = fma(-e[1], L, Sx);
+    Sy = fma(e[0], L, Sy);
+    Sz = 2.0 * half_solid_angle(z, zz, e[3], x0, y0, R0, x1, y1, R1, x2, y2, R2);
+    return z > 0.0;
+  }
+  double xp = x0, yp = y0, Rp = R0;
+  Sx = Sy = Sz = 0.0;
+  for (int j = 0; j < nv; j++) {
+    double xn = x0, yn = y0, Rn = R0;
+    if (j + 1 < nv) {
+      xn = vtx[2 * j + 2] - P.x;
+      yn = vtx[2 * j + 3] - P.y;
+      Rn = sqrt64(fma(xn, xn, fma(yn, yn, zz)));
+    }
+    edge(j, e);
+    const double L = edge_L(xp, yp, Rp, xn, yn, Rn, e[2]);
+    Sx = fma(-e[1], L, Sx);
+    Sy = fma(e[0], L, Sy);
+    if (j > 0 && j + 1 < nv) Sz += 2.0 * half_solid_angle(z, zz, e[3], x0, y0, R0, xp, yp, Rp, xn, yn, Rn);
+    xp = xn; yp = yn; Rp = Rn;
+  }
+  return z > 0.0;
+}
+
+// ---- triangle face in three dimensions -------------------------------------------
+// For polyhedra of triangles (meshes): the same face integral from the face's
+// own vertices in the object frame.  Record, TRI_REC doubles:
+//   [0,9) vertices  [9,12) edge lengths (01 12 20)  [12,15) m, normal times
+//   twice the area  [15,18) -c n  [18,27) c nu of the edges (outward, in plane)
+//   [27] the length guard's step off the plane (0 without guards)
+// c = M.n / (4 pi) with the face form's pi, so that H += sum L c nu - half angle * 2 c n.
+constexpr int TRI_REC = 28;
+
+// adds the face's H to h; returns 1 when q is on the inner side
+__device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double *h)
+{
+  double x[3], y[3], z[3], R[3], S[3], L[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) { x[k] = rec[3 * k] - q.x; y[k] = rec[3 * k + 1] - q.y; z[k] = rec[3 * k + 2] - q.z; }
+  const double m0 = rec[12], m1 = rec[13], m2 = rec[14];
+  double num = fma(x[0], m0, fma(y[0], m1, z[0] * m2));
+  if (num == 0.0 && rec[27] > 0.0) {  // on the plane, guards on
+    const double mm = sqrt64(fma(m0, m0, fma(m1, m1, m2 * m2))), s = rec[27] / mm;
+    for (int k = 0; k < 3; k++) { x[k] += s * m0; y[k] += s * m1; z[k] += s * m2; }
+    num = rec[27] * mm;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; k++) R[k] = sqrt64(fma(x[k], x[k], fma(y[k], y[k], z[k] * z[k])));
+  S[0] = R[0] + R[1]; S[1] = R[1] + R[2]; S[2] = R[2] + R[0];
+  edge_logs64<3>(S, rec + 9, L, [&](int e) {
+    const int b = e == 2 ? 0 : e + 1;
+    return edge_D64(x[e], y[e], z[e], R[e], x[b], y[b], z[b], R[b]);
+  });
+  const double d01 = fma(x[0], x[1], fma(y[0], y[1], z[0] * z[1])), d12 = fma(x[1], x[2], fma(y[1], y[2], z[1] * z[2])),
+               d02 = fma(x[0], x[2], fma(y[0], y[2], z[0] * z[2]));
+  const double w = 2.0 * atan2_64(num, fma(fma(R[0], R[1], d01), R[2], fma(d02, R[1], d12 * R[0])));
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    h[c] += fma(L[0], rec[18 + c], fma(L[1], rec[21 + c], fma(L[2], rec[24 + c], w * rec[15 + c])));
+  return num > 0.0;
 }
 
 // Arc current field at q (object frame), record a = [cx cy cz rmin rmax
@@ -475,10 +619,31 @@ struct TopoView {
 
 constexpr int POLY_NV_FAST = 8;  // vertices handled in registers
 
-template <typename T>
-__device__ __forceinline__ T log1pT(T x);
-template <> __device__ __forceinline__ double log1pT<double>(double x) { return log1p(x); }
-template <> __device__ __forceinline__ float log1pT<float>(float x) { return log1pf(x); }
+// the vertex/edge forms' elements in either precision: distance, edge
+// integral L (ends a, b, their distances and dot product d) and angle
+__device__ __forceinline__ double edge_R(double x, double y, double z) { return sqrt64(fma(x, x, fma(y, y, z * z))); }
+__device__ __forceinline__ float edge_R(float x, float y, float z) { return sqrtf(x * x + y * y + z * z); }
+__device__ __forceinline__ double edge_L(double ax, double ay, double az, double Ra, double bx, double by, double bz,
+                                         double Rb, double, double l)
+{
+  const double S = Ra + Rb;
+  double L;
+  edge_logs64<1>(&S, &l, &L, [&](int) { return edge_D64(ax, ay, az, Ra, bx, by, bz, Rb); });
+  return L;
+}
+__device__ __forceinline__ float edge_L(float ax, float ay, float az, float Ra, float bx, float by, float bz, float Rb,
+                                        float d, float l)
+{
+  float D;
+  if (d >= 0.f) D = Ra * Rb + d;
+  else {
+    const float cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
+    D = (cx * cx + cy * cy + cz * cz) / (Ra * Rb - d);
+  }
+  return log1pf(l * (Ra + Rb + l) / D);
+}
+__device__ __forceinline__ double face_angle(double y, double x) { return atan2_64(y, x); }
+__device__ __forceinline__ float face_angle(float y, float x) { return atan2f(y, x); }
 
 // Solid angles and edge logs of polyhedron p at q (object frame).
 // Accumulates H (field mode, a_f / g_e set) or the tensor Q (tensor mode).
@@ -495,7 +660,7 @@ __device__ __forceinline__ int poly_fast(const TopoView &tp, int p, V3<double> q
     if (k < nv) {
       const double *v = tp.tv + 3 * (size_t)(v0 + k);
       rx[k] = T(__ldg(v) - q.x); ry[k] = T(__ldg(v + 1) - q.y); rz[k] = T(__ldg(v + 2) - q.z);
-      R[k] = sqrtT(rx[k] * rx[k] + ry[k] * ry[k] + rz[k] * rz[k]);
+      R[k] = edge_R(rx[k], ry[k], rz[k]);
     } else {
       rx[k] = ry[k] = rz[k] = R[k] = T(0);
     }
@@ -513,14 +678,7 @@ __device__ __forceinline__ int poly_fast(const TopoView &tp, int p, V3<double> q
       if (k == ab.x) { ax = rx[k]; ay = ry[k]; az = rz[k]; Ra = R[k]; }
       if (k == ab.y) { bx = rx[k]; by = ry[k]; bz = rz[k]; Rb = R[k]; }
     }
-    T s = ax * bx + ay * by + az * bz;
-    T D;
-    if (s >= T(0)) D = Ra * Rb + s;
-    else {
-      T cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
-      D = (cx * cx + cy * cy + cz * cz) / (Ra * Rb - s);
-    }
-    T L = log1pT<T>(l * (Ra + Rb + l) / D);
+    T L = edge_L(ax, ay, az, Ra, bx, by, bz, Rb, ax * bx + ay * by + az * bz, l);
     double Ld = (double)L;
     if (TENSOR) {
       const double *G = tp.teG + 9 * (size_t)e;
@@ -566,7 +724,7 @@ __device__ __forceinline__ int poly_fast(const TopoView &tp, int p, V3<double> q
     T num = xa * T(__ldg(m)) + ya * T(__ldg(m + 1)) + za * T(__ldg(m + 2));
     T den = Ra * Rb * Rc + (xa * xb + ya * yb + za * zb) * Rc + (xa * xc + ya * yc + za * zc) * Rb +
             (xb * xc + yb * yc + zb * zc) * Ra;
-    om += 2.0 * (double)atan2T(-num, den);
+    om += 2.0 * (double)face_angle(-num, den);
   }
 #pragma unroll
   for (int k = 0; k < (TENSOR ? 9 : 3); k++) out[k] = C * acc[k];
@@ -580,8 +738,10 @@ __device__ __forceinline__ int poly_fast(const TopoView &tp, int p, V3<double> q
 // unrolled.  Record (object frame), TET_REC_FIELD doubles:
 //   [0,12) vertices  [12,18) edge lengths  [18,30) m_t  [30,42) a_f = sigma_f n_f
 //   [42,60) g_e = sum_f sigma_f nu_{e,f}
-// TET_REC_TENSOR doubles: [0,30) as above, [30,42) n_f, [42,96) G_e (3x3 each).
-constexpr int TET_REC_FIELD = 60, TET_REC_TENSOR = 96;
+// TET_REC_TENSOR doubles: [0,30) as above, [30,42) n_f, [42,78) the symmetric
+// parts of G_e (xx xy xz yy yz zz each): the tensor is symmetric, so the
+// antisymmetric parts cancel in its sum over edges.
+constexpr int TET_REC_FIELD = 60, TET_REC_TENSOR = 78;
 __host__ __device__ constexpr int tet_edge_a(int e) { return e < 3 ? 0 : (e < 5 ? 1 : 2); }
 __host__ __device__ constexpr int tet_edge_b(int e) { return e == 0 ? 1 : e == 1 ? 2 : e == 2 ? 3 : e == 3 ? 2 : 3; }
 // face f (opposite vertex f) = triangle (a, b, c)
@@ -614,7 +774,7 @@ __device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<doubl
     rx[k] = T(rd_rec<SMEM>(rec + 3 * k) - q.x);
     ry[k] = T(rd_rec<SMEM>(rec + 3 * k + 1) - q.y);
     rz[k] = T(rd_rec<SMEM>(rec + 3 * k + 2) - q.z);
-    R[k] = sqrtT(rx[k] * rx[k] + ry[k] * ry[k] + rz[k] * rz[k]);
+    R[k] = edge_R(rx[k], ry[k], rz[k]);
   }
   T d[6];  // r_i . r_j per edge
 #pragma unroll
@@ -622,27 +782,34 @@ __device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<doubl
     const int a = tet_edge_a(e), b = tet_edge_b(e);
     d[e] = rx[a] * rx[b] + ry[a] * ry[b] + rz[a] * rz[b];
   }
-  double acc[TENSOR ? 9 : 3];
+  double acc[TENSOR ? 6 : 3];
 #pragma unroll
-  for (int k = 0; k < (TENSOR ? 9 : 3); k++) acc[k] = 0.0;
+  for (int k = 0; k < (TENSOR ? 6 : 3); k++) acc[k] = 0.0;
+  T Le[6];
+  if constexpr (sizeof(T) == 8) {
+    double S[6], l[6];
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      S[e] = R[tet_edge_a(e)] + R[tet_edge_b(e)];
+      l[e] = rd_rec<SMEM>(rec + 12 + e);
+    }
+    edge_logs64<6>(S, l, Le, [&](int e) {
+      const int a = tet_edge_a(e), b = tet_edge_b(e);
+      return edge_D64(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b]);
+    });
+  } else {
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      const int a = tet_edge_a(e), b = tet_edge_b(e);
+      const T l = fl ? T(recf[e]) : T(rd_rec<SMEM>(rec + 12 + e));
+      Le[e] = edge_L(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b], d[e], l);
+    }
+  }
 #pragma unroll
   for (int e = 0; e < 6; e++) {
-    const int a = tet_edge_a(e), b = tet_edge_b(e);
-    T l = fl ? T(recf[e]) : T(rd_rec<SMEM>(rec + 12 + e));
-    T D;
-    if (d[e] >= T(0)) D = R[a] * R[b] + d[e];
-    else {
-      T cx = ry[a] * rz[b] - rz[a] * ry[b], cy = rz[a] * rx[b] - rx[a] * rz[b], cz = rx[a] * ry[b] - ry[a] * rx[b];
-      D = (cx * cx + cy * cy + cz * cz) / (R[a] * R[b] - d[e]);
-    }
-    double L = (double)log1pT<T>(l * (R[a] + R[b] + l) / D);
-    if (TENSOR) {
+    const double L = (double)Le[e];
 #pragma unroll
-      for (int k = 0; k < 9; k++) acc[k] += L * rd_rec<SMEM>(rec + 42 + 9 * e + k);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 3; k++) acc[k] += L * rd_rec<SMEM>(rec + 42 + 3 * e + k);
-    }
+    for (int k = 0; k < (TENSOR ? 6 : 3); k++) acc[k] += L * rd_rec<SMEM>(rec + 42 + (TENSOR ? 6 : 3) * e + k);
   }
   double omega_tot = 0.0;
 #pragma unroll
@@ -653,20 +820,28 @@ __device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<doubl
     const T m2 = fl ? T(recf[8 + 3 * f]) : T(rd_rec<SMEM>(rec + 20 + 3 * f));
     T num = rx[a] * m0 + ry[a] * m1 + rz[a] * m2;
     T den = R[a] * R[b] * R[c] + d[tet_pair(a, b)] * R[c] + d[tet_pair(a, c)] * R[b] + d[tet_pair(b, c)] * R[a];
-    double om = 2.0 * (double)atan2T(-num, den);
+    double om = 2.0 * (double)face_angle(-num, den);
     omega_tot += om;
+    const double n0 = rd_rec<SMEM>(rec + 30 + 3 * f), n1 = rd_rec<SMEM>(rec + 31 + 3 * f), n2 = rd_rec<SMEM>(rec + 32 + 3 * f);
     if (TENSOR) {
-      double n0 = rd_rec<SMEM>(rec + 30 + 3 * f), n1 = rd_rec<SMEM>(rec + 31 + 3 * f), n2 = rd_rec<SMEM>(rec + 32 + 3 * f);
-      acc[0] += om * n0 * n0; acc[1] += om * n0 * n1; acc[2] += om * n0 * n2;
-      acc[3] += om * n1 * n0; acc[4] += om * n1 * n1; acc[5] += om * n1 * n2;
-      acc[6] += om * n2 * n0; acc[7] += om * n2 * n1; acc[8] += om * n2 * n2;
+      const double o0 = om * n0, o1 = om * n1, o2 = om * n2;
+      acc[0] += o0 * n0; acc[1] += o0 * n1; acc[2] += o0 * n2;
+      acc[3] += o1 * n1; acc[4] += o1 * n2; acc[5] += o2 * n2;
     } else {
-#pragma unroll
-      for (int k = 0; k < 3; k++) acc[k] += om * rd_rec<SMEM>(rec + 30 + 3 * f + k);
+      acc[0] += om * n0; acc[1] += om * n1; acc[2] += om * n2;
     }
   }
+  if (TENSOR) {
+    out[0] = C * acc[0];
+    out[4] = C * acc[3];
+    out[8] = C * acc[5];
+    out[1] = out[3] = C * acc[1];
+    out[2] = out[6] = C * acc[2];
+    out[5] = out[7] = C * acc[4];
+  } else {
 #pragma unroll
-  for (int k = 0; k < (TENSOR ? 9 : 3); k++) out[k] = C * acc[k];
+    for (int k = 0; k < 3; k++) out[k] = C * acc[k];
+  }
   return omega_tot < -6.283185307179586;
 }
 

@@ -113,8 +113,8 @@ struct DBuf {
 // computed once per tile, and the edges and faces the tile owns (each unique
 // edge or face belongs to exactly one tile).
 constexpr int MESH_VT = 32, MESH_EMAX = 128, MESH_FMAX = 160;
-constexpr int MESH_E = 6;   // edge record: a, b (tile-local vertices), l, G (3)
-constexpr int MESH_F = 13;  // face record: a, b, c, l_ab, l_ac, l_bc, m (3, unnormalized normal), v_a . m, A (3)
+constexpr int MESH_E = 5;   // edge record: a, b (tile-local vertices, packed in the low word), l, G (3)
+constexpr int MESH_F = 11;  // face record: a, b, c (packed), l_ab^2/2, l_ac^2/2, l_bc^2/2, m (3, unnormalized normal), v_a . m, A (3)
 struct MeshView {
   int n_tiles = 0;
   const int4 *tile = nullptr;   // [2 per tile] {first vertex slot, vertices, first edge, edges}, {first face, faces, transform, 0}
@@ -139,6 +139,7 @@ struct GeomView {
   const double *face;
   const int *face_vtx;
   const double *vtx2d;
+  const double *edge;  // [n_vtx * EDGE_REC] of every face's vertices (edge_record)
   const double *arc;
   const double *bkg;
   const int4 *units;  // {kind, source, transform, 1 if its point map is diagonal}, ordered by kind
@@ -150,22 +151,29 @@ struct GeomView {
   const double *tetrec;
   int all_tets;       // every polyhedron has a tetrahedron record
   int tet_single;     // ... and the sources are only those tetrahedra, one image each
+  const double *tri;  // [n_face * TRI_REC] when every polyhedron has at most TRI_TILE faces, all triangles (else null)
   int fast;           // 1: evaluate polyhedra in the vertex/edge form
   MeshView mesh;      // all-tetrahedron models: unique edges and faces (n_tiles 0: none)
 };
 
 struct DevGeom {
-  DBuf trf, rec, rec_img, poly, poly_info, face, face_vtx, vtx2d, arc, bkg, units;
+  DBuf trf, rec, rec_img, poly, poly_info, face, face_vtx, vtx2d, edge, arc, bkg, units;
   // polyhedron topology (vertex/edge form), see TopoView in formulas.cuh
   DBuf tinfo, tinfo2, tv, te, tel, teg, teG, tt, ttm, tfn, tfa;
+  DBuf tri;             // triangle faces of the face form (tri_face)
+  int all_tri = 0;
   DBuf tetidx, tetrec;  // fixed-topology tetrahedron records (tet_fast)
   DBuf m_tile, m_v, m_e, m_f, m_group, m_gbox, m_gtet;  // mesh form (MeshView)
   int m_tiles = 0, m_groups = 0;
   int n_units = 0, n_rec = 0, n_poly = 0;
   int ustart[5] = {0, 0, 0, 0, 0};
-  int all_tets = 0, tet_single = 0;
+  int all_tets = 0, tet_single = 0, has_topo = 0;
   Guard g{0, 0, 0};
-  int upload(const RadB200Geom *G, bool tensor_coeffs = false, bool mesh = true);
+  // forms of the polyhedra to prepare: faces only (view(0)), the vertex/edge
+  // form with field coefficients, the same with the mesh form, or with tensor
+  // coefficients
+  enum Form { FACES, FIELD, MESH, TENSOR };
+  int upload(const RadB200Geom *G, Form form);
   GeomView view(int fast = 0) const;
 };
 
@@ -269,6 +277,7 @@ int launch_round_f32(const double *a, float *b, size_t n, cudaStream_t st);
 struct Op {
   virtual int apply(const double *v, double *out) = 0;  // out = A v
   virtual int precond(double *v) = 0;                   // v <- P v
+  bool cheap = false;  // no preconditioner: a product may be queued ahead of need
   virtual ~Op() {}
 };
 int gmres(Op &op, int n3, int ld, const double *b, double *x, double rtol, int max_iter, int restart, double *relres,
@@ -293,19 +302,43 @@ int tc_gemm_f32_inplace(float *C, int ldc, int m, int n, int k, float *A, int ld
                         cudaStream_t st, int *used, bool c_is_a, int slot = 0);
 int tc_error_flag(int *flag);  // 2 when a tensor-core CTA hit its wait limit
 
+#ifdef __CUDACC__
+// true in the last block of the launch to arrive; its threads then see every
+// block's writes
+__device__ __forceinline__ bool last_block(unsigned *count)
+{
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (last) *count = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+#endif
+
 // ---- kernels (launch wrappers) ---------------------------------------------
 int launch_field(const GeomView &g, const double *d_pts, int64_t npts, int what, int precision,
                  double *d_out, DBuf &scratch, cudaStream_t st);
 int launch_assemble(const GeomView &g, const int *elem_src, const double *obs, const double *rowT, int nr, int n,
                     int ld, float *N32, double *N64, cudaStream_t st);
+// faces staged at a time by the triangle-face field kernel
+constexpr int TRI_TILE = 64;
+// records of triangle faces with the polyhedra's magnetizations (field.cu)
+int launch_tri_records(const GeomView &g, int n_poly, double *tri, cudaStream_t st);
+// edge records of all faces (field.cu)
+int launch_edge_records(const int *face_vtx, const double *vtx2d, int n_face, double *edge, cudaStream_t st);
 int launch_rowtrans_vec(const double *rowT, const double *in, double *out, int n, cudaStream_t st);
 // mesh form of an all-tetrahedron geometry from its tetrahedron records
 // (mesh.cu); tetidx[p] = record of polyhedron p
 int build_mesh(const RadB200Geom *G, const std::vector<int> &tetidx, const std::vector<double> &tetrec, DevGeom &dg);
 // field of the tetrahedra in the mesh form, all units of kind polyhedron
 // (what 0 B, 1 H; mesh.cu)
-int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int what, int precision, double *d_out,
-                      int accumulate, DBuf &scratch, cudaStream_t st);
+int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int accumulate,
+                      DBuf &scratch, cudaStream_t st);
 // near lists of mixed storage from the element geometry (host, near.cu);
 // obs: [3n] element centres (main images)
 int build_near(Intrc &I, const RadB200Geom *elems, const RadB200Relax *r, const double *obs);

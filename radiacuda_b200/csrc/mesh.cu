@@ -20,9 +20,10 @@
 // the 20,000-tetrahedron model at 1e6 points in FP64).  Points inside a
 // tetrahedron add its magnetization (B), found by a separate inside test that
 // only points in a group's bounding box run.  The field dispatch uses this
-// form in FP64; the FP32-term variant is compiled but not dispatched (its
-// largest per-point error was 2.7x that of the per-tetrahedron FP32 kernel).
+// form in FP64 (with FP32 terms its largest per-point error was 2.7x that of
+// the per-tetrahedron FP32 kernel).
 #include <math.h>
+#include <string.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -65,6 +66,15 @@ struct MeshHost {
   std::vector<double> gbox;
   std::vector<int> gtet;
 };
+
+// up to three tile-local vertex slots in the low word of a record's first double
+double packed_slots(int a, int b, int c)
+{
+  const int64_t w = a | (b << 8) | (c << 16);
+  double d;
+  memcpy(&d, &w, sizeof(d));
+  return d;
+}
 
 // One image transform's tetrahedra (polyhedron indices) into tiles.
 void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, const std::vector<double> &tetrec, int trf,
@@ -180,14 +190,15 @@ void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, 
     };
     for (int id : tedges) {
       int a = ev[2 * (size_t)id], b = ev[2 * (size_t)id + 1];
-      double r[MESH_E] = {(double)slot[a], (double)slot[b], len(a, b), G[3 * (size_t)id], G[3 * (size_t)id + 1],
+      double r[MESH_E] = {packed_slots(slot[a], slot[b], 0), len(a, b), G[3 * (size_t)id], G[3 * (size_t)id + 1],
                           G[3 * (size_t)id + 2]};
       out.e.insert(out.e.end(), r, r + MESH_E);
     }
     for (int id : tfaces) {
       int a = fv[3 * (size_t)id], b = fv[3 * (size_t)id + 1], c = fv[3 * (size_t)id + 2];
       const double *m = &M[3 * (size_t)id], *pa = &V[3 * (size_t)a];
-      double r[MESH_F] = {(double)slot[a], (double)slot[b], (double)slot[c], len(a, b), len(a, c), len(b, c),
+      const double lab = len(a, b), lac = len(a, c), lbc = len(b, c);
+      double r[MESH_F] = {packed_slots(slot[a], slot[b], slot[c]), 0.5 * lab * lab, 0.5 * lac * lac, 0.5 * lbc * lbc,
                           m[0], m[1], m[2], pa[0] * m[0] + pa[1] * m[1] + pa[2] * m[2],
                           A[3 * (size_t)id], A[3 * (size_t)id + 1], A[3 * (size_t)id + 2]};
       out.f.insert(out.f.end(), r, r + MESH_F);
@@ -256,12 +267,12 @@ int build_mesh(const RadB200Geom *G, const std::vector<int> &tetidx, const std::
 
 // dynamic shared memory: the tile's vertices, edges and faces, then every
 // thread's distances to the tile's vertices
-template <typename T> constexpr size_t mesh_smem()
-{
-  return sizeof(double) * (MESH_VT * 3 + MESH_EMAX * MESH_E + MESH_FMAX * MESH_F) + sizeof(T) * MESH_VT * 128;
-}
+constexpr size_t MESH_SMEM = sizeof(double) * (MESH_VT * 3 + MESH_EMAX * MESH_E + MESH_FMAX * MESH_F + MESH_VT * 128);
 
-template <typename T>
+// Bound by the FP64 pipe and its latency: about 33 operations per unique edge
+// and 50 per unique face with the elements of elem64.cuh.  6,000 tetrahedra at
+// 100,000 points: 13.1 ms (4.6e10 tetrahedron pairs/s, FP64 pipe 54% busy);
+// 23 ms with the library's log1p, atan2 and square root.
 __global__ void __launch_bounds__(128) mesh_field_kernel(GeomView g, const double *__restrict__ pts, int64_t npts,
                                                          double *__restrict__ out, int chunk, int accumulate)
 {
@@ -269,7 +280,7 @@ __global__ void __launch_bounds__(128) mesh_field_kernel(GeomView g, const doubl
   double *sv = smem;
   double *se = sv + MESH_VT * 3;
   double *sf = se + MESH_EMAX * MESH_E;
-  T(*sR)[128] = reinterpret_cast<T(*)[128]>(sf + MESH_FMAX * MESH_F);
+  double(*sR)[128] = reinterpret_cast<double(*)[128]>(sf + MESH_FMAX * MESH_F);
   const int tid = threadIdx.x;
   const int64_t i = (int64_t)blockIdx.x * 128 + tid;
   const MeshView &mv = g.mesh;
@@ -290,47 +301,50 @@ __global__ void __launch_bounds__(128) mesh_field_kernel(GeomView g, const doubl
     const V3<double> q = mk3<double>(__ldg(Tr + 0) * dx + __ldg(Tr + 1) * dy + __ldg(Tr + 2) * dz,
                                      __ldg(Tr + 3) * dx + __ldg(Tr + 4) * dy + __ldg(Tr + 5) * dz,
                                      __ldg(Tr + 6) * dx + __ldg(Tr + 7) * dy + __ldg(Tr + 8) * dz);
-    for (int v = 0; v < ta.y; v++) {
-      T rx = T(sv[3 * v] - q.x), ry = T(sv[3 * v + 1] - q.y), rz = T(sv[3 * v + 2] - q.z);
-      sR[v][tid] = sqrtT(rx * rx + ry * ry + rz * rz);
-    }
+#pragma unroll 2
+    for (int v = 0; v < ta.y; v++) sR[v][tid] = edge_R(sv[3 * v] - q.x, sv[3 * v + 1] - q.y, sv[3 * v + 2] - q.z);
     double h0 = 0, h1 = 0, h2 = 0;
-    for (int e = 0; e < ta.w; e++) {
-      const double *r = se + MESH_E * e;
-      const int a = (int)r[0], b = (int)r[1];
-      const T l = T(r[2]), Ra = sR[a][tid], Rb = sR[b][tid];
-      // r_a . r_b from the distances and the edge length
-      const T d = T(0.5) * (Ra * Ra + Rb * Rb - l * l);
-      T D;
-      if (d >= T(0)) D = Ra * Rb + d;
-      else {
-        // the point sees the edge under more than 90 degrees: Ra Rb + d cancels,
-        // use |r_a x r_b|^2 / (Ra Rb - d) from the vectors themselves
-        T ax = T(sv[3 * a] - q.x), ay = T(sv[3 * a + 1] - q.y), az = T(sv[3 * a + 2] - q.z);
-        T bx = T(sv[3 * b] - q.x), by = T(sv[3 * b + 1] - q.y), bz = T(sv[3 * b + 2] - q.z);
-        T cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx;
-        T dd = ax * bx + ay * by + az * bz;
-        D = (cx * cx + cy * cy + cz * cz) / (Ra * Rb - dd);
+    // two edges at a time: independent chains with one branch for the rare near edges
+    for (int e = 0; e < ta.w; e += 2) {
+      const double *r[2] = {se + MESH_E * e, se + MESH_E * min(e + 1, ta.w - 1)};
+      int a[2], b[2];
+      double Ra[2], Rb[2], S[2], l[2], L[2];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int ab = __double2loint(r[k][0]);
+        a[k] = ab & 255;
+        b[k] = ab >> 8;
+        Ra[k] = sR[a[k]][tid];
+        Rb[k] = sR[b[k]][tid];
+        S[k] = Ra[k] + Rb[k];
+        l[k] = r[k][1];
       }
-      const double L = (double)log1pT<T>(l * (Ra + Rb + l) / D);
-      h0 += L * r[3];
-      h1 += L * r[4];
-      h2 += L * r[5];
+      edge_logs64<2>(S, l, L, [&](int k) {
+        const double *va = sv + 3 * a[k], *vb = sv + 3 * b[k];
+        return edge_D64(va[0] - q.x, va[1] - q.y, va[2] - q.z, Ra[k], vb[0] - q.x, vb[1] - q.y, vb[2] - q.z, Rb[k]);
+      });
+      if (e + 1 >= ta.w) L[1] = 0.0;
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        h0 = fma(L[k], r[k][2], h0);
+        h1 = fma(L[k], r[k][3], h1);
+        h2 = fma(L[k], r[k][4], h2);
+      }
     }
+#pragma unroll 2
     for (int f = 0; f < tb.y; f++) {
       const double *r = sf + MESH_F * f;
-      const int a = (int)r[0], b = (int)r[1], c = (int)r[2];
-      const T Ra = sR[a][tid], Rb = sR[b][tid], Rc = sR[c][tid];
-      const T lab = T(r[3]), lac = T(r[4]), lbc = T(r[5]);
-      const T dab = T(0.5) * (Ra * Ra + Rb * Rb - lab * lab), dac = T(0.5) * (Ra * Ra + Rc * Rc - lac * lac),
-              dbc = T(0.5) * (Rb * Rb + Rc * Rc - lbc * lbc);
-      // (v_a - q) . m in FP64
-      const T num = T(r[9] - (q.x * r[6] + q.y * r[7] + q.z * r[8]));
-      const T den = Ra * Rb * Rc + dab * Rc + dac * Rb + dbc * Ra;
-      const double om = 2.0 * (double)atan2T(-num, den);
-      h0 += om * r[10];
-      h1 += om * r[11];
-      h2 += om * r[12];
+      const int abc = __double2loint(r[0]);
+      const double Ra = sR[abc & 255][tid], Rb = sR[(abc >> 8) & 255][tid], Rc = sR[abc >> 16][tid];
+      // dot products by the law of cosines
+      const double Ha = 0.5 * Ra * Ra, Hb = 0.5 * Rb * Rb, Hc = 0.5 * Rc * Rc;
+      const double dab = Ha + Hb - r[1], dac = Ha + Hc - r[2], dbc = Hb + Hc - r[3];
+      // (v_a - q) . m
+      const double num = r[7] - (q.x * r[4] + q.y * r[5] + q.z * r[6]);
+      const double om = 2.0 * atan2_64(-num, fma(fma(Ra, Rb, dab), Rc, fma(dac, Rb, dbc * Ra)));
+      h0 = fma(om, r[8], h0);
+      h1 = fma(om, r[9], h1);
+      h2 = fma(om, r[10], h2);
     }
     const double *F = Tr + 12;  // s M: object frame -> lab
     acc[0] += C * (__ldg(F + 0) * h0 + __ldg(F + 1) * h1 + __ldg(F + 2) * h2);
@@ -394,7 +408,7 @@ __global__ void mesh_reduce_kernel(const double *__restrict__ part, int nc, int6
   out[i] = accumulate ? out[i] + s : s;
 }
 
-int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int what, int precision, double *d_out,
+int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out,
                       int accumulate, DBuf &scratch, cudaStream_t st)
 {
   const int64_t nblk = (npts + 127) / 128;
@@ -416,14 +430,10 @@ int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int 
   }
   static bool attr = false;
   if (!attr) {
-    RB_CUDA(cudaFuncSetAttribute(mesh_field_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mesh_smem<float>()));
-    RB_CUDA(cudaFuncSetAttribute(mesh_field_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mesh_smem<double>()));
+    RB_CUDA(cudaFuncSetAttribute(mesh_field_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MESH_SMEM));
     attr = true;
   }
-  if (precision == 1) mesh_field_kernel<float><<<grid, 128, mesh_smem<float>(), st>>>(g, d_pts, npts, dst, chunk, acc);
-  else mesh_field_kernel<double><<<grid, 128, mesh_smem<double>(), st>>>(g, d_pts, npts, dst, chunk, acc);
+  mesh_field_kernel<<<grid, 128, MESH_SMEM, st>>>(g, d_pts, npts, dst, chunk, acc);
   RB_TRY(check_launch("mesh_field_kernel"));
   if (nchunk > 1) {
     const int64_t n3 = npts * 3;

@@ -79,15 +79,10 @@ __device__ V3<double> noalloc_source(const RadB200Geom &G, const Guard &gd, int 
         const double *R = G.face + (size_t)fi * RADB200_FACE_STRIDE;
         int v0 = G.face_vtx[2 * fi], nv = G.face_vtx[2 * fi + 1];
         const double *vt = G.vtx2d + 2 * (size_t)v0;
-        double cx = 0, cy = 0;
-        if (gd.absr != 0.0 || gd.relr != 0.0 || gd.zeror != 0.0) {
-          for (int k = 0; k < nv; k++) { cx += vt[2 * k]; cy += vt[2 * k + 1]; }
-          cx /= nv; cy /= nv;
-        }
         V3<double> pl = mk3<double>(R[0] * q.x + R[1] * q.y + R[2] * q.z, R[3] * q.x + R[4] * q.y + R[5] * q.z,
                                     R[6] * q.x + R[7] * q.y + R[8] * q.z);
         double s0, s1, s2;
-        if (!polygon_S<double, double>(vt, nv, R[9], cx, cy, pl, gd, s0, s1, s2)) inside = 0;
+        if (!polygon_S(vt, nullptr, nv, R[9], pl, gd, s0, s1, s2)) inside = 0;
         double w = -C * (R[6] * pr[3] + R[7] * pr[4] + R[8] * pr[5]);
         hx += w * (R[0] * s0 + R[3] * s1 + R[6] * s2);
         hy += w * (R[1] * s0 + R[4] * s1 + R[7] * s2);

@@ -55,7 +55,7 @@ __device__ __forceinline__ void elem_tensor(const GeomView &g, int kind, int idx
     }
     V3<double> pl = mk3<double>(r0 * q.x + r1 * q.y + r2 * q.z, r3 * q.x + r4 * q.y + r5 * q.z, r6 * q.x + r7 * q.y + r8 * q.z);
     double s0, s1, s2;
-    polygon_S<double, double>(vt, nv, cz, cx, cy, pl, g.g, s0, s1, s2);
+    polygon_S_terms<double, double>(vt, nv, cz, cx, cy, pl, g.g, s0, s1, s2);
     // Q += (R^T (-C S)) n^T, n = row 2 of R
     double wx = -CH * (r0 * s0 + r3 * s1 + r6 * s2);
     double wy = -CH * (r1 * s0 + r4 * s1 + r7 * s2);

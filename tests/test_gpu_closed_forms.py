@@ -103,3 +103,112 @@ def test_cuboid_guards_and_singular_points(cuda, rad):
             else:
                 assert np.array_equal(np.isfinite(got[:6]), np.isfinite(exp[:6]))
     rad.FldLenRndSw("off")
+
+
+def _octasphere(levels):
+    """A convex polyhedron of 8 * 4^levels triangles."""
+    V = [np.array(v, float) for v in ((1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1))]
+    F = [[a, b, c] for a in (0, 1) for b in (2, 3) for c in (4, 5)]
+    for _ in range(levels):
+        G = []
+        for a, b, c in F:
+            m = []
+            for i, j in ((a, b), (b, c), (c, a)):
+                p = V[i] + V[j]
+                p = p / np.linalg.norm(p)
+                k = next((q for q, v in enumerate(V) if np.abs(v - p).max() < 1e-12), None)
+                if k is None:
+                    k = len(V)
+                    V.append(p)
+                m.append(k)
+            G += [[a, m[0], m[2]], [m[0], b, m[1]], [m[2], m[1], c], m]
+        F = G
+    return np.array(V), F
+
+
+def _poly_H(P, V, faces, M):
+    """H of a convex polyhedron in long double: per face the solid angle and
+    the logarithms of its edges."""
+    V, P, M = (np.asarray(a, LD) for a in (V, P, M))
+    cen = V.mean(0)
+    H = np.zeros_like(P)
+    for f in faces:
+        w = V[f]
+        n = np.cross(w[1] - w[0], w[2] - w[0])
+        n /= np.sqrt((n * n).sum())
+        if (n * (w[0] - cen)).sum() < 0:
+            n, w = -n, w[::-1]
+        s = (M * n).sum()
+        r = w[None] - P[:, None]
+        R = np.sqrt((r * r).sum(-1))
+        om = np.zeros(len(P), LD)
+        for j in range(1, len(f) - 1):
+            i = (0, j, j + 1)
+            num = (r[:, 0] * np.cross(w[j] - w[0], w[j + 1] - w[0])).sum(-1)
+            d = lambda a, b: (r[:, i[a]] * r[:, i[b]]).sum(-1)
+            den = R[:, 0] * R[:, j] * R[:, j + 1] + d(0, 1) * R[:, j + 1] + d(0, 2) * R[:, j] + d(1, 2) * R[:, 0]
+            om -= 2 * np.arctan2(num, den)
+        H += s * om[:, None] * n
+        for j in range(len(f)):
+            k = (j + 1) % len(f)
+            e = w[k] - w[j]
+            l = np.sqrt((e * e).sum())
+            L = np.log1p(l * (R[:, j] + R[:, k] + l) / (R[:, j] * R[:, k] + (r[:, j] * r[:, k]).sum(-1)))
+            H += s * L[:, None] * np.cross(e / l, n)
+    return (H / (4 * LD(np.pi))).astype(float)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["double", "fast"])
+@pytest.mark.parametrize("npts", [1, 127, 129, 700])
+@pytest.mark.parametrize("ntets", [1, 2, 15, 16, 17, 33])
+def test_tetrahedra(cuda, rad, ntets, npts, precision):
+    """Tiles of up to 16 units and 64 faces, blocks of 128 points.  Vertices
+    rebuilt from the face frames are off by a few ulp of their coordinates
+    (below 8); 0.01 from a face or edge that changes a term by at most
+    8 * 10 ulp / 0.01 = 2e-12."""
+    rng = np.random.default_rng(ntets)
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    faces = [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]]
+    base = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
+    V = [1.5 * np.array([k % 4, (k // 4) % 4, k // 16]) + base + rng.uniform(-0.1, 0.1, (4, 3)) for k in range(ntets)]
+    M = rng.normal(size=(ntets, 3))
+    obj = rad.ObjCnt([rad.ObjPolyhdr(v, faces, m) for v, m in zip(V, M)])
+    P = rng.uniform(-1, 7, size=(npts, 3))
+    exp = sum(_poly_H(P, v, [[i - 1 for i in f] for f in faces], m) for v, m in zip(V, M))
+    got = rad.Fld(obj, "h", P, precision=precision)
+    # the long double sums lose half their digits next to an edge too: keep to points off them
+    far = np.array([min(np.abs(np.linalg.norm(p - v, axis=1)).min() for v in V) > 0.05 for p in P])
+    assert np.abs(got - exp)[far].max(initial=0.0) <= 2e-12 * np.sqrt(ntets)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ["prism", "octahedron", "sphere128"])
+def test_polyhedra_by_faces(cuda, rad, shape):
+    """Faces of more than three vertices, and more triangle faces than one
+    staged tile holds: the general kernel.  Far points too."""
+    rng = np.random.default_rng(5)
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    if shape == "prism":
+        a = np.arange(5) * 2 * np.pi / 5
+        V = np.concatenate([np.stack([np.cos(a), np.sin(a), np.full(5, z)], 1) for z in (-0.7, 0.9)])
+        F = [[4, 3, 2, 1, 0], [5, 6, 7, 8, 9]] + [[k, (k + 1) % 5, 5 + (k + 1) % 5, 5 + k] for k in range(5)]
+    else:
+        V, F = _octasphere(0 if shape == "octahedron" else 2)
+    M = np.array([0.4, -1.1, 0.7])
+    obj = rad.ObjPolyhdr(V, [[i + 1 for i in f] for f in F], M)
+    for scale in (1.5, 30.0):
+        P = rng.uniform(-scale, scale, size=(300, 3))
+        exp = _poly_H(P, V, F, M)
+        # a few ulp of rebuilt vertices at 1e-3 or more from every edge
+        assert np.abs(rad.Fld(obj, "h", P) - exp).max() <= 64 * EPS * len(F) / 1e-3 * 1e-1
+    # inside, B carries the magnetization
+    P = rng.uniform(-0.3, 0.3, size=(20, 3))
+    assert np.abs(rad.Fld(obj, "b", P) - (_poly_H(P, V, F, M) + M)).max() <= 1e-12
+    # on a face, an edge and a corner with the guards on: finite
+    rad.FldLenRndSw("on")
+    P = np.array([V[F[0]].mean(0), 0.5 * (V[F[0][0]] + V[F[0][1]]), V[0]])
+    assert np.all(np.isfinite(rad.Fld(obj, "b", P)))
+    rad.FldLenRndSw("off")

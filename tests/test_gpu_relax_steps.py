@@ -1,0 +1,83 @@
+"""The device-resident Anderson iteration and the fused Arnoldi steps at sizes
+around their tiles (128 rows of a basis slice, 256 threads), against dense
+solves of the same matrix."""
+import numpy as np
+import pytest
+
+import models as MD
+import oracle.oracle as O
+from radiacuda_b200 import _native, model
+from util import rel_err
+
+
+def _blocks(rad, n, sat=False):
+    """n cuboids on a line, anisotropic linear or saturating in a background."""
+    MD.reset(rad)
+    rng = np.random.default_rng(n)
+    hs = []
+    iron = rad.MatSatIsoFrm([2000, 1.5], [100, 0.4], [10, 0.2])
+    for k in range(n):
+        m = rng.normal(size=3)
+        h = rad.ObjRecMag([3.0 * k, 0.7 * (k % 3), 0.3 * (k % 5)], [2.0, 2.0, 2.0], (0 * m if sat else m).tolist())
+        rad.MatApl(h, iron if sat else rad.MatLin([0.06, 0.17], m.tolist()))
+        hs.append(h)
+    return rad.ObjCnt(hs + [rad.ObjBckg([0.02, -0.01, 0.05])])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 42, 43, 85, 86, 171])
+def test_jacobi_and_newton_reach_the_dense_solution(cuda, rad, n):
+    h = _blocks(rad, n)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    exp = O.linear_direct(pack, O.assemble(pack), O.extfield(pack))
+    nat = _native.NativeInteraction(pack, 1)
+    try:
+        for method in (0, 1):
+            M, H, st = nat.relax(method, 1e-13, 500, True, 1.0, np.zeros(3 * n))
+            assert st[0] <= 1e-13 and 1 <= st[3] <= 500
+            assert rel_err(M, exp) < 1e-11
+            again, _, st2 = nat.relax(method, 1e-13, 500, True, 1.0, np.zeros(3 * n))
+            assert np.array_equal(M, again) and st2[3] == st[3]   # bitwise reproducible
+        # the step count is exact, in and across batches (one or two linear
+        # elements reach a misfit of zero before the limit)
+        for k in (1, 5, 6, 7) if n > 2 else (1,):
+            _, _, st = nat.relax(0, 1e-300, k, True, 1.0, np.zeros(3 * n))
+            assert st[3] == k
+    finally:
+        nat.free()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [7, 60])
+def test_saturating_methods_agree(cuda, rad, n):
+    h = _blocks(rad, n, sat=True)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    nat = _native.NativeInteraction(pack, 1)
+    try:
+        a, _, sa = nat.relax(0, 1e-12, 3000, True, 1.0, np.zeros(3 * n))
+        b, _, sb = nat.relax(1, 1e-12, 3000, True, 1.0, np.zeros(3 * n))
+        # restarting from the solution ends at once
+        c, _, sc = nat.relax(0, 1e-11, 3000, False, 1.0, b)
+    finally:
+        nat.free()
+    assert sa[0] <= 1e-12 and sb[0] <= 1e-12
+    assert rel_err(a, b) < 1e-9
+    assert sc[3] <= 2 and rel_err(c, b) < 1e-9
+
+
+@pytest.mark.gpu
+def test_adjoint_gmres_restarts(cuda, rad):
+    """More Krylov vectors than one cycle holds: the restarted iteration still
+    reaches the tolerance on a strongly coupled system without a preconditioner
+    that would end it at once."""
+    h, body = MD.tet_mesh(rad, ncell=3, n_tets=100, chi=1000.0)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    n = pack.elem_src.shape[0]
+    exp = O.linear_direct(pack, O.assemble(pack), O.extfield(pack))
+    nat = _native.NativeInteraction(pack, 1)
+    try:
+        M, _, st = nat.relax(1, 1e-11, 20000, True, 1.0, np.zeros(3 * n))
+    finally:
+        nat.free()
+    assert st[0] <= 1e-11
+    assert rel_err(M, exp) < 1e-6

@@ -169,36 +169,53 @@ __device__ __forceinline__ V3<double> find_new_h(int kind, const double *m, cons
   return H;
 }
 
-// Newton polish of the element's implicit field, H = Hq + Q M(H), from
-// find_new_h's result: J = I - Q dM/dH, at most 20 steps, each kept only if
-// it lowers the residual.  find_new_h stops after 15 passes of a linearly
-// converging secant, so its H carries an error that changes from one
-// iteration to the next: a Newton iteration on the relaxation as a whole
-// falls back to linear convergence on it, and Anderson mixing stalls (a
-// 12-element saturating hybrid stopped at a misfit of 4e-5 after 2,000
-// Jacobi iterations).  Polished, the fixed-point map is exact to rounding:
-// the outer Newton converges quadratically and the Jacobi iteration reaches
-// 1e-12 in about a hundred iterations.
-__device__ __forceinline__ double implicit_residual(int kind, const double *m, const double *Q, V3<double> Hq,
-                                                    V3<double> H, const double *__restrict__ mh, double *r)
+// M(H) and dM/dH of a saturating law at one H (one set of tanh)
+__device__ __forceinline__ void sat_law(int kind, const double *m, V3<double> H, const double *__restrict__ mh, V3<double> &M,
+                                        double *D)
 {
-  const V3<double> M = mat_M(kind, m, H, mh);
+  if (kind == RADB200_MAT_TABLE) {
+    M = mat_M(kind, m, H, mh);
+    mat_D(kind, m, H, D, mh);
+    return;
+  }
+  const double h = sqrt(H.x * H.x + H.y * H.y + H.z * H.z);
+  double f, df;
+  tanh_law(m, h, f, df);
+  const bool zero = h < 1e-10;
+  const double ih = zero ? 0.0 : 1.0 / h, ksi = zero ? tanh_ksi0(m) : f * ih;
+  M = mk3<double>(ksi * H.x + m[9], ksi * H.y + m[10], ksi * H.z + m[11]);
+  // D = df u u^T + (f / h)(1 - u u^T), u = H / h
+  const double ux = H.x * ih, uy = H.y * ih, uz = H.z * ih, t = zero ? df : ksi, c = df - t;
+  D[0] = fma(c * ux, ux, t);
+  D[4] = fma(c * uy, uy, t);
+  D[8] = fma(c * uz, uz, t);
+  D[1] = D[3] = c * ux * uy;
+  D[2] = D[6] = c * ux * uz;
+  D[5] = D[7] = c * uy * uz;
+}
+
+__device__ __forceinline__ double implicit_residual(const double *Q, V3<double> Hq, V3<double> H, V3<double> M, double *r)
+{
   r[0] = H.x - Hq.x - (Q[0] * M.x + Q[1] * M.y + Q[2] * M.z);
   r[1] = H.y - Hq.y - (Q[3] * M.x + Q[4] * M.y + Q[5] * M.z);
   r[2] = H.z - Hq.z - (Q[6] * M.x + Q[7] * M.y + Q[8] * M.z);
   return sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
 }
 
+// Newton steps on the element's implicit field, H = Hq + Q M(H), from H: J = I
+// - Q dM/dH, at most 20 steps, each kept only if it lowers the residual.  Sets
+// ok when the residual ended at the rounding of its terms.
 __device__ __forceinline__ V3<double> polish_h(int kind, const double *m, const double *Q, V3<double> Hq, V3<double> H,
-                                               const double *__restrict__ mh)
+                                               const double *__restrict__ mh, bool &ok)
 {
-  if (kind == RADB200_MAT_LINEAR) return H;
-  double r[3], rn = implicit_residual(kind, m, Q, Hq, H, mh, r);
+  V3<double> M;
+  double D[9], r[3];
+  sat_law(kind, m, H, mh, M, D);
+  double rn = implicit_residual(Q, Hq, H, M, r);
   for (int it = 0; it < 20; it++) {
     const double hn = sqrt(H.x * H.x + H.y * H.y + H.z * H.z);
     if (!(rn > 1e-16 * fmax(hn, 1e-30))) break;
-    double D[9], A[9], Ai[9];
-    mat_D(kind, m, H, D, mh);
+    double A[9], Ai[9];
     for (int a = 0; a < 3; a++)
       for (int b = 0; b < 3; b++)
         A[3 * a + b] = (a == b ? 1.0 : 0.0) - (Q[3 * a] * D[b] + Q[3 * a + 1] * D[3 + b] + Q[3 * a + 2] * D[6 + b]);
@@ -206,12 +223,43 @@ __device__ __forceinline__ V3<double> polish_h(int kind, const double *m, const 
     const V3<double> Hn = mk3<double>(H.x - (Ai[0] * r[0] + Ai[1] * r[1] + Ai[2] * r[2]),
                                       H.y - (Ai[3] * r[0] + Ai[4] * r[1] + Ai[5] * r[2]),
                                       H.z - (Ai[6] * r[0] + Ai[7] * r[1] + Ai[8] * r[2]));
-    double r2[3];
-    const double rn2 = implicit_residual(kind, m, Q, Hq, Hn, mh, r2);
+    V3<double> M2;
+    double D2[9], r2[3];
+    sat_law(kind, m, Hn, mh, M2, D2);
+    const double rn2 = implicit_residual(Q, Hq, Hn, M2, r2);
     if (!(rn2 < rn)) break;
     H = Hn;
+    M = M2;
     rn = rn2;
-    r[0] = r2[0]; r[1] = r2[1]; r[2] = r2[2];
+    for (int a = 0; a < 9; a++) D[a] = D2[a];
+    for (int a = 0; a < 3; a++) r[a] = r2[a];
+  }
+  const double scale = sqrt(Hq.x * Hq.x + Hq.y * Hq.y + Hq.z * Hq.z) + sqrt(M.x * M.x + M.y * M.y + M.z * M.z);
+  ok = rn <= 1e-15 * scale;
+  return H;
+}
+
+// The element's implicit field to rounding.  find_new_h stops after 15 passes
+// of a linearly converging secant, so its H carries an error that changes from
+// one iteration to the next: a Newton iteration on the relaxation as a whole
+// falls back to linear convergence on it, and Anderson mixing stalls (a
+// 12-element saturating hybrid stopped at a misfit of 4e-5 after 2,000 Jacobi
+// iterations).  Polished, the fixed-point map is exact to rounding: the outer
+// Newton converges quadratically and the Jacobi iteration reaches 1e-12 in
+// about a hundred iterations.  The root is unique (-Q is positive
+// semi-definite and the laws are monotone), so Newton starts from the field of
+// the last iteration, which a converging relaxation brings close, and the
+// secant runs only where that does not reach the root: one lane's serial chain
+// of 9,000 instructions an element was half of a relaxation step.
+__device__ __forceinline__ V3<double> solve_h(int kind, const double *m, const double *Q, V3<double> Hq, V3<double> H0,
+                                              double prec_e2, const double *__restrict__ mh)
+{
+  if (kind == RADB200_MAT_LINEAR) return find_new_h(kind, m, Q, Hq, H0, prec_e2, mh);
+  bool ok = false;
+  V3<double> H = H0;
+  for (int pass = 0; pass < 2 && !ok; pass++) {
+    if (pass) H = find_new_h(kind, m, Q, Hq, H0, prec_e2, mh);
+    H = polish_h(kind, m, Q, Hq, H, mh, ok);
   }
   return H;
 }

@@ -150,7 +150,7 @@ __device__ void and_decide(AndState &s, double m)
   s.have_prev = 1;
 }
 
-// One Jacobi proposal: H = N M + H_ext; per element H' = FindNewH(H - Q_ii M),
+// One Jacobi proposal: H = N M + H_ext; per element H' = solve_h(H - Q_ii M),
 // M' = M(H'); writes Mp, Hn, F = M' - M; the last CTA sums |F|^2 (per-CTA
 // partial sums in a fixed order) into sum[0] and, with an Anderson state,
 // settles what the step means for the iteration (and_decide).  A step after
@@ -158,15 +158,19 @@ __device__ void and_decide(AndState &s, double m)
 // N holds n rows, or the rows of elements e0 .. e0 + n - 1 of a row block
 // (hext, kind, mat, Hn, Mp, F then hold those rows; M is always the full
 // magnetization).
+// 4 CTAs per SM (64 registers, the material's serial part spills): 32 warps
+// stream while others solve.  3,936 saturating elements with 4 images, 0.56 GB
+// of matrix: 0.145 ms a step of the iteration, 0.16 at 2 CTAs, 0.18 at 3; 0.205
+// with the secant solve on every step (HBM alone: 0.086).
 template <typename MT>
-__global__ void __launch_bounds__(32 * RLX_WARPS) jacobi_kernel(const MT *__restrict__ N, int ld, int n,
+__global__ void __launch_bounds__(32 * RLX_WARPS, 4) jacobi_kernel(const MT *__restrict__ N, int ld, int n,
                                                                const double *__restrict__ M, const double *__restrict__ hext,
                                                                const int *__restrict__ kind, const double *__restrict__ mat,
                                                                const double *__restrict__ mh,
                                                                double prec_e2, double *__restrict__ Hn,
                                                                double *__restrict__ Mp, double *__restrict__ F,
-                                                               double *__restrict__ part, NearView nv, int exact,
-                                                               int e0, double *__restrict__ sum,
+                                                               double *__restrict__ part, NearView nv, int e0,
+                                                               double *__restrict__ sum,
                                                                unsigned *__restrict__ count, AndState *as)
 {
   __shared__ double ssq[32 * RLX_WARPS];
@@ -192,8 +196,7 @@ __global__ void __launch_bounds__(32 * RLX_WARPS) jacobi_kernel(const MT *__rest
       int k = kind[e];
       const double *mr = mat + (size_t)e * RADB200_MAT_STRIDE;
       V3<double> H0 = mk3<double>(Hn[3 * e], Hn[3 * e + 1], Hn[3 * e + 2]);
-      V3<double> H = find_new_h(k, mr, Q, Hq, H0, prec_e2, mh);
-      if (exact) H = polish_h(k, mr, Q, Hq, H, mh);
+      const V3<double> H = solve_h(k, mr, Q, Hq, H0, prec_e2, mh);
       V3<double> Mn = mat_M(k, mr, H, mh);
       Hn[3 * e] = H.x; Hn[3 * e + 1] = H.y; Hn[3 * e + 2] = H.z;
       Mp[3 * e] = Mn.x; Mp[3 * e + 1] = Mn.y; Mp[3 * e + 2] = Mn.z;
@@ -344,10 +347,8 @@ struct Ctx {
 
 static int grid_elems(int n) { return (n + RLX_WARPS - 1) / RLX_WARPS; }
 
-// one step on the stream; exact: polish each element's implicit field
-// (polish_h) -- the map the Newton relaxation differentiates; as: the Anderson
-// state, or null
-static int jacobi_enqueue(Intrc &I, Ctx &c, double prec_e2, int exact, AndState *as)
+// one step on the stream; as: the Anderson state, or null
+static int jacobi_enqueue(Intrc &I, Ctx &c, double prec_e2, AndState *as)
 {
   const int nb = grid_elems(I.n);
   RB_TRY(c.part.alloc((size_t)nb * sizeof(double)));
@@ -355,16 +356,16 @@ static int jacobi_enqueue(Intrc &I, Ctx &c, double prec_e2, int exact, AndState 
   auto go = [&](auto *N) -> int {
     jacobi_kernel<<<nb, 32 * RLX_WARPS, 0, c.st>>>(N, I.ld, I.n, I.M.as<double>(), I.hext.as<double>(), I.mat_kind.as<int>(),
                                                    I.mat.as<double>(), I.mh.as<double>(), prec_e2, I.H.as<double>(),
-                                                   I.Mp.as<double>(), I.F.as<double>(), c.part.as<double>(), I.near(), exact,
-                                                   0, c.scal.as<double>(), c.count(), as);
+                                                   I.Mp.as<double>(), I.F.as<double>(), c.part.as<double>(), I.near(), 0,
+                                                   c.scal.as<double>(), c.count(), as);
     return check_launch("jacobi_kernel");
   };
   return I.N64.p ? go((const double *)I.N64.p) : go((const float *)I.N32.p);
 }
 
-static int jacobi_step(Intrc &I, Ctx &c, double prec_e2, double *misfit, int exact)
+static int jacobi_step(Intrc &I, Ctx &c, double prec_e2, double *misfit)
 {
-  RB_TRY(jacobi_enqueue(I, c, prec_e2, exact, nullptr));
+  RB_TRY(jacobi_enqueue(I, c, prec_e2, nullptr));
   double s;
   RB_CUDA(cudaMemcpyAsync(&s, c.scal.as<double>(), sizeof(double), cudaMemcpyDeviceToHost, c.st));
   RB_CUDA(cudaStreamSynchronize(c.st));
@@ -568,7 +569,7 @@ int relax_jacobi(Intrc &I, double prec, int max_iter, double omega0, double *sta
     if (h.it > 1) need = h.misfit < h.first ? ceil(log(h.misfit / prec) / log(h.first / h.misfit) * (h.it - 1)) : 8.0;
     batch = std::min((int)std::min(std::max(need, 1.0), 32.0), left);
     for (int k = 0; k < batch; k++) {
-      RB_TRY(jacobi_enqueue(I, c, loc_prec_e2, 1, as));
+      RB_TRY(jacobi_enqueue(I, c, loc_prec_e2, as));
       anderson_diff_kernel<<<nb, AND_T, 0, c.st>>>(I.M.as<double>(), I.F.as<double>(), Xprev, Fprev, dX, dF, n3, I.ld,
                                                    ab.as<double>(), as);
       RB_TRY(check_launch("anderson_diff_kernel"));
@@ -694,7 +695,7 @@ int relax_newton(Intrc &I, double prec, int max_iter, double *status)
   double *d = buf.as<double>(), *tmp = d + ld, *M0 = tmp + ld, *R0 = M0 + ld, *B = R0 + ld;
   double *M = I.M.as<double>();
   const double loc = prec * prec / n;
-  auto step = [&](double *mis) -> int { return jacobi_step(I, c, loc, mis, 1); };
+  auto step = [&](double *mis) -> int { return jacobi_step(I, c, loc, mis); };
   double misfit;
   RB_TRY(step(&misfit));
   int matvecs = 1, newton = 0;
@@ -765,12 +766,12 @@ int relax_rows_step(Intrc &I, const double *M, double prec, double *Mp, double *
   if (I.N64.p)
     jacobi_kernel<double><<<nb, 32 * RLX_WARPS, 0, c.st>>>(I.N64.as<double>(), I.ld, I.nr, M, I.hext.as<double>(), kind, mat,
                                                            I.mh.as<double>(), loc, I.H.as<double>(), Mp, F,
-                                                           c.part.as<double>(), NearView(), 1, I.e0,
+                                                           c.part.as<double>(), NearView(), I.e0,
                                                            c.scal.as<double>(), c.count(), nullptr);
   else
     jacobi_kernel<float><<<nb, 32 * RLX_WARPS, 0, c.st>>>(I.N32.as<float>(), I.ld, I.nr, M, I.hext.as<double>(), kind, mat,
                                                           I.mh.as<double>(), loc, I.H.as<double>(), Mp, F,
-                                                          c.part.as<double>(), NearView(), 1, I.e0,
+                                                          c.part.as<double>(), NearView(), I.e0,
                                                            c.scal.as<double>(), c.count(), nullptr);
   RB_TRY(check_launch("jacobi_kernel"));
   RB_CUDA(cudaMemcpyAsync(sq_sum, c.scal.as<double>(), sizeof(double), cudaMemcpyDeviceToHost, c.st));

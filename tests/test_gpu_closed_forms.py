@@ -212,3 +212,61 @@ def test_polyhedra_by_faces(cuda, rad, shape):
     P = np.array([V[F[0]].mean(0), 0.5 * (V[F[0][0]] + V[F[0][1]]), V[0]])
     assert np.all(np.isfinite(rad.Fld(obj, "b", P)))
     rad.FldLenRndSw("off")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntets,npts", [(1, 1), (31, 130), (32, 32767), (33, 32768), (65, 33001)])
+def test_tetrahedra_with_fp32_terms(cuda, rad, ntets, npts):
+    """Near and far pairs, tiles of 32 tetrahedra, point sets just below and
+    above the size that is put in Morton order.  An FP32 term is off by a few
+    units of 6e-8 and a distant tetrahedron's terms cancel by (R / l)^2, 400
+    at the far corner of this box: 5e-5 of the field, the bar of the FP32
+    option for polyhedra."""
+    rng = np.random.default_rng(npts)
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    faces = [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]]
+    base = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
+    V = [1.2 * np.array([k % 5, (k // 5) % 5, k // 25]) + base + rng.uniform(-0.1, 0.1, (4, 3)) for k in range(ntets)]
+    obj = rad.ObjCnt([rad.ObjPolyhdr(v, faces, m) for v, m in zip(V, rng.normal(size=(ntets, 3)) + [0, 0, 3.0])])
+    P = rng.uniform(-6, 14, size=(npts, 3))
+    b64 = rad.Fld(obj, "b", P, precision="fast")
+    b32 = rad.Fld(obj, "b", P, precision="single")
+    far = np.array([min(np.linalg.norm(p - v.mean(0)) for v in V) > 1.0 for p in P[:2000]])
+    d = np.linalg.norm(b32 - b64, axis=1)[:2000][far]
+    assert np.all(d <= 5e-5 * np.maximum(np.linalg.norm(b64, axis=1)[:2000][far], 1e-5))
+    assert np.linalg.norm((b32 - b64)[:2000][far]) <= 2e-6 * np.linalg.norm(b64[:2000][far])
+    # the order of the points does not matter to a point (sums over chunks of
+    # tetrahedra differ by FP64 rounding), nor do points that are not numbers
+    sub = rad.Fld(obj, "b", np.ascontiguousarray(P[::7]), precision="single")
+    assert np.abs(sub - b32[::7]).max() <= 1e-13 * np.abs(b32).max()
+    Q = P.copy()
+    Q[0] = np.nan
+    assert np.array_equal(rad.Fld(obj, "b", Q, precision="single")[1:], b32[1:])
+    assert np.array_equal(rad.Fld(obj, "m", P[:500], precision="single"), rad.Fld(obj, "m", P[:500]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 18, 19, 37, 74, 149])
+def test_trajectories_do_not_depend_on_their_number(cuda, rad, n):
+    """Clusters of 8, 4, 2 and 1 CTAs by the number of trajectories: the same
+    rows bit for bit as one alone, coils (arc nodes, current blocks) included."""
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    rng = np.random.default_rng(1)
+    blocks = [rad.ObjRecMag([4.0 * i - 60, 0.3, 20.0 + 0.1 * i], [3.0, 30.0, 5.0], rng.normal(size=3).tolist())
+              for i in range(30)]
+    yoke = rad.ObjCnt(blocks)
+    rad.TrfZerPerp(yoke, [0, 0, 0], [1, 0, 0])
+    rad.TrfZerPara(yoke, [0, 0, 0], [0, 0, 1])
+    tet = rad.ObjPolyhdr([[70, 0, 5], [75, 1, 5], [71, 6, 5], [72, 2, 11]], [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]],
+                         [0.2, 0.3, 0.9])
+    obj = rad.ObjCnt([yoke, tet, rad.ObjRaceTrk([0.1, 0.2, 30.3], [2, 22], [60, 80], 30, 6, 15.0, "man", "z")])
+    init = rng.uniform([-3, -2e-3, -3, -2e-3], [3, 2e-3, 3, 2e-3], size=(n, 4))
+    batch = rad.FldPtcTrj(obj, 0.3, init, [-60, 59.5], 12)
+    for k in (0, n - 1):
+        assert np.array_equal(batch[k], np.array(rad.FldPtcTrj(obj, 0.3, init[k], [-60, 59.5], 12)))
+    # the same field as the field kernels', through one slope
+    P = np.array([init[0, 0], -60.0, init[0, 2]])
+    assert np.abs(np.array(rad.Fld(obj, "b", P.tolist())) - O.field(model.pack_sources(rad._objs, obj, tuple(rad._rand)),
+                                                                   P[None], 0)[0]).max() < 1e-10

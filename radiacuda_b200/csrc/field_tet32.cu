@@ -1,0 +1,356 @@
+// field_tet32.cu -- field of an all-tetrahedron model with FP32 terms.
+//
+// The vertex/edge form of tet_fast (formulas.cuh): vertex offsets formed in
+// FP64 and rounded to FP32; distances, edge integrals and solid angles in
+// FP32; weights and sums in FP64.  Bound by instruction issue: the library's
+// log1pf, atan2f, division and square root made 793 thread-instructions a
+// pair.  Most pairs are distant, and there each element is short:
+//   L / 2 = artanh(x),   x = l / (Ra + Rb) <= 1/6:    a quotient, 3 terms;
+//   half solid angle = arctan(num / den) <= 0.025:     a quotient, 2 terms,
+// when the point is at least 4 times the longest edge from vertex 0 (every
+// distance is then at least 3 of them).  This L has less error than the
+// log1pf form (2-norm of B against FP64 on 3,000 tetrahedra 1.9e-7 against
+// 2.6e-7): it takes the exact length and two distances, no dot product.
+// Nearer pairs take the log1pf and atan2f forms.  A warp pays for the longer
+// path when any of its lanes needs it, so larger point sets are first put in
+// Morton order; each point's sum runs over the tetrahedra in their own order
+// either way.
+#include <cub/device/device_radix_sort.cuh>
+
+#include <algorithm>
+
+#include "internal.cuh"
+
+namespace rb {
+
+namespace {
+
+constexpr int T32_TILE = 32;
+constexpr int T32_D = 66;  // doubles per unit: v (12), 2 C a_f (12), 2 C g_e (18), point map (12), field map (9), M (3)
+constexpr int T32_F = 20;  // floats per unit: edge lengths (6), face normals m (12), (4 longest edge)^2, 1 if both maps are diagonal
+
+__device__ __forceinline__ float rcp32(float d)
+{
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+  return y;
+}
+// n / d by the approximate reciprocal and one Newton correction of the quotient
+__device__ __forceinline__ float quot32(float n, float d)
+{
+  const float y = rcp32(d), q = n * y;
+  return fmaf(fmaf(-d, q, n), y, q);
+}
+// sqrt by the approximate reciprocal root and one Newton correction
+__device__ __forceinline__ float root32(float s)
+{
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+  const float g = s * y;
+  return fmaf(0.5f * y, fmaf(-g, g, s), g);
+}
+
+struct D3 {
+  double x, y, z;
+};
+
+// one pair: acc += its B or H in the lab frame
+__device__ __forceinline__ void tet32_pair(const double *__restrict__ sd, const float *__restrict__ sf, D3 P, int what,
+                                           double *acc)
+{
+  const double *T = sd + 42, *F = sd + 54;
+  const bool diag = sf[19] != 0.f;
+  const double dx = P.x - T[9], dy = P.y - T[10], dz = P.z - T[11];
+  double qx, qy, qz;
+  if (diag) {
+    qx = T[0] * dx;
+    qy = T[4] * dy;
+    qz = T[8] * dz;
+  } else {
+    qx = T[0] * dx + T[1] * dy + T[2] * dz;
+    qy = T[3] * dx + T[4] * dy + T[5] * dz;
+    qz = T[6] * dx + T[7] * dy + T[8] * dz;
+  }
+  float rx[4], ry[4], rz[4], R[4], d[6];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    rx[k] = (float)(sd[3 * k] - qx);
+    ry[k] = (float)(sd[3 * k + 1] - qy);
+    rz[k] = (float)(sd[3 * k + 2] - qz);
+    R[k] = fmaf(rx[k], rx[k], fmaf(ry[k], ry[k], rz[k] * rz[k]));
+  }
+  const bool far = R[0] >= sf[18];
+#pragma unroll
+  for (int e = 0; e < 6; e++) {
+    const int a = tet_edge_a(e), b = tet_edge_b(e);
+    d[e] = fmaf(rx[a], rx[b], fmaf(ry[a], ry[b], rz[a] * rz[b]));
+  }
+  double h0 = 0.0, h1 = 0.0, h2 = 0.0;
+  bool inside = false;
+  auto edge_add = [&](int e, float half_L) {
+    const double L = (double)half_L;
+    h0 = fma(L, sd[24 + 3 * e], h0);
+    h1 = fma(L, sd[25 + 3 * e], h1);
+    h2 = fma(L, sd[26 + 3 * e], h2);
+  };
+  auto face_add = [&](int f, float half_omega) {
+    const double w = (double)half_omega;
+    h0 = fma(w, sd[12 + 3 * f], h0);
+    h1 = fma(w, sd[13 + 3 * f], h1);
+    h2 = fma(w, sd[14 + 3 * f], h2);
+  };
+  if (far) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) R[k] = root32(R[k]);
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      const float x = quot32(sf[e], R[tet_edge_a(e)] + R[tet_edge_b(e)]), z = x * x;
+      // artanh(x) = x (1 + z p(z)), least maximum error 2.3e-9 for z <= 1/36
+      const float p = fmaf(fmaf(0.1477081972f, z, 0.1999480270f), z, 0.3333334154f);
+      edge_add(e, fmaf(x * z, p, x));
+    }
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const int a = tet_face_a(f), b = tet_face_b(f), c = tet_face_c(f);
+      const float num = fmaf(rx[a], sf[6 + 3 * f], fmaf(ry[a], sf[7 + 3 * f], rz[a] * sf[8 + 3 * f]));
+      const float den = fmaf(fmaf(R[a], R[b], d[tet_pair(a, b)]), R[c], fmaf(d[tet_pair(a, c)], R[b], d[tet_pair(b, c)] * R[a]));
+      const float w = quot32(-num, den), u = w * w;
+      // arctan(w) = w (1 + u p(u)), least maximum error 3e-11 for u <= 0.0012
+      face_add(f, fmaf(w * u, fmaf(0.1998287159f, u, -0.3333333076f), w));
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) R[k] = sqrtf(R[k]);
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+      const int a = tet_edge_a(e), b = tet_edge_b(e);
+      edge_add(e, 0.5f * edge_L(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b], d[e], sf[e]));
+    }
+    double total = 0.0;
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const int a = tet_face_a(f), b = tet_face_b(f), c = tet_face_c(f);
+      const float num = rx[a] * sf[6 + 3 * f] + ry[a] * sf[7 + 3 * f] + rz[a] * sf[8 + 3 * f];
+      const float den = R[a] * R[b] * R[c] + d[tet_pair(a, b)] * R[c] + d[tet_pair(a, c)] * R[b] + d[tet_pair(b, c)] * R[a];
+      const float w = atan2f(-num, den);
+      total += (double)w;
+      face_add(f, w);
+    }
+    inside = total < -3.141592653589793;
+  }
+  if (what == 2) h0 = h1 = h2 = 0.0;
+  if (what != 1 && inside) {
+    h0 += sd[63];
+    h1 += sd[64];
+    h2 += sd[65];
+  }
+  if (diag) {
+    acc[0] = fma(F[0], h0, acc[0]);
+    acc[1] = fma(F[4], h1, acc[1]);
+    acc[2] = fma(F[8], h2, acc[2]);
+  } else {
+    acc[0] += F[0] * h0 + F[1] * h1 + F[2] * h2;
+    acc[1] += F[3] * h0 + F[4] * h1 + F[5] * h2;
+    acc[2] += F[6] * h0 + F[7] * h1 + F[8] * h2;
+  }
+}
+
+// PPT points per thread; perm: the order of the points (null: as they are)
+template <int PPT>
+__global__ void __launch_bounds__(128) field_tet32_kernel(GeomView g, const double *__restrict__ pts, int64_t npts,
+                                                          const unsigned *__restrict__ perm, int what,
+                                                          double *__restrict__ out, int ub, int ue, int chunk, int accumulate)
+{
+  __shared__ __align__(16) double sd[T32_TILE * T32_D];
+  __shared__ __align__(16) float sf[T32_TILE * T32_F];
+  const int tid = threadIdx.x;
+  const int u0 = ub + blockIdx.y * chunk, u1 = min(ue, u0 + chunk);
+  int64_t idx[PPT];
+  D3 P[PPT];
+  double acc[PPT][3];
+#pragma unroll
+  for (int p = 0; p < PPT; p++) {
+    const int64_t i = (int64_t)blockIdx.x * (128 * PPT) + p * 128 + tid;
+    idx[p] = i < npts ? (perm ? (int64_t)perm[i] : i) : -1;
+    P[p] = D3{0, 0, 0};
+    if (idx[p] >= 0) P[p] = D3{pts[3 * idx[p]], pts[3 * idx[p] + 1], pts[3 * idx[p] + 2]};
+    acc[p][0] = acc[p][1] = acc[p][2] = 0.0;
+  }
+  const double C2 = 2.0 / (4.0 * 3.141592653589793238);
+  for (int base = u0; base < u1; base += T32_TILE) {
+    const int cnt = min(T32_TILE, u1 - base);
+    __syncthreads();
+    for (int e = tid; e < cnt * T32_D; e += 128) {
+      const int k = e / T32_D, f = e - k * T32_D;
+      const int4 un = __ldg(g.units + base + k);  // {kind, polyhedron, transform, diagonal point map}
+      const double *rec = g.tetrec + (size_t)__ldg(g.tetidx + un.y) * TET_REC_FIELD;
+      double v;
+      if (f < 12) v = __ldg(rec + f);
+      else if (f < 42) v = C2 * __ldg(rec + 18 + f);  // a_f from 30, g_e from 42
+      else if (f < 63) v = __ldg(g.trf + (size_t)un.z * RADB200_TRF_STRIDE + (f - 42));
+      else v = __ldg(g.poly + (size_t)un.y * RADB200_POLY_STRIDE + 3 + (f - 63));
+      sd[e] = v;
+    }
+    for (int e = tid; e < cnt * T32_F; e += 128) {
+      const int k = e / T32_F, f = e - k * T32_F;
+      const int4 un = __ldg(g.units + base + k);
+      const double *rec = g.tetrec + (size_t)__ldg(g.tetidx + un.y) * TET_REC_FIELD + 12;  // lengths, then normals
+      float v;
+      if (f < 18) v = (float)__ldg(rec + f);
+      else if (f == 18) {
+        double m = 0.0;
+        for (int q = 0; q < 6; q++) m = fmax(m, __ldg(rec + q));
+        v = (float)(16.0 * m * m);
+      } else {
+        const double *F = g.trf + (size_t)un.z * RADB200_TRF_STRIDE + 12;
+        v = un.w && F[1] == 0.0 && F[2] == 0.0 && F[3] == 0.0 && F[5] == 0.0 && F[6] == 0.0 && F[7] == 0.0 ? 1.f : 0.f;
+      }
+      sf[e] = v;
+    }
+    __syncthreads();
+    for (int k = 0; k < cnt; k++)
+#pragma unroll
+      for (int p = 0; p < PPT; p++) tet32_pair(sd + k * T32_D, sf + k * T32_F, P[p], what, acc[p]);
+  }
+#pragma unroll
+  for (int p = 0; p < PPT; p++)
+    if (idx[p] >= 0) {
+      double *o = out + ((size_t)blockIdx.y * npts + idx[p]) * 3;
+#pragma unroll
+      for (int c = 0; c < 3; c++) o[c] = accumulate ? o[c] + acc[p][c] : acc[p][c];
+    }
+}
+
+// floats in an order that unsigned integers share
+__device__ __forceinline__ unsigned ordered(float x)
+{
+  const unsigned u = __float_as_uint(x);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float unordered(unsigned u)
+{
+  return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
+}
+
+// box[0..2] the smallest, box[3..5] the largest coordinates (ordered bits)
+__global__ void point_box_kernel(const double *__restrict__ pts, int64_t n, unsigned *__restrict__ box)
+{
+  unsigned lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0, 0, 0};
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    for (int c = 0; c < 3; c++) {
+      const float x = (float)pts[3 * i + c];
+      if (!isfinite(x)) continue;
+      lo[c] = min(lo[c], ordered(x));
+      hi[c] = max(hi[c], ordered(x));
+    }
+  for (int c = 0; c < 3; c++) {
+    lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
+    hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(box + c, lo[c]);
+      atomicMax(box + 3 + c, hi[c]);
+    }
+  }
+}
+
+__device__ __forceinline__ unsigned spread3(unsigned x)
+{
+  x = (x | (x << 16)) & 0x030000FF;
+  x = (x | (x << 8)) & 0x0300F00F;
+  x = (x | (x << 4)) & 0x030C30C3;
+  return (x | (x << 2)) & 0x09249249;
+}
+
+__global__ void point_key_kernel(const double *__restrict__ pts, int64_t n, const unsigned *__restrict__ box,
+                                 unsigned *__restrict__ key, unsigned *__restrict__ idx)
+{
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  float ext = 0.f, lo[3];
+  for (int c = 0; c < 3; c++) {
+    lo[c] = unordered(box[c]);
+    ext = fmaxf(ext, unordered(box[3 + c]) - lo[c]);
+  }
+  unsigned k = 0;
+  for (int c = 0; c < 3; c++) {
+    const float t = ((float)pts[3 * i + c] - lo[c]) / ext * 1023.f;
+    k |= spread3(t > 0.f ? min((unsigned)t, 1023u) : 0u) << c;  // NaN: 0
+  }
+  key[i] = k;
+  idx[i] = (unsigned)i;
+}
+
+__global__ void tet32_reduce_kernel(const double *__restrict__ part, int nc, int64_t n3, double *__restrict__ out, int accumulate)
+{
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n3) return;
+  double s = accumulate ? out[i] : 0.0;
+  for (int c = 0; c < nc; c++) s += part[(size_t)c * n3 + i];
+  out[i] = s;
+}
+
+// The Morton order of the points into perm.buf; scratch from the block pool
+struct PointOrder {
+  DBuf box, key, key2, idx, idx2, tmp;
+  const unsigned *perm = nullptr;
+  int build(const double *d_pts, int64_t n, cudaStream_t st)
+  {
+    const unsigned init[6] = {~0u, ~0u, ~0u, 0, 0, 0};
+    RB_TRY(box.upload(init, sizeof(init)));
+    for (DBuf *b : {&key, &key2, &idx, &idx2}) RB_TRY(b->alloc((size_t)n * sizeof(unsigned)));
+    point_box_kernel<<<148 * 2, 256, 0, st>>>(d_pts, n, box.as<unsigned>());
+    RB_TRY(check_launch("point_box_kernel"));
+    point_key_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_pts, n, box.as<unsigned>(), key.as<unsigned>(),
+                                                                  idx.as<unsigned>());
+    RB_TRY(check_launch("point_key_kernel"));
+    size_t bytes = 0;
+    RB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, key.as<unsigned>(), key2.as<unsigned>(), idx.as<unsigned>(),
+                                            idx2.as<unsigned>(), (int)n, 0, 30, st));
+    RB_TRY(tmp.alloc(bytes));
+    RB_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, key.as<unsigned>(), key2.as<unsigned>(), idx.as<unsigned>(),
+                                            idx2.as<unsigned>(), (int)n, 0, 30, st));
+    perm = idx2.as<unsigned>();
+    return 0;
+  }
+};
+
+template <int PPT>
+int launch_ppt(const GeomView &g, const double *d_pts, int64_t npts, const unsigned *perm, int what, double *d_out, int ub,
+               int ue, int accumulate, DBuf &scratch, cudaStream_t st)
+{
+  const int64_t nblk = (npts + 128 * PPT - 1) / (128 * PPT);
+  const int nu = ue - ub;
+  // too few points for the GPU: split the tetrahedra as well
+  const int64_t target = 148 * 6;
+  int nchunk = nblk < target ? (int)((target + nblk - 1) / nblk) : 1;
+  nchunk = std::min(std::min(nchunk, nu), 65535);
+  const int chunk = (nu + nchunk - 1) / nchunk;
+  nchunk = (nu + chunk - 1) / chunk;
+  double *dst = d_out;
+  if (nchunk > 1) {
+    RB_TRY(scratch.alloc((size_t)nchunk * npts * 3 * sizeof(double)));
+    dst = scratch.as<double>();
+  }
+  field_tet32_kernel<PPT><<<dim3((unsigned)nblk, (unsigned)nchunk), 128, 0, st>>>(g, d_pts, npts, perm, what, dst, ub, ue, chunk,
+                                                                                 nchunk > 1 ? 0 : accumulate);
+  RB_TRY(check_launch("field_tet32_kernel"));
+  if (nchunk == 1) return 0;
+  const int64_t n3 = npts * 3;
+  tet32_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(scratch.as<double>(), nchunk, n3, d_out, accumulate);
+  return check_launch("tet32_reduce_kernel");
+}
+
+}  // namespace
+
+#ifndef T32_PPT
+#define T32_PPT 1
+#endif
+int launch_tet32_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int ub, int ue,
+                       int accumulate, DBuf &scratch, cudaStream_t st)
+{
+  PointOrder order;
+  if (npts >= T32_SORT_MIN && npts <= INT32_MAX) RB_TRY(order.build(d_pts, npts, st));
+  return launch_ppt<T32_PPT>(g, d_pts, npts, order.perm, what, d_out, ub, ue, accumulate, scratch, st);
+}
+
+}  // namespace rb

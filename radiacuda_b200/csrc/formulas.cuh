@@ -49,18 +49,6 @@ template <typename T> __device__ __forceinline__ T trans_atans(T x, T y, T &pimu
   return (x + y) / buf;
 }
 
-// Sum of four arctangents with branch bookkeeping, as the cuboid formula
-// evaluates T0/T1 components (radrec.cpp:117-128).
-template <typename T> __device__ __forceinline__ T atan4(T a, T b, T c, T d)
-{
-  const T Pi = T(3.141592653589793238);
-  T p1, p2, p3;
-  T u = trans_atans(a, b, p1);
-  T v = trans_atans(c, d, p2);
-  T w = trans_atans(u, v, p3);
-  return atanT(w) + Pi * (p1 + p2 + p3);
-}
-
 // ---- cuboid -------------------------------------------------------------------
 // Q of a uniformly magnetized cuboid (radrec.cpp:115-283) at q from its centre:
 //   4 pi Tx = sum of 8 arctan(+-y_j z_k / (x_i D_ijk)),
@@ -84,31 +72,43 @@ template <typename T> __device__ __forceinline__ T atan4(T a, T b, T c, T d)
 //   - the third diagonal entry is what the trace leaves: 0 outside, -1 inside.
 // elem64.cuh has the square root, arctangent and logarithm.
 
-// one axis: T of the faces at a0 and a1 (offsets along the axis), p_jk the
-// products of the other two offsets, D_jk the distances of the corners;
-// inner: the point projects into the faces
+// The product of one face's four numbers: offset a along the axis, p_jk the
+// products of the other two offsets, u = p00 p01, v = p10 p11, D_jk the
+// distances of its corners
+RB_HD void cuboid_face(double a, double p00, double p01, double p10, double p11, double u, double v, double D00, double D01,
+                       double D10, double D11, double &re, double &im)
+{
+  const double r0 = a * D00, r1 = a * D01, r2 = a * D10, r3 = a * D11;
+  const double e0 = fma(r0, r1, u), f0 = fma(p00, r1, -(r0 * p01));
+  const double e1 = fma(r2, r3, v), f1 = fma(r2, p11, -(p10 * r3));
+  re = fma(e0, e1, -(f0 * f1));
+  im = fma(e0, f1, f0 * e1);
+}
+// The face's angle by quadrant, in units of pi/4 (the centre), with the sign of
+// its offset a, which the product carries; inner: the point projects into it
+RB_HD int cuboid_face_quadrant(double a, double re, double im, bool inner)
+{
+  const int s = hi32(a);
+  const int c = hi32(re) < 0 ? ((hi32(im) ^ s) < 0 ? 5 : 3) : ((hi32(im) ^ s) < 0 ? (inner ? 7 : -1) : 1);
+  return s < 0 ? -c : c;
+}
+RB_HD int plain_quadrant(double re, double im)
+{
+  return hi32(re) < 0 ? (hi32(im) < 0 ? -3 : 3) : (hi32(im) < 0 ? -1 : 1);
+}
+
+// one axis: T of the faces at a0 and a1
 RB_HD double cuboid_axis_T(double a0, double a1, double p00, double p01, double p10, double p11, double D000,
                            double D001, double D010, double D011, double D100, double D101, double D110, double D111,
                            bool inner)
 {
   const double u = p00 * p01, v = p10 * p11;
-  const double r0 = a0 * D000, r1 = a0 * D001, r2 = a0 * D010, r3 = a0 * D011;
-  const double e0 = fma(r0, r1, u), f0 = fma(p00, r1, -(r0 * p01));
-  const double e1 = fma(r2, r3, v), f1 = fma(r2, p11, -(p10 * r3));
-  const double re0 = fma(e0, e1, -(f0 * f1)), im0 = fma(e0, f1, f0 * e1);
-  const double t0 = a1 * D100, t1 = a1 * D101, t2 = a1 * D110, t3 = a1 * D111;
-  const double g0 = fma(t0, t1, u), h0 = fma(p00, t1, -(t0 * p01));
-  const double g1 = fma(t2, t3, v), h1 = fma(t2, p11, -(p10 * t3));
-  const double re1 = fma(g0, g1, -(h0 * h1)), im1 = fma(g0, h1, h0 * g1);
+  double re0, im0, re1, im1;
+  cuboid_face(a0, p00, p01, p10, p11, u, v, D000, D001, D010, D011, re0, im0);
+  cuboid_face(a1, p00, p01, p10, p11, u, v, D100, D101, D110, D111, re1, im1);
   const double re = fma(re0, re1, im0 * im1), im = fma(im0, re1, -(re0 * im1));
-  // quadrant centres in units of pi/4; s: sign of the offset, which the products carry
-  const int s0 = hi32(a0), s1 = hi32(a1);
-  const int last = inner ? 7 : -1;
-  const int c0 = hi32(re0) < 0 ? ((hi32(im0) ^ s0) < 0 ? 5 : 3) : ((hi32(im0) ^ s0) < 0 ? last : 1);
-  const int c1 = hi32(re1) < 0 ? ((hi32(im1) ^ s1) < 0 ? 5 : 3) : ((hi32(im1) ^ s1) < 0 ? last : 1);
-  const int c = hi32(re) < 0 ? (hi32(im) < 0 ? -3 : 3) : (hi32(im) < 0 ? -1 : 1);
-  const int turns = ((s0 < 0 ? -c0 : c0) - (s1 < 0 ? -c1 : c1) - c + 4) >> 3;
-  return angle64(im, re, turns);
+  const int c0 = cuboid_face_quadrant(a0, re0, im0, inner), c1 = cuboid_face_quadrant(a1, re1, im1, inner);
+  return angle64(im, re, (c0 - c1 - plain_quadrant(re, im) + 4) >> 3);
 }
 
 // one axis: the logarithm of S.  b_ijk = |a_k| + D of the corners, the axis's
@@ -220,61 +220,67 @@ __device__ __forceinline__ int cuboid_TS(V3<double> q, V3<double> hd, const Guar
   return in;
 }
 
+// x0 T0 + x1 T1 of one axis: the faces' own angles, weighted by their offsets
+RB_HD double cuboid_axis_xT(double a0, double a1, double p00, double p01, double p10, double p11, double D000, double D001,
+                            double D010, double D011, double D100, double D101, double D110, double D111, bool inner)
+{
+  const double u = p00 * p01, v = p10 * p11;
+  double re, im;
+  cuboid_face(a0, p00, p01, p10, p11, u, v, D000, D001, D010, D011, re, im);
+  const double t0 = angle64(im, re, (cuboid_face_quadrant(a0, re, im, inner) - plain_quadrant(re, im) + 4) >> 3);
+  cuboid_face(a1, p00, p01, p10, p11, u, v, D100, D101, D110, D111, re, im);
+  const double t1 = angle64(im, re, (cuboid_face_quadrant(a1, re, im, inner) - plain_quadrant(re, im) + 4) >> 3);
+  return fma(a0, t0, -(a1 * t1));
+}
+// log((z0 + D0) / (z1 + D1)) along an edge at rho^2 from the point's axis, from
+// b = |z| + D (a sum with z < 0 is rho^2 / b)
+RB_HD double cuboid_edge_L(double b0, double b1, double rho2, bool mixed, bool neg)
+{
+  return log_ratio64(mixed ? rho2 : (neg ? b1 : b0), mixed ? b0 * b1 : (neg ? b0 : b1));
+}
+
 // Field of a current-carrying cuboid (radrec.cpp:183-249, J branch), q
-// relative to the centre, J in A/mm^2; returns B (= H) in T.
+// relative to the centre, J in A/mm^2; returns B (= H) in T.  Single blocks
+// of coils lie on the critical path of a trajectory's field evaluations: with
+// the elements of cuboid_TS, 12 logarithms and 6 arctangents without quotients.
 __device__ __forceinline__ V3<double> cuboid_J(V3<double> q, V3<double> hd, V3<double> J, const Guard &g)
 {
-  typedef double T;
-  T x0 = -q.x - hd.x, x1 = -q.x + hd.x, y0 = -q.y - hd.y, y1 = -q.y + hd.y, z0 = -q.z - hd.z, z1 = -q.z + hd.z;
-  if (x0 == 0.) x0 = abs_rand(g, hd.x);
-  if (x1 == 0.) x1 = abs_rand(g, hd.x);
-  if (y0 == 0.) y0 = abs_rand(g, hd.y);
-  if (y1 == 0.) y1 = abs_rand(g, hd.y);
-  if (z0 == 0.) z0 = abs_rand(g, hd.z);
-  if (z1 == 0.) z1 = abs_rand(g, hd.z);
-  T x0e2 = x0 * x0, x1e2 = x1 * x1, y0e2 = y0 * y0, y1e2 = y1 * y1, z0e2 = z0 * z0, z1e2 = z1 * z1;
-  T D000 = sqrt(x0e2 + y0e2 + z0e2), D100 = sqrt(x1e2 + y0e2 + z0e2), D010 = sqrt(x0e2 + y1e2 + z0e2), D110 = sqrt(x1e2 + y1e2 + z0e2);
-  T D001 = sqrt(x0e2 + y0e2 + z1e2), D101 = sqrt(x1e2 + y0e2 + z1e2), D011 = sqrt(x0e2 + y1e2 + z1e2), D111 = sqrt(x1e2 + y1e2 + z1e2);
-  T T0x = atan4(y0 * z0 / (x0 * D000), -y0 * z1 / (x0 * D001), -y1 * z0 / (x0 * D010), y1 * z1 / (x0 * D011));
-  T T1x = atan4(-y0 * z0 / (x1 * D100), y0 * z1 / (x1 * D101), y1 * z0 / (x1 * D110), -y1 * z1 / (x1 * D111));
-  T T0y = atan4(x0 * z0 / (y0 * D000), -x0 * z1 / (y0 * D001), -x1 * z0 / (y0 * D100), x1 * z1 / (y0 * D101));
-  T T1y = atan4(-x0 * z0 / (y1 * D010), x0 * z1 / (y1 * D011), x1 * z0 / (y1 * D110), -x1 * z1 / (y1 * D111));
-  T T0z = atan4(x0 * y0 / (z0 * D000), -x1 * y0 / (z0 * D100), -x0 * y1 / (z0 * D010), x1 * y1 / (z0 * D110));
-  T T1z = atan4(-x0 * y0 / (z1 * D001), x1 * y0 / (z1 * D101), x0 * y1 / (z1 * D011), -x1 * y1 / (z1 * D111));
-  T R000 = 10. * abs_rand(g, D000), R010 = 10. * abs_rand(g, D010), R001 = 10. * abs_rand(g, D001), R011 = 10. * abs_rand(g, D011);
-  T R100 = 10. * abs_rand(g, D100), R110 = 10. * abs_rand(g, D110), R101 = 10. * abs_rand(g, D101), R111 = 10. * abs_rand(g, D111);
-  T z0pD100 = z0 + D100; if (z0pD100 < R100) z0pD100 = 0.5 * (x1e2 + y0e2) / fabs(z0);
-  T z1pD101 = z1 + D101; if (z1pD101 < R101) z1pD101 = 0.5 * (x1e2 + y0e2) / fabs(z1);
-  T z1pD001 = z1 + D001; if (z1pD001 < R001) z1pD001 = 0.5 * (x0e2 + y0e2) / fabs(z1);
-  T z0pD000 = z0 + D000; if (z0pD000 < R000) z0pD000 = 0.5 * (x0e2 + y0e2) / fabs(z0);
-  T z0pD010 = z0 + D010; if (z0pD010 < R010) z0pD010 = 0.5 * (x0e2 + y1e2) / fabs(z0);
-  T z1pD011 = z1 + D011; if (z1pD011 < R011) z1pD011 = 0.5 * (x0e2 + y1e2) / fabs(z1);
-  T z1pD111 = z1 + D111; if (z1pD111 < R111) z1pD111 = 0.5 * (x1e2 + y1e2) / fabs(z1);
-  T z0pD110 = z0 + D110; if (z0pD110 < R110) z0pD110 = 0.5 * (x1e2 + y1e2) / fabs(z0);
-  T y0pD100 = y0 + D100; if (y0pD100 < R100) y0pD100 = 0.5 * (x1e2 + z0e2) / fabs(y0);
-  T y1pD110 = y1 + D110; if (y1pD110 < R110) y1pD110 = 0.5 * (x1e2 + z0e2) / fabs(y1);
-  T y1pD010 = y1 + D010; if (y1pD010 < R010) y1pD010 = 0.5 * (x0e2 + z0e2) / fabs(y1);
-  T y0pD000 = y0 + D000; if (y0pD000 < R000) y0pD000 = 0.5 * (x0e2 + z0e2) / fabs(y0);
-  T y0pD001 = y0 + D001; if (y0pD001 < R001) y0pD001 = 0.5 * (x0e2 + z1e2) / fabs(y0);
-  T y1pD011 = y1 + D011; if (y1pD011 < R011) y1pD011 = 0.5 * (x0e2 + z1e2) / fabs(y1);
-  T y1pD111 = y1 + D111; if (y1pD111 < R111) y1pD111 = 0.5 * (x1e2 + z1e2) / fabs(y1);
-  T y0pD101 = y0 + D101; if (y0pD101 < R101) y0pD101 = 0.5 * (x1e2 + z1e2) / fabs(y0);
-  T x0pD010 = x0 + D010; if (x0pD010 < R010) x0pD010 = 0.5 * (y1e2 + z0e2) / fabs(x0);
-  T x1pD110 = x1 + D110; if (x1pD110 < R110) x1pD110 = 0.5 * (y1e2 + z0e2) / fabs(x1);
-  T x1pD100 = x1 + D100; if (x1pD100 < R100) x1pD100 = 0.5 * (y0e2 + z0e2) / fabs(x1);
-  T x0pD000 = x0 + D000; if (x0pD000 < R000) x0pD000 = 0.5 * (y0e2 + z0e2) / fabs(x0);
-  T x0pD001 = x0 + D001; if (x0pD001 < R001) x0pD001 = 0.5 * (y0e2 + z1e2) / fabs(x0);
-  T x1pD101 = x1 + D101; if (x1pD101 < R101) x1pD101 = 0.5 * (y0e2 + z1e2) / fabs(x1);
-  T x1pD111 = x1 + D111; if (x1pD111 < R111) x1pD111 = 0.5 * (y1e2 + z1e2) / fabs(x1);
-  T x0pD011 = x0 + D011; if (x0pD011 < R011) x0pD011 = 0.5 * (y1e2 + z1e2) / fabs(x0);
-  T lza = log(z0pD100 / z1pD101), lzb = log(z1pD001 / z0pD000), lzc = log(z0pD010 / z1pD011), lzd = log(z1pD111 / z0pD110);
-  T lya = log(y0pD100 / y1pD110), lyb = log(y1pD010 / y0pD000), lyc = log(y0pD001 / y1pD011), lyd = log(y1pD111 / y0pD101);
-  T lxa = log(x0pD010 / x1pD110), lxb = log(x1pD100 / x0pD000), lxc = log(x0pD001 / x1pD101), lxd = log(x1pD111 / x0pD011);
-  V3<T> bv = mk3<T>(x0 * T0x + x1 * T1x + y0 * (lza + lzb) + y1 * (lzc + lzd) + z0 * (lya + lyb) + z1 * (lyc + lyd),
-                    y0 * T0y + y1 * T1y + x0 * (lzc + lzb) + x1 * (lza + lzd) + z0 * (lxa + lxb) + z1 * (lxc + lxd),
-                    z0 * T0z + z1 * T1z + y0 * (lxc + lxb) + y1 * (lxa + lxd) + x0 * (lyc + lyb) + x1 * (lya + lyd));
-  const T c = 0.0001;
-  return mk3<T>(c * (J.y * bv.z - J.z * bv.y), c * (J.z * bv.x - J.x * bv.z), c * (J.x * bv.y - J.y * bv.x));
+  double x0 = -q.x - hd.x, x1 = -q.x + hd.x, y0 = -q.y - hd.y, y1 = -q.y + hd.y, z0 = -q.z - hd.z, z1 = -q.z + hd.z;
+  int nan = 0;
+  if (x0 == 0. || x1 == 0.) { const double r = abs_rand(g, hd.x); if (x0 == 0.) x0 = r; if (x1 == 0.) x1 = r; nan |= r == 0.; }
+  if (y0 == 0. || y1 == 0.) { const double r = abs_rand(g, hd.y); if (y0 == 0.) y0 = r; if (y1 == 0.) y1 = r; nan |= (r == 0.) << 1; }
+  if (z0 == 0. || z1 == 0.) { const double r = abs_rand(g, hd.z); if (z0 == 0.) z0 = r; if (z1 == 0.) z1 = r; nan |= (r == 0.) << 2; }
+  const bool mx = (hi32(x0) & ~hi32(x1)) < 0, my = (hi32(y0) & ~hi32(y1)) < 0, mz = (hi32(z0) & ~hi32(z1)) < 0;
+  const bool nx = hi32(x0) < 0, ny = hi32(y0) < 0, nz = hi32(z0) < 0;
+  const double xx0 = x0 * x0, xx1 = x1 * x1, yy0 = y0 * y0, yy1 = y1 * y1, zz0 = z0 * z0, zz1 = z1 * z1;
+  const double D000 = sqrt64(xx0 + yy0 + zz0), D001 = sqrt64(xx0 + yy0 + zz1), D010 = sqrt64(xx0 + yy1 + zz0),
+               D011 = sqrt64(xx0 + yy1 + zz1), D100 = sqrt64(xx1 + yy0 + zz0), D101 = sqrt64(xx1 + yy0 + zz1),
+               D110 = sqrt64(xx1 + yy1 + zz0), D111 = sqrt64(xx1 + yy1 + zz1);
+  const double xT = cuboid_axis_xT(x0, x1, y0 * z0, y0 * z1, y1 * z0, y1 * z1, D000, D001, D010, D011, D100, D101, D110, D111, my && mz);
+  const double yT = cuboid_axis_xT(y0, y1, x0 * z0, x0 * z1, x1 * z0, x1 * z1, D000, D001, D100, D101, D010, D011, D110, D111, mx && mz);
+  const double zT = cuboid_axis_xT(z0, z1, x0 * y0, x0 * y1, x1 * y0, x1 * y1, D000, D010, D100, D110, D001, D011, D101, D111, mx && my);
+  const bool near = g.absr > 0.0 && fmin(fmin(fmin(D000, D001), fmin(D010, D011)), fmin(fmin(D100, D101), fmin(D110, D111))) < 10.0 * g.absr;
+  auto b = [&](double z, double D, double rho2) { return near ? cuboid_guard_b(g, z, D, rho2) : fabs(z) + D; };
+  auto L = [&](double c0, double c1, double D0, double D1, double rho2, bool m, bool n) {
+    return cuboid_edge_L(b(c0, D0, rho2), b(c1, D1, rho2), rho2, m, n);
+  };
+  const double lz00 = L(z0, z1, D000, D001, xx0 + yy0, mz, nz), lz01 = L(z0, z1, D010, D011, xx0 + yy1, mz, nz),
+               lz10 = L(z0, z1, D100, D101, xx1 + yy0, mz, nz), lz11 = L(z0, z1, D110, D111, xx1 + yy1, mz, nz);
+  const double ly00 = L(y0, y1, D000, D010, xx0 + zz0, my, ny), ly01 = L(y0, y1, D001, D011, xx0 + zz1, my, ny),
+               ly10 = L(y0, y1, D100, D110, xx1 + zz0, my, ny), ly11 = L(y0, y1, D101, D111, xx1 + zz1, my, ny);
+  const double lx00 = L(x0, x1, D000, D100, yy0 + zz0, mx, nx), lx01 = L(x0, x1, D001, D101, yy0 + zz1, mx, nx),
+               lx10 = L(x0, x1, D010, D110, yy1 + zz0, mx, nx), lx11 = L(x0, x1, D011, D111, yy1 + zz1, mx, nx);
+  V3<double> bv = mk3<double>(xT + y0 * (lz10 - lz00) + y1 * (lz01 - lz11) + z0 * (ly10 - ly00) + z1 * (ly01 - ly11),
+                              yT + x0 * (lz01 - lz00) + x1 * (lz10 - lz11) + z0 * (lx10 - lx00) + z1 * (lx01 - lx11),
+                              zT + y0 * (lx01 - lx00) + y1 * (lx10 - lx11) + x0 * (ly01 - ly00) + x1 * (ly10 - ly11));
+  if (nan) {  // on a face plane without guards the angle is undefined, as in the reference
+    const double bad = __longlong_as_double(0x7ff8000000000000LL);
+    if (nan & 1) bv.x = bad;
+    if (nan & 2) bv.y = bad;
+    if (nan & 4) bv.z = bad;
+  }
+  const double c = 0.0001;
+  return mk3<double>(c * (J.y * bv.z - J.z * bv.y), c * (J.z * bv.x - J.x * bv.z), c * (J.x * bv.y - J.y * bv.x));
 }
 
 // Planar polygon face integrals (Sx,Sy,Sz) at a point given in the face frame
@@ -515,67 +521,57 @@ __device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double 
 // Arc current field at q (object frame), record a = [cx cy cz rmin rmax
 // phimin phimax h j nseg]; trapezoid rule in phi with nseg sectors
 // (radTArcCur::B_compWithTrapeth, radarccu.cpp:30-236).
+// One node i of the rule with its weight; the field is f times the nodes' sum.
+// The reference's terms with the elements of the cuboid: a sum u + D that
+// cancels for u < 0 is the square of the other legs over |u| + D, a pair of
+// arctangents is the argument of one product, and the angle between the point
+// and the node comes from their directions.
+__device__ __forceinline__ V3<double> arc_node(const double *a, V3<double> P, int i, double &f)
+{
+  const double ZeroTol = 1.E-10, SP = 1.E-10;
+  const double px = P.x - a[0], py = P.y - a[1], pz = P.z - a[2];
+  const double Rmin = a[3], Rmax = a[4], Phimin = a[5], Phimax = a[6], Height = a[7], Jaz = a[8];
+  const int nsec = (int)a[9];
+  const double rr = px * px + py * py + SP, r = sqrt64(rr);
+  // direction of the point, with SP on the y side as in the reference's arccosine of px / r
+  const double ir = rcp64(r), cp = px * ir, spa = sqrt64(fma(py, py, SP)) * ir, sp = py < 0 ? -spa : spa;
+  const double z1 = -Height / 2. - pz, z2 = z1 + Height;
+  const double step = (Phimax - Phimin + SP) / nsec;
+  double sph, cph;
+  sincos(Phimin + SP + i * step, &sph, &cph);
+  const double sdp = sph * cp - cph * sp, cdp = cph * cp + sph * sp;
+  const double rs = r * fabs(sdp), rCos = r * cdp, r1 = Rmin - rCos, r2 = Rmax - rCos;
+  const double z1z1 = z1 * z1, z2z2 = z2 * z2, ss = rs * rs, zz1 = z1z1 + ss, zz2 = z2z2 + ss;
+  const double h1 = fma(r1, r1, ss), h2 = fma(r2, r2, ss);  // squared distances in the plane
+  const double D11 = sqrt64(fmax(h1 + z1z1, ZeroTol)), D12 = sqrt64(fmax(h1 + z2z2, 1e-290));
+  const double D21 = sqrt64(fmax(h2 + z1z1, ZeroTol)), D22 = sqrt64(fmax(h2 + z2z2, 1e-290));
+  const double b1 = fabs(r1), b2 = fabs(r2), c1 = fabs(z1), c2 = fabs(z2);
+  const bool mr = r1 < 0.0 && r2 > 0.0, nr = r1 < 0.0, mz = z1 < 0.0 && z2 > 0.0, nz = z1 < 0.0;
+  const double ln1 = cuboid_edge_L(b1 + D11, b2 + D21, zz1, mr, nr);   // log((r1 + D11) / (r2 + D21))
+  const double ln2 = -cuboid_edge_L(b1 + D12, b2 + D22, zz2, mr, nr);  // log((r2 + D22) / (r1 + D12))
+  const double lz = cuboid_edge_L(c1 + D11, c2 + D12, h1, mz, nz) - cuboid_edge_L(c1 + D21, c2 + D22, h2, mz, nz);
+  // arctan(z2 |r1| / (rs D12)) - arctan(z1 |r1| / (rs D11)), and the outer radius with the sign turned
+  const double e1 = rs * D12, g1 = z2 * b1, e2 = rs * D11, g2 = z1 * b1;
+  const double at1 = angle64(fma(g1, e2, -(e1 * g2)), fma(e1, e2, g1 * g2), 0);
+  const double e3 = rs * D21, g3 = z1 * b2, e4 = rs * D22, g4 = z2 * b2;
+  const double at2 = angle64(fma(g3, e4, -(e3 * g4)), fma(e3, e4, g3 * g4), 0);
+  const double Buf = rs * ((r1 < 0 ? -at1 : at1) + (r2 < 0 ? -at2 : at2)) + z1 * ln1 + z2 * ln2;
+  const double FBxy = D11 - D21 + D22 - D12 + rCos * (ln1 + ln2);
+  const double FBz = Buf - rCos * lz;
+  const double wgt = (i == 0 || i == nsec) ? 0.5 : 1.0;
+  f = 0.0001 * Jaz * step;
+  return mk3<double>(wgt * cph * FBxy, wgt * sph * FBxy, wgt * FBz);
+}
 __device__ __forceinline__ V3<double> arc_field(const double *a, V3<double> P)
 {
-  const double Pi = 3.141592653589793238, ZeroTol = 1.E-10, RZ = 1.E-07, SP = 1.E-10;
-  double px = P.x - a[0], py = P.y - a[1], pz = P.z - a[2];
-  double Rmin = a[3], Rmax = a[4], Phimin = a[5], Phimax = a[6], Height = a[7], Jaz = a[8];
-  int nsec = (int)a[9];
-  double r = sqrt(px * px + py * py + SP);
-  double phi = (py < 0) ? (2 * Pi - acos(px / r)) : acos(px / r);
-  double z1 = -Height / 2. - pz, z2 = z1 + Height;
-  double z1z1 = z1 * z1, z2z2 = z2 * z2, rr = r * r, r1r1 = Rmin * Rmin, r2r2 = Rmax * Rmax;
-  double a11 = rr + r1r1 + z1z1, a12 = rr + r1r1 + z2z2, a21 = rr + r2r2 + z1z1, a22 = rr + r2r2 + z2z2;
-  double two_rr1 = 2. * r * Rmin, two_rr2 = 2. * r * Rmax;
-  int npoi = nsec + 1;
-  double step = (Phimax - Phimin + SP) / (npoi - 1);
-  double dphi = Phimin - phi + SP;
-  double SBx = 0., SBy = 0., SBz = 0.;
-  for (int i = 0; i < npoi; i++) {
-    double sdp, cdp;
-    sincos(dphi, &sdp, &cdp);
-    double asdp = fabs(sdp);
-    double t1 = two_rr1 * cdp, t2 = two_rr2 * cdp;
-    double b11 = fabs(a11 - t1); if (b11 < ZeroTol) b11 = ZeroTol;
-    double D11 = sqrt(b11), D12 = sqrt(fabs(a12 - t1));
-    double b21 = fabs(a21 - t2); if (b21 < ZeroTol) b21 = ZeroTol;
-    double D21 = sqrt(b21), D22 = sqrt(fabs(a22 - t2));
-    double rCos = r * cdp, r1m = Rmin - rCos, r2m = Rmax - rCos;
-    double d11 = D11 * RZ, d12 = D12 * RZ, d21 = D21 * RZ, d22 = D22 * RZ;
-    double zz = z1z1 + rr * asdp * asdp;
-    double r1me2 = r1m * r1m, r2me2 = r2m * r2m;
-    double u11 = r1m + D11; if ((fabs(u11) < d11) && (zz < r1me2 * RZ)) u11 = 0.5 * zz / fabs(r1m);
-    double u12 = r1m + D12; if ((fabs(u12) < d12) && (zz < r1me2 * RZ)) u12 = 0.5 * zz / fabs(r1m);
-    double u21 = r2m + D21; if ((fabs(u21) < d21) && (zz < r2me2 * RZ)) u21 = 0.5 * zz / fabs(r2m);
-    double u22 = r2m + D22; if ((fabs(u22) < d22) && (zz < r2me2 * RZ)) u22 = 0.5 * zz / fabs(r2m);
-    double ln1 = log(u11 / u21), ln2 = log(u22 / u12);
-    double rAbsSin = r * asdp;
-    double q1 = fabs(r1m) / rAbsSin, q2 = fabs(r2m) / rAbsSin;
-    double pm1 = 0., pm2 = 0.;
-    double at1 = atan(trans_atans(z2 * q1 / D12, -z1 * q1 / D11, pm1)) + Pi * pm1;
-    double at2 = atan(trans_atans(z1 * q2 / D21, -z2 * q2 / D22, pm2)) + Pi * pm2;
-    double Buf = rAbsSin * ((r1m < 0 ? -1. : 1.) * at1 + (r2m < 0 ? -1. : 1.) * at2) + z1 * ln1 + z2 * ln2;
-    double w11 = z1 + D11, s1 = rr + r1r1 - t1;
-    double z1t = z1z1 * RZ, z2t = z2z2 * RZ;
-    if ((fabs(w11) < d11) && (s1 < z1t)) w11 = 0.5 * s1 / fabs(z1);
-    double w21 = z1 + D21, s2 = rr + r2r2 - t2;
-    if ((fabs(w21) < d21) && (s2 < z1t)) w21 = 0.5 * s2 / fabs(z1);
-    double w12 = z2 + D12;
-    if ((fabs(w12) < d12) && (s1 < z2t)) w12 = 0.5 * s1 / fabs(z2);
-    double w22 = z2 + D22;
-    if ((fabs(w22) < d22) && (s2 < z2t)) w22 = 0.5 * s2 / fabs(z2);
-    double php = dphi + phi, sph, cph;
-    sincos(php, &sph, &cph);
-    double FBxy = D11 - D21 + D22 - D12 + rCos * (ln1 + ln2);
-    double FBz = Buf - rCos * log((w11 / w12) * (w22 / w21));
-    double wgt = (i == 0 || i == npoi - 1) ? 0.5 : 1.0;
-    SBx += wgt * cph * FBxy;
-    SBy += wgt * sph * FBxy;
-    SBz += wgt * FBz;
-    dphi += step;
+  const int n = (int)a[9] + 1;
+  V3<double> s = mk3<double>(0, 0, 0);
+  double f = 0.0;
+  for (int i = 0; i < n; i++) {
+    const V3<double> v = arc_node(a, P, i, f);
+    s.x += v.x; s.y += v.y; s.z += v.z;
   }
-  double f = 0.0001 * Jaz * step;
-  return mk3<double>(f * SBx, f * SBy, f * SBz);
+  return mk3<double>(f * s.x, f * s.y, f * s.z);
 }
 
 // ---------------------------------------------------------------------------
@@ -759,14 +755,9 @@ __device__ __forceinline__ double rd_rec(const double *p)
 }
 
 // SMEM: the record lives in shared memory (plain loads instead of __ldg).
-// recf (T = float, optional): the edge lengths (6) and face normals (12) of
-// the record already rounded to float, so that a pair reads them without a
-// conversion each (the same values as T(record entry)).
 template <typename T, bool TENSOR, bool SMEM = false>
-__device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<double> q, double *out,
-                                        const float *__restrict__ recf = nullptr)
+__device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<double> q, double *out)
 {
-  const bool fl = sizeof(T) == 4 && recf != nullptr;
   const double C = 1.0 / (4.0 * 3.141592653589793238);
   T rx[4], ry[4], rz[4], R[4];
 #pragma unroll
@@ -801,7 +792,7 @@ __device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<doubl
 #pragma unroll
     for (int e = 0; e < 6; e++) {
       const int a = tet_edge_a(e), b = tet_edge_b(e);
-      const T l = fl ? T(recf[e]) : T(rd_rec<SMEM>(rec + 12 + e));
+      const T l = T(rd_rec<SMEM>(rec + 12 + e));
       Le[e] = edge_L(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b], d[e], l);
     }
   }
@@ -815,9 +806,9 @@ __device__ __forceinline__ int tet_fast(const double *__restrict__ rec, V3<doubl
 #pragma unroll
   for (int f = 0; f < 4; f++) {
     const int a = tet_face_a(f), b = tet_face_b(f), c = tet_face_c(f);
-    const T m0 = fl ? T(recf[6 + 3 * f]) : T(rd_rec<SMEM>(rec + 18 + 3 * f));
-    const T m1 = fl ? T(recf[7 + 3 * f]) : T(rd_rec<SMEM>(rec + 19 + 3 * f));
-    const T m2 = fl ? T(recf[8 + 3 * f]) : T(rd_rec<SMEM>(rec + 20 + 3 * f));
+    const T m0 = T(rd_rec<SMEM>(rec + 18 + 3 * f));
+    const T m1 = T(rd_rec<SMEM>(rec + 19 + 3 * f));
+    const T m2 = T(rd_rec<SMEM>(rec + 20 + 3 * f));
     T num = rx[a] * m0 + ry[a] * m1 + rz[a] * m2;
     T den = R[a] * R[b] * R[c] + d[tet_pair(a, b)] * R[c] + d[tet_pair(a, c)] * R[b] + d[tet_pair(b, c)] * R[a];
     double om = 2.0 * (double)face_angle(-num, den);

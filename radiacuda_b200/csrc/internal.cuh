@@ -339,6 +339,11 @@ int build_mesh(const RadB200Geom *G, const std::vector<int> &tetidx, const std::
 // (what 0 B, 1 H; mesh.cu)
 int launch_mesh_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int accumulate,
                       DBuf &scratch, cudaStream_t st);
+// field of an all-tetrahedron model with FP32 terms (field_tet32.cu); at
+// least this many points are put in Morton order first
+constexpr int64_t T32_SORT_MIN = 32768;
+int launch_tet32_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int ub, int ue,
+                       int accumulate, DBuf &scratch, cudaStream_t st);
 // near lists of mixed storage from the element geometry (host, near.cu);
 // obs: [3n] element centres (main images)
 int build_near(Intrc &I, const RadB200Geom *elems, const RadB200Relax *r, const double *obs);

@@ -569,7 +569,7 @@ int field_int_impl(const RadB200Geom *g, const PointField &fld, const double *P1
 DevGeom g_int_geom;
 DBuf g_int_pts, g_int_out, g_int_scratch;
 DevGeom g_trj_geom;
-DBuf g_trj_init, g_trj_out, g_trj_status;
+DBuf g_trj_init, g_trj_out, g_trj_status, g_trj_items;
 
 }  // namespace
 }  // namespace rb
@@ -643,8 +643,32 @@ int radb200_trajectories(const RadB200Geom *g, double energy_gev, int n_traj, co
   size_t ob = (size_t)n_traj * np * 5 * sizeof(double);
   RB_TRY(g_trj_out.alloc(ob));
   RB_TRY(g_trj_status.alloc((size_t)n_traj * sizeof(int)));
-  RB_TRY(launch_trajectories(g_trj_geom.view(0), energy_gev, g_trj_init.as<double>(), n_traj, y0, y1, np, prec,
-                             g_trj_out.as<double>(), g_trj_status.as<int>(), 0));
+  // work items, an arc's nodes one by one; groups of 32 of one kind (a warp
+  // that mixes kinds pays for each), filled up with -1
+  const GeomView view = g_trj_geom.view(0);
+  std::vector<int2> items;
+  auto fill = [&] { items.resize((items.size() + 31) / 32 * 32, make_int2(-1, -1)); };
+  for (int i = 0, u = view.ustart[2]; i < g->n_arc; i++) {
+    const int nodes = (int)g->arc[(size_t)i * RADB200_ARC_STRIDE + 9] + 1;
+    for (int t = 0; t < g->arc_img[2 * i + 1]; t++, u++)
+      for (int k = 0; k < nodes; k++) items.push_back(make_int2(u, k));
+  }
+  fill();
+  for (int pass = 0; pass < 2; pass++) {  // current blocks, then magnetized ones
+    for (int i = 0, u = 0; i < g->n_rec; i++) {
+      const double *q = g->rec + (size_t)i * RADB200_REC_STRIDE + 9;
+      const bool cur = q[0] != 0.0 || q[1] != 0.0 || q[2] != 0.0;
+      for (int t = 0; t < g->rec_img[2 * i + 1]; t++, u++)
+        if (cur == (pass == 0)) items.push_back(make_int2(u, -1));
+    }
+    fill();
+  }
+  for (int u = view.ustart[1]; u < view.ustart[2]; u++) items.push_back(make_int2(u, -1));
+  fill();
+  for (int u = view.ustart[3]; u < view.ustart[4]; u++) items.push_back(make_int2(u, -1));
+  RB_TRY(g_trj_items.upload(items.data(), items.size() * sizeof(int2)));
+  RB_TRY(launch_trajectories(view, energy_gev, g_trj_init.as<double>(), n_traj, y0, y1, np, prec,
+                             g_trj_items.as<int2>(), (int)items.size(), g_trj_out.as<double>(), g_trj_status.as<int>(), 0));
   RB_CUDA(cudaMemcpy(out, g_trj_out.p, ob, cudaMemcpyDeviceToHost));
   std::vector<int> st(n_traj);
   RB_CUDA(cudaMemcpy(st.data(), g_trj_status.p, (size_t)n_traj * sizeof(int), cudaMemcpyDeviceToHost));

@@ -352,9 +352,11 @@ int launch_assemble_near(const GeomView &g, const int *elem_src, const double *o
                          const float *N32, const int *row, const int *col, int64_t nnz, double *D, cudaStream_t st);
 // out[j] += sum over near entries (i, j) of D_ij^T x_i (near.cu)
 int launch_near_t(const Intrc &I, const double *x, double *out, cudaStream_t st);
-// electron trajectories, one CTA each (field.cu); prec NULL: one RK4 step per
-// tabulation interval, else step-doubling control with these [4] accuracies
+// electron trajectories, a cluster of CTAs each (field.cu); prec NULL: one RK4
+// step per tabulation interval, else step-doubling control with these [4]
+// accuracies; items: {unit, arc node or -1} of every unit, arcs by node
 int launch_trajectories(const GeomView &g, double energy_gev, const double *d_init, int n_traj, double y0, double y1,
-                        int np, const double *prec, double *d_out, int *d_status, cudaStream_t st);
+                        int np, const double *prec, const int2 *d_items, int n_items, double *d_out, int *d_status,
+                        cudaStream_t st);
 
 }  // namespace rb

@@ -218,24 +218,26 @@ def test_polyhedra_by_faces(cuda, rad, shape):
 @pytest.mark.parametrize("ntets,npts", [(1, 1), (31, 130), (32, 32767), (33, 32768), (65, 33001)])
 def test_tetrahedra_with_fp32_terms(cuda, rad, ntets, npts):
     """Near and far pairs, tiles of 32 tetrahedra, point sets just below and
-    above the size that is put in Morton order.  An FP32 term is off by a few
-    units of 6e-8 and a distant tetrahedron's terms cancel by (R / l)^2, 400
-    at the far corner of this box: 5e-5 of the field, the bar of the FP32
-    option for polyhedra."""
+    above the size that is put in Morton order.  A tetrahedron's terms are its 6
+    edge integrals, about 2 l / R each with weights up to 1.4 |M| / (4 pi); an
+    FP32 term is off by at most 4 units of 2^-24, so B by at most
+    6 * 2 * 1.4 / (4 pi) * 4 * 2^-24 |M| l / R = 3.2e-7 |M| l / R a tetrahedron,
+    twice that with the solid angles."""
     rng = np.random.default_rng(npts)
     rad.UtiDelAll()
     rad.FldLenRndSw("off")
     faces = [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]]
     base = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], float)
     V = [1.2 * np.array([k % 5, (k // 5) % 5, k // 25]) + base + rng.uniform(-0.1, 0.1, (4, 3)) for k in range(ntets)]
-    obj = rad.ObjCnt([rad.ObjPolyhdr(v, faces, m) for v, m in zip(V, rng.normal(size=(ntets, 3)) + [0, 0, 3.0])])
+    M = rng.normal(size=(ntets, 3)) + [0, 0, 3.0]
+    obj = rad.ObjCnt([rad.ObjPolyhdr(v, faces, m) for v, m in zip(V, M)])
     P = rng.uniform(-6, 14, size=(npts, 3))
     b64 = rad.Fld(obj, "b", P, precision="fast")
     b32 = rad.Fld(obj, "b", P, precision="single")
-    far = np.array([min(np.linalg.norm(p - v.mean(0)) for v in V) > 1.0 for p in P[:2000]])
-    d = np.linalg.norm(b32 - b64, axis=1)[:2000][far]
-    assert np.all(d <= 5e-5 * np.maximum(np.linalg.norm(b64, axis=1)[:2000][far], 1e-5))
-    assert np.linalg.norm((b32 - b64)[:2000][far]) <= 2e-6 * np.linalg.norm(b64[:2000][far])
+    R = np.array([[np.linalg.norm(p - v.mean(0)) for v in V] for p in P[:2000]])
+    far = R.min(1) > 1.0
+    bound = 6.4e-7 * (np.linalg.norm(M, axis=1) * 1.6 / R).sum(1)
+    assert np.all((np.linalg.norm(b32 - b64, axis=1)[:2000] <= bound)[far])
     # the order of the points does not matter to a point (sums over chunks of
     # tetrahedra differ by FP64 rounding), nor do points that are not numbers
     sub = rad.Fld(obj, "b", np.ascontiguousarray(P[::7]), precision="single")

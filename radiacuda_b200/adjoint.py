@@ -127,11 +127,9 @@ class FieldProblem:
                           f"relaxation (misfit {st[0]:.3e}).", RuntimeWarning)
         t2 = time.perf_counter()
         g = {k: v.copy() for k, v in self.pack.elems.items()}
-        for e, (kind, idx) in enumerate(self.pack.elem_src):
-            if kind == 0:
-                g["rec"][idx, 6:9] = M[3 * e:3 * e + 3]
-            else:
-                g["poly"][idx, 3:6] = M[3 * e:3 * e + 3]
+        idx, rows = self.pack.elem_src[:, 1], M.reshape(-1, 3)
+        g["rec"][idx[self.rect], 6:9] = rows[self.rect]
+        g["poly"][idx[~self.rect], 3:6] = rows[~self.rect]
         F = _native.field(g, self.pts, self.what, 0)
         if self.pack.ext is not None:
             F = F + _native.field(self.pack.ext, self.pts, self.what, 0)

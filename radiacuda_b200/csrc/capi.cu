@@ -200,6 +200,34 @@ void pool_free(void *p, size_t b)
 }
 
 
+int Staging::upload(DBuf &blob)
+{
+  size_t total = 0, small = 0;
+  for (Part &q : parts) {  // the small ones first, side by side
+    if (q.bytes > STAGE_MAX) continue;
+    q.off = total;
+    total += (q.bytes + 255) / 256 * 256;
+  }
+  small = total;
+  for (Part &q : parts) {
+    if (q.bytes <= STAGE_MAX) continue;
+    q.off = total;
+    total += (q.bytes + 255) / 256 * 256;
+  }
+  RB_TRY(blob.alloc(total));
+  const double t0 = timing_on() ? now_s() : 0.0;
+  std::vector<char> host(small);
+  for (Part &q : parts) {
+    q.ref->p = q.bytes ? (char *)blob.p + q.off : nullptr;
+    if (q.bytes == 0) continue;
+    if (q.bytes <= STAGE_MAX) memcpy(host.data() + q.off, q.src, q.bytes);
+    else RB_CUDA(cudaMemcpy(q.ref->p, q.src, q.bytes, cudaMemcpyHostToDevice));
+  }
+  if (small) RB_CUDA(cudaMemcpy(blob.p, host.data(), small, cudaMemcpyHostToDevice));
+  if (t0 > 0.0) g_tm[2] += now_s() - t0;
+  return 0;
+}
+
 static int validate_geom(const RadB200Geom *G)
 {
   if (!G) { set_error("null geometry"); return RADB200_E_ARG; }
@@ -247,11 +275,10 @@ struct HostTopo {
 
 // Fixed-topology record of a tetrahedron (formulas.cuh, tet_fast) from its
 // deduplicated vertices V[4] and counter-clockwise face loops.
-static void build_tet_record(const std::vector<double> &V, const std::vector<std::vector<int>> &loops, const double *M,
-                             bool tensor, std::vector<double> &out)
+__host__ __device__ static void build_tet_record(const double *V, const int (*loops)[3], const double *M, bool tensor,
+                                                 double *rec)
 {
-  double rec[TET_REC_TENSOR] = {0};
-  for (int k = 0; k < 12; k++) rec[k] = V[k];
+  for (int k = 0; k < (tensor ? TET_REC_TENSOR : TET_REC_FIELD); k++) rec[k] = k < 12 ? V[k] : 0.0;
   for (int e = 0; e < 6; e++) {
     int a = tet_edge_a(e), b = tet_edge_b(e);
     double dx = V[3 * b] - V[3 * a], dy = V[3 * b + 1] - V[3 * a + 1], dz = V[3 * b + 2] - V[3 * a + 2];
@@ -259,10 +286,10 @@ static void build_tet_record(const std::vector<double> &V, const std::vector<std
   }
   for (int f = 0; f < 4; f++) {
     // the loop of face f is the one without vertex f
-    const std::vector<int> *L = nullptr;
-    for (auto &lp : loops)
-      if (lp[0] != f && lp[1] != f && lp[2] != f) L = &lp;
-    const double *p0 = &V[3 * (*L)[0]], *p1 = &V[3 * (*L)[1]], *p2 = &V[3 * (*L)[2]];
+    const int *L = loops[0];
+    for (int k = 0; k < 4; k++)
+      if (loops[k][0] != f && loops[k][1] != f && loops[k][2] != f) L = loops[k];
+    const double *p0 = &V[3 * L[0]], *p1 = &V[3 * L[1]], *p2 = &V[3 * L[2]];
     double u[3] = {p1[0] - p0[0], p1[1] - p0[1], p1[2] - p0[2]}, w[3] = {p2[0] - p0[0], p2[1] - p0[1], p2[2] - p0[2]};
     double m[3] = {u[1] * w[2] - u[2] * w[1], u[2] * w[0] - u[0] * w[2], u[0] * w[1] - u[1] * w[0]};
     double mn = sqrt(m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
@@ -273,12 +300,12 @@ static void build_tet_record(const std::vector<double> &V, const std::vector<std
       rec[30 + 3 * f + c] = tensor ? n[c] : sigma * n[c];
     }
     for (int j = 0; j < 3; j++) {  // directed edges of the counter-clockwise loop
-      int a = (*L)[j], b = (*L)[(j + 1) % 3];
+      int a = L[j], b = L[(j + 1) % 3];
       double t[3] = {V[3 * b] - V[3 * a], V[3 * b + 1] - V[3 * a + 1], V[3 * b + 2] - V[3 * a + 2]};
       double tl = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
       for (int c = 0; c < 3; c++) t[c] /= tl;
       double nu[3] = {t[1] * n[2] - t[2] * n[1], t[2] * n[0] - t[0] * n[2], t[0] * n[1] - t[1] * n[0]};
-      int e = tet_pair(std::min(a, b), std::max(a, b));
+      int e = a < b ? tet_pair(a, b) : tet_pair(b, a);
       if (tensor) {
         for (int r = 0, k = 0; r < 3; r++)
           for (int c = r; c < 3; c++, k++) rec[42 + 6 * e + k] += 0.5 * (nu[r] * n[c] + nu[c] * n[r]);
@@ -287,7 +314,53 @@ static void build_tet_record(const std::vector<double> &V, const std::vector<std
       }
     }
   }
-  out.insert(out.end(), rec, rec + (tensor ? TET_REC_TENSOR : TET_REC_FIELD));
+}
+
+// Records of a model of tetrahedra on the device, a thread each: vertices back
+// in 3-D from the face frames and merged within 1e-6 of the extent, in the
+// faces' order, as build_topo_range does.  *bad is set when one does not come
+// out with four vertices.  (16 host threads took 23 ms for 20,000 tetrahedra
+// with the topology of general polyhedra that nothing read.)
+__global__ void tet_records_kernel(const double *__restrict__ poly, const int *__restrict__ poly_info,
+                                   const double *__restrict__ face, const int *__restrict__ face_vtx,
+                                   const double *__restrict__ vtx2d, int n_poly, int tensor, double *__restrict__ rec,
+                                   int *__restrict__ idx, int *__restrict__ bad)
+{
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n_poly) return;
+  const int f0 = poly_info[4 * p];
+  double P[12][3], V[12], lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+  for (int k = 0; k < 4; k++) {
+    const double *R = face + (size_t)(f0 + k) * RADB200_FACE_STRIDE;
+    const int a0 = face_vtx[2 * (f0 + k)];
+    for (int j = 0; j < 3; j++) {
+      const double x = vtx2d[2 * (size_t)(a0 + j)], y = vtx2d[2 * (size_t)(a0 + j) + 1], z = R[9];
+      for (int c = 0; c < 3; c++) {
+        const double v = x * R[c] + y * R[3 + c] + z * R[6 + c];
+        P[3 * k + j][c] = v;
+        lo[c] = fmin(lo[c], v);
+        hi[c] = fmax(hi[c], v);
+      }
+    }
+  }
+  const double tol = 1e-6 * fmax(hi[0] - lo[0], fmax(hi[1] - lo[1], hi[2] - lo[2]));
+  int loops[4][3], nv = 0;
+  bool ok = true;
+  for (int k = 0; k < 12; k++) {
+    int found = -1;
+    for (int q = 0; q < nv && found < 0; q++)
+      if (fabs(V[3 * q] - P[k][0]) <= tol && fabs(V[3 * q + 1] - P[k][1]) <= tol && fabs(V[3 * q + 2] - P[k][2]) <= tol) found = q;
+    if (found < 0) {
+      if (nv == 4) { ok = false; break; }
+      found = nv++;
+      for (int c = 0; c < 3; c++) V[3 * found + c] = P[k][c];
+    }
+    loops[k / 3][k % 3] = found;
+  }
+  if (!ok || nv != 4) { *bad = 1; return; }
+  idx[p] = p;
+  build_tet_record(V, loops, poly + (size_t)p * RADB200_POLY_STRIDE + 3, tensor != 0,
+                   rec + (size_t)p * (tensor ? TET_REC_TENSOR : TET_REC_FIELD));
 }
 
 // Polyhedra [pa, pb) into h, their entries of tinfo / tinfo2 / tetidx at
@@ -349,7 +422,12 @@ static void build_topo_range(const RadB200Geom *G, bool tensor, int pa, int pb, 
     int nv = (int)(V.size() / 3);
     if (nv == 4 && nf == 4 && loops[0].size() == 3 && loops[1].size() == 3 && loops[2].size() == 3 && loops[3].size() == 3) {
       h.tetidx[p] = (int)(h.tetrec.size() / (tensor ? TET_REC_TENSOR : TET_REC_FIELD));
-      build_tet_record(V, loops, M, tensor, h.tetrec);
+      int lp[4][3];
+      for (int k = 0; k < 4; k++)
+        for (int c = 0; c < 3; c++) lp[k][c] = loops[k][c];
+      double rec[TET_REC_TENSOR];
+      build_tet_record(V.data(), lp, M, tensor, rec);
+      h.tetrec.insert(h.tetrec.end(), rec, rec + (tensor ? TET_REC_TENSOR : TET_REC_FIELD));
     }
     if (nv > POLY_NV_FAST) {  // too many vertices for the register form: reference form only
       h.tinfo[p] = make_int4(v0, -1, e0, 0);
@@ -450,6 +528,76 @@ static void build_topo(const RadB200Geom *G, bool tensor, HostTopo &h)
   }
 }
 
+// The vertex/edge form of the polyhedra: tetrahedron records on the device when
+// all are tetrahedra, else the host's topology of general polyhedra.
+int DevGeom::upload_topo(const RadB200Geom *G, Form form)
+{
+  PhaseClock pc;
+  const int tensor = form == TENSOR;
+  const size_t rs = tensor ? TET_REC_TENSOR : TET_REC_FIELD;
+  std::vector<int> idx;
+  std::vector<double> rec;
+  bool tets = true;
+  for (int i = 0; i < G->n_poly && tets; i++) {
+    const int f0 = G->poly_info[4 * i];
+    tets = G->poly_info[4 * i + 1] == 4;
+    for (int f = f0; f < f0 + 4 && tets; f++) tets = G->face_vtx[2 * f + 1] == 3;
+  }
+  if (tets) {
+    const size_t rb = (size_t)G->n_poly * rs * sizeof(double), ib = ((size_t)G->n_poly + 1) * sizeof(int);
+    RB_TRY(topo_blob.alloc(rb + ib));
+    tetrec.p = topo_blob.p;
+    tetidx.p = (char *)topo_blob.p + rb;
+    int *bad = tetidx.as<int>() + G->n_poly, hbad = 0;
+    RB_CUDA(cudaMemsetAsync(bad, 0, sizeof(int)));
+    tet_records_kernel<<<(G->n_poly + 127) / 128, 128>>>(poly.as<double>(), poly_info.as<int>(), face.as<double>(),
+                                                         face_vtx.as<int>(), vtx2d.as<double>(), G->n_poly, tensor,
+                                                         tetrec.as<double>(), tetidx.as<int>(), bad);
+    RB_TRY(check_launch("tet_records_kernel"));
+    RB_CUDA(cudaMemcpy(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost));
+    tets = hbad == 0;
+    if (tets && form == MESH) {
+      idx.resize(G->n_poly);
+      rec.resize((size_t)G->n_poly * rs);
+      for (int i = 0; i < G->n_poly; i++) idx[i] = i;
+      RB_CUDA(cudaMemcpy(rec.data(), tetrec.p, rb, cudaMemcpyDeviceToHost));
+    }
+    pc.mark("geometry: tetrahedra");
+  }
+  if (!tets) {
+    HostTopo h;
+    build_topo(G, tensor != 0, h);
+    pc.mark("geometry: topology (host)");
+    Staging st;
+    st.add(tinfo, h.tinfo.data(), h.tinfo.size() * sizeof(int4));
+    st.add(tinfo2, h.tinfo2.data(), h.tinfo2.size() * sizeof(int4));
+    st.add(tv, h.tv.data(), h.tv.size() * sizeof(double));
+    st.add(te, h.te.data(), h.te.size() * sizeof(int2));
+    st.add(tel, h.tel.data(), h.tel.size() * sizeof(double));
+    st.add(teg, h.teg.data(), h.teg.size() * sizeof(double));
+    st.add(teG, h.teG.data(), h.teG.size() * sizeof(double));
+    st.add(tt, h.tt.data(), h.tt.size() * sizeof(int4));
+    st.add(ttm, h.ttm.data(), h.ttm.size() * sizeof(double));
+    st.add(tfn, h.tfn.data(), h.tfn.size() * sizeof(double));
+    st.add(tfa, h.tfa.data(), h.tfa.size() * sizeof(double));
+    st.add(tetidx, h.tetidx.data(), h.tetidx.size() * sizeof(int));
+    st.add(tetrec, h.tetrec.data(), h.tetrec.size() * sizeof(double));
+    RB_TRY(st.upload(topo_blob));
+    tets = std::all_of(h.tetidx.begin(), h.tetidx.end(), [](int t) { return t >= 0; });
+    idx = std::move(h.tetidx);
+    rec = std::move(h.tetrec);
+  }
+  all_tets = tets ? 1 : 0;
+  tet_single = all_tets && G->n_rec == 0 && G->n_arc == 0 && G->n_bkg == 0;
+  for (int i = 0; i < G->n_poly && tet_single; i++) tet_single = G->poly_info[4 * i + 3] == 1;
+  has_topo = 1;
+  // field geometry of an all-tetrahedron model: the mesh form (unique edges and faces)
+  pc.mark("geometry: topology upload");
+  if (all_tets && form == MESH) RB_TRY(build_mesh(G, idx, rec, *this));
+  pc.mark("geometry: mesh form");
+  return 0;
+}
+
 int DevGeom::upload(const RadB200Geom *G, Form form)
 {
   RB_TRY(validate_geom(G));
@@ -458,53 +606,6 @@ int DevGeom::upload(const RadB200Geom *G, Form form)
   tet_single = 0;
   has_topo = 0;
   m_tiles = m_groups = 0;
-  if (G->n_poly > 0 && form != FACES) {
-    const bool tensor_coeffs = form == TENSOR;
-    HostTopo h;
-    PhaseClock pc;
-    build_topo(G, tensor_coeffs, h);
-    pc.mark("geometry: topology (host)");
-    RB_TRY(tinfo.upload(h.tinfo.data(), h.tinfo.size() * sizeof(int4)));
-    RB_TRY(tinfo2.upload(h.tinfo2.data(), h.tinfo2.size() * sizeof(int4)));
-    RB_TRY(tv.upload(h.tv.data(), h.tv.size() * sizeof(double)));
-    RB_TRY(te.upload(h.te.data(), h.te.size() * sizeof(int2)));
-    RB_TRY(tel.upload(h.tel.data(), h.tel.size() * sizeof(double)));
-    RB_TRY(teg.upload(h.teg.data(), h.teg.size() * sizeof(double)));
-    RB_TRY(teG.upload(h.teG.data(), h.teG.size() * sizeof(double)));
-    RB_TRY(tt.upload(h.tt.data(), h.tt.size() * sizeof(int4)));
-    RB_TRY(ttm.upload(h.ttm.data(), h.ttm.size() * sizeof(double)));
-    RB_TRY(tfn.upload(h.tfn.data(), h.tfn.size() * sizeof(double)));
-    RB_TRY(tfa.upload(h.tfa.data(), h.tfa.size() * sizeof(double)));
-    RB_TRY(tetidx.upload(h.tetidx.data(), h.tetidx.size() * sizeof(int)));
-    RB_TRY(tetrec.upload(h.tetrec.data(), h.tetrec.size() * sizeof(double)));
-    all_tets = std::all_of(h.tetidx.begin(), h.tetidx.end(), [](int t) { return t >= 0; }) ? 1 : 0;
-    tet_single = all_tets && G->n_rec == 0 && G->n_arc == 0 && G->n_bkg == 0;
-    for (int i = 0; i < G->n_poly && tet_single; i++) tet_single = G->poly_info[4 * i + 3] == 1;
-    has_topo = 1;
-    // field geometry of an all-tetrahedron model: the mesh form (unique edges and faces)
-    pc.mark("geometry: topology upload");
-    if (all_tets && form == MESH) RB_TRY(build_mesh(G, h.tetidx, h.tetrec, *this));
-    pc.mark("geometry: mesh form");
-  }
-  RB_TRY(trf.upload(G->trf, (size_t)G->n_trf * RADB200_TRF_STRIDE * sizeof(double)));
-  RB_TRY(rec.upload(G->rec, (size_t)G->n_rec * RADB200_REC_STRIDE * sizeof(double)));
-  RB_TRY(rec_img.upload(G->rec_img, (size_t)G->n_rec * 2 * sizeof(int)));
-  RB_TRY(poly.upload(G->poly, (size_t)G->n_poly * RADB200_POLY_STRIDE * sizeof(double)));
-  RB_TRY(poly_info.upload(G->poly_info, (size_t)G->n_poly * 4 * sizeof(int)));
-  RB_TRY(face.upload(G->face, (size_t)G->n_face * RADB200_FACE_STRIDE * sizeof(double)));
-  RB_TRY(face_vtx.upload(G->face_vtx, (size_t)G->n_face * 2 * sizeof(int)));
-  RB_TRY(vtx2d.upload(G->vtx2d, (size_t)G->n_vtx * 2 * sizeof(double)));
-  RB_TRY(edge.alloc((size_t)G->n_vtx * EDGE_REC * sizeof(double)));
-  RB_TRY(launch_edge_records(face_vtx.as<int>(), vtx2d.as<double>(), G->n_face, edge.as<double>(), 0));
-  all_tri = form == FACES && G->n_poly > 0;
-  for (int f = 0; f < G->n_face && all_tri; f++) all_tri = G->face_vtx[2 * f + 1] == 3;
-  for (int i = 0; i < G->n_poly && all_tri; i++) all_tri = G->poly_info[4 * i + 1] <= TRI_TILE;
-  if (all_tri) {
-    RB_TRY(tri.alloc((size_t)G->n_face * TRI_REC * sizeof(double)));
-    RB_TRY(launch_tri_records(view(0), G->n_poly, tri.as<double>(), 0));
-  }
-  RB_TRY(arc.upload(G->arc, (size_t)G->n_arc * RADB200_ARC_STRIDE * sizeof(double)));
-  RB_TRY(bkg.upload(G->bkg, (size_t)G->n_bkg * 3 * sizeof(double)));
   // unit table: one entry per (source, image); cuboids, polyhedra, arcs, backgrounds
   std::vector<int4> u;
   std::vector<char> diag(G->n_trf);
@@ -526,7 +627,29 @@ int DevGeom::upload(const RadB200Geom *G, Form form)
     for (int t = 0; t < G->bkg_img[2 * i + 1]; t++) u.push_back(make_int4(3, i, G->bkg_img[2 * i] + t, diag[G->bkg_img[2 * i] + t]));
   ustart[4] = (int)u.size();
   n_units = (int)u.size();
-  RB_TRY(units.upload(u.data(), u.size() * sizeof(int4)));
+  Staging st;
+  st.add(trf, G->trf, (size_t)G->n_trf * RADB200_TRF_STRIDE * sizeof(double));
+  st.add(rec, G->rec, (size_t)G->n_rec * RADB200_REC_STRIDE * sizeof(double));
+  st.add(rec_img, G->rec_img, (size_t)G->n_rec * 2 * sizeof(int));
+  st.add(poly, G->poly, (size_t)G->n_poly * RADB200_POLY_STRIDE * sizeof(double));
+  st.add(poly_info, G->poly_info, (size_t)G->n_poly * 4 * sizeof(int));
+  st.add(face, G->face, (size_t)G->n_face * RADB200_FACE_STRIDE * sizeof(double));
+  st.add(face_vtx, G->face_vtx, (size_t)G->n_face * 2 * sizeof(int));
+  st.add(vtx2d, G->vtx2d, (size_t)G->n_vtx * 2 * sizeof(double));
+  st.add(arc, G->arc, (size_t)G->n_arc * RADB200_ARC_STRIDE * sizeof(double));
+  st.add(bkg, G->bkg, (size_t)G->n_bkg * 3 * sizeof(double));
+  st.add(units, u.data(), u.size() * sizeof(int4));
+  RB_TRY(st.upload(blob));
+  RB_TRY(edge.alloc((size_t)G->n_vtx * EDGE_REC * sizeof(double)));
+  RB_TRY(launch_edge_records(face_vtx.as<int>(), vtx2d.as<double>(), G->n_face, edge.as<double>(), 0));
+  all_tri = form == FACES && G->n_poly > 0;
+  for (int f = 0; f < G->n_face && all_tri; f++) all_tri = G->face_vtx[2 * f + 1] == 3;
+  for (int i = 0; i < G->n_poly && all_tri; i++) all_tri = G->poly_info[4 * i + 1] <= TRI_TILE;
+  if (all_tri) {
+    RB_TRY(tri.alloc((size_t)G->n_face * TRI_REC * sizeof(double)));
+    RB_TRY(launch_tri_records(view(0), G->n_poly, tri.as<double>(), 0));
+  }
+  if (G->n_poly > 0 && form != FACES) RB_TRY(upload_topo(G, form));
   n_rec = G->n_rec;
   n_poly = G->n_poly;
   return 0;
@@ -678,6 +801,26 @@ static uint64_t fnv1a(uint64_t h, const void *p, size_t n)
   return h;
 }
 
+// The stamp of an interaction, before its materials change or when a state is
+// saved or restored.  (Formed at creation it was a seventh of a small model's
+// relaxation: a serial hash over 200 bytes an element.)
+static uint64_t intrc_stamp(Intrc &I)
+{
+  if (!I.has_stamp) {
+    uint64_t st = 1469598103934665603ULL;
+    const int32_t hdr[5] = {I.n, I.storage, I.fast, I.e0, I.e0 + I.nr};
+    st = fnv1a(st, hdr, sizeof(hdr));
+    st = fnv1a(st, I.h_obs.data(), I.h_obs.size() * sizeof(double));
+    st = fnv1a(st, I.h_rowT.data(), I.h_rowT.size() * sizeof(double));
+    st = fnv1a(st, I.h_elem_src.data(), 2 * (size_t)I.n * sizeof(int32_t));
+    st = fnv1a(st, I.h_mat_kind.data(), (size_t)I.n * sizeof(int32_t));
+    st = fnv1a(st, I.h_mat.data(), (size_t)I.n * RADB200_MAT_STRIDE * sizeof(double));
+    I.stamp = st;
+    I.has_stamp = true;
+  }
+  return I.stamp;
+}
+
 // Material records: linear and tanh laws, and tables whose rows lie inside
 // mh_table with H ascending (the reference's MatSatIsoTab check,
 // radapl2.cpp:152-166) and at least two points.
@@ -773,28 +916,26 @@ static int intrc_create_impl(const RadB200Geom *elems, const RadB200Relax *r, co
     }
   }
   // observers of the rows held (all of them unless a row block)
-  RB_TRY(I->obs.upload(obs.data() + 3 * (size_t)e0, 3 * (size_t)nr * sizeof(double)));
-  RB_TRY(I->rowT.upload(rowT.data() + 9 * (size_t)e0, 9 * (size_t)nr * sizeof(double)));
   {
-    uint64_t st = 1469598103934665603ULL;
-    int32_t hdr[5] = {n, storage, fast, e0, e1};
-    st = fnv1a(st, hdr, sizeof(hdr));
-    st = fnv1a(st, obs.data(), obs.size() * sizeof(double));
-    st = fnv1a(st, rowT.data(), rowT.size() * sizeof(double));
-    st = fnv1a(st, r->elem_src, 2 * (size_t)n * sizeof(int32_t));
-    st = fnv1a(st, r->mat_kind, (size_t)n * sizeof(int32_t));
-    st = fnv1a(st, r->mat, (size_t)n * RADB200_MAT_STRIDE * sizeof(double));
-    I->stamp = st;
+    Staging st;
+    st.add(I->obs, obs.data() + 3 * (size_t)e0, 3 * (size_t)nr * sizeof(double));
+    st.add(I->rowT, rowT.data() + 9 * (size_t)e0, 9 * (size_t)nr * sizeof(double));
+    st.add(I->elem_src, r->elem_src, 2 * (size_t)n * sizeof(int));
+    RB_TRY(st.upload(I->elem_blob));
   }
-  RB_TRY(I->elem_src.upload(r->elem_src, 2 * (size_t)n * sizeof(int)));
   RB_TRY(upload_materials(*I, r));
   pc.mark("create: observers, materials");
   size_t nn = (size_t)3 * nr * I->ld;
   // mixed: every block in FP32, the near ones also as their FP64 residue
   if (storage == RADB200_STORE_F64) RB_TRY(I->N64.alloc(nn * sizeof(double)));
   if (storage == RADB200_STORE_F32 || storage == RADB200_STORE_MIXED) RB_TRY(I->N32.alloc(nn * sizeof(float)));
-  if (I->N64.p) RB_CUDA(cudaMemsetAsync(I->N64.p, 0, nn * sizeof(double)));
-  if (I->N32.p) RB_CUDA(cudaMemsetAsync(I->N32.p, 0, nn * sizeof(float)));
+  // the rows' padding (products read whole rows); assembly writes the rest
+  if (const size_t pad = (size_t)I->ld - I->n3) {
+    if (I->N64.p)
+      RB_CUDA(cudaMemset2DAsync(I->N64.as<double>() + I->n3, I->ld * sizeof(double), 0, pad * sizeof(double), 3 * (size_t)nr));
+    if (I->N32.p)
+      RB_CUDA(cudaMemset2DAsync(I->N32.as<float>() + I->n3, I->ld * sizeof(float), 0, pad * sizeof(float), 3 * (size_t)nr));
+  }
   if (assemble)
     RB_TRY(launch_assemble(I->geom.view(fast), I->elem_src.as<int>(), I->obs.as<double>(), I->rowT.as<double>(), nr, n,
                            I->ld, I->N32.as<float>(), I->N64.as<double>(), 0));
@@ -804,7 +945,7 @@ static int intrc_create_impl(const RadB200Geom *elems, const RadB200Relax *r, co
   // external field at element centres, in element frames
   size_t vb = (size_t)I->ld * sizeof(double);
   RB_TRY(I->hext.alloc(vb));
-  RB_CUDA(cudaMemset(I->hext.p, 0, vb));
+  RB_CUDA(cudaMemsetAsync(I->hext.p, 0, vb));
   if (ext && (ext->n_rec + ext->n_poly + ext->n_arc + ext->n_bkg) > 0) {
     DevGeom &xg = I->xgeom;
     RB_TRY(xg.upload(ext, fast ? DevGeom::MESH : DevGeom::FACES));
@@ -815,10 +956,11 @@ static int intrc_create_impl(const RadB200Geom *elems, const RadB200Relax *r, co
     RB_TRY(launch_rowtrans_vec(I->rowT.as<double>(), tmp.as<double>(), I->hext.as<double>(), nr, 0));
   }
   RB_TRY(I->M.alloc(vb)); RB_TRY(I->H.alloc(vb)); RB_TRY(I->Mp.alloc(vb)); RB_TRY(I->F.alloc(vb));
-  RB_CUDA(cudaMemset(I->M.p, 0, vb)); RB_CUDA(cudaMemset(I->H.p, 0, vb));
-  RB_CUDA(cudaMemset(I->Mp.p, 0, vb)); RB_CUDA(cudaMemset(I->F.p, 0, vb));
+  for (DBuf *b : {&I->M, &I->H, &I->Mp, &I->F}) RB_CUDA(cudaMemsetAsync(b->p, 0, vb));
   RB_CUDA(cudaDeviceSynchronize());
   pc.mark("create: external field");
+  I->h_obs = std::move(obs);
+  I->h_rowT = std::move(rowT);
   int64_t h = g_next_handle++;
   g_intrc[h] = std::move(I);
   *handle = h;
@@ -881,6 +1023,7 @@ int radb200_intrc_load(const RadB200Relax *r, const float *N, const double *h_ex
     st = fnv1a(st, r->mat_kind, (size_t)n * sizeof(int32_t));
     st = fnv1a(st, r->mat, (size_t)n * RADB200_MAT_STRIDE * sizeof(double));
     I->stamp = st;
+    I->has_stamp = true;
   }
   RB_CUDA(cudaDeviceSynchronize());
   int64_t h = g_next_handle++;
@@ -895,6 +1038,7 @@ int radb200_intrc_set_materials(int64_t handle, const RadB200Relax *r)
   if (!I) return RADB200_E_HANDLE;
   if (!r || !r->mat_kind || !r->mat || r->n_elem != I->n) { set_error("bad arguments"); return RADB200_E_ARG; }
   RB_TRY(check_materials(r));
+  intrc_stamp(*I);  // of the materials it was created with
   RB_TRY(upload_materials(*I, r));
   // factors and the converged state belong to the old materials
   I->drop_lu_graphs();
@@ -955,7 +1099,7 @@ int radb200_intrc_save(int64_t handle, void *buf, int64_t capacity, int64_t *byt
   if (capacity < total) { set_error("state buffer too small: %lld bytes needed", (long long)total); return RADB200_E_ARG; }
   StateHeader h{};
   memcpy(h.magic, STATE_MAGIC, 8);
-  h.n = I->n; h.ld = I->ld; h.storage = I->storage; h.fast = I->fast; h.stamp = I->stamp;
+  h.n = I->n; h.ld = I->ld; h.storage = I->storage; h.fast = I->fast; h.stamp = intrc_stamp(*I);
   h.lu_mode = I->lu_mode; h.lu_tc = I->lu_tc; h.lu_of_d = I->lu_of_d; h.last_kind = I->last_kind;
   h.solve_id = I->solve_id; h.lu_solve_id = I->lu_solve_id; h.nsec = (int32_t)secs.size();
   char *o = (char *)buf;
@@ -988,7 +1132,7 @@ int radb200_intrc_restore(const RadB200Geom *elems, const RadB200Relax *r, const
   };
   if (h.n != I->n || h.ld != I->ld || h.storage != I->storage || h.fast != I->fast)
     return fail("sizes or storage differ from this geometry");
-  if (h.stamp != I->stamp) return fail("geometry stamp differs (other elements, images or materials)");
+  if (h.stamp != intrc_stamp(*I)) return fail("geometry stamp differs (other elements, images or materials)");
   const char *p = (const char *)buf + sizeof(h), *end = (const char *)buf + bytes;
   const int64_t nn = (int64_t)I->n3 * I->ld;
   for (int k = 0; k < h.nsec; k++) {

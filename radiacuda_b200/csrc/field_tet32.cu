@@ -25,9 +25,11 @@ namespace rb {
 
 namespace {
 
-constexpr int T32_TILE = 32;
+constexpr int T32_TILE = 32, T32_T = 256;
 constexpr int T32_D = 66;  // doubles per unit: v (12), 2 C a_f (12), 2 C g_e (18), point map (12), field map (9), M (3)
 constexpr int T32_F = 20;  // floats per unit: edge lengths (6), face normals m (12), (4 longest edge)^2, 1 if both maps are diagonal
+constexpr int T32_REC = T32_D * 8 + T32_F * 4;  // bytes of a unit's record: the doubles, then the floats
+static_assert(T32_REC % 16 == 0 && (T32_D * 8) % 16 == 0, "records are copied 16 bytes at a time");
 
 __device__ __forceinline__ float rcp32(float d)
 {
@@ -155,70 +157,82 @@ __device__ __forceinline__ void tet32_pair(const double *__restrict__ sd, const 
   }
 }
 
-// PPT points per thread; perm: the order of the points (null: as they are)
-template <int PPT>
-__global__ void __launch_bounds__(128) field_tet32_kernel(GeomView g, const double *__restrict__ pts, int64_t npts,
-                                                          const unsigned *__restrict__ perm, int what,
-                                                          double *__restrict__ out, int ub, int ue, int chunk, int accumulate)
+// the records of units [ub, ub + nu)
+__global__ void tet32_record_kernel(GeomView g, int ub, int nu, unsigned char *__restrict__ rec)
 {
-  __shared__ __align__(16) double sd[T32_TILE * T32_D];
-  __shared__ __align__(16) float sf[T32_TILE * T32_F];
-  const int tid = threadIdx.x;
-  const int u0 = ub + blockIdx.y * chunk, u1 = min(ue, u0 + chunk);
-  int64_t idx[PPT];
-  D3 P[PPT];
-  double acc[PPT][3];
-#pragma unroll
-  for (int p = 0; p < PPT; p++) {
-    const int64_t i = (int64_t)blockIdx.x * (128 * PPT) + p * 128 + tid;
-    idx[p] = i < npts ? (perm ? (int64_t)perm[i] : i) : -1;
-    P[p] = D3{0, 0, 0};
-    if (idx[p] >= 0) P[p] = D3{pts[3 * idx[p]], pts[3 * idx[p] + 1], pts[3 * idx[p] + 2]};
-    acc[p][0] = acc[p][1] = acc[p][2] = 0.0;
-  }
-  const double C2 = 2.0 / (4.0 * 3.141592653589793238);
-  for (int base = u0; base < u1; base += T32_TILE) {
-    const int cnt = min(T32_TILE, u1 - base);
-    __syncthreads();
-    for (int e = tid; e < cnt * T32_D; e += 128) {
-      const int k = e / T32_D, f = e - k * T32_D;
-      const int4 un = __ldg(g.units + base + k);  // {kind, polyhedron, transform, diagonal point map}
-      const double *rec = g.tetrec + (size_t)__ldg(g.tetidx + un.y) * TET_REC_FIELD;
+  const int64_t tot = (int64_t)nu * (T32_D + T32_F);
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
+    const int k = (int)(e / (T32_D + T32_F)), f = (int)(e - (int64_t)k * (T32_D + T32_F));
+    const int4 un = g.units[ub + k];  // {kind, polyhedron, transform, diagonal point map}
+    const double *t = g.tetrec + (size_t)g.tetidx[un.y] * TET_REC_FIELD, *T = g.trf + (size_t)un.z * RADB200_TRF_STRIDE;
+    unsigned char *o = rec + (size_t)k * T32_REC;
+    if (f < T32_D) {
+      const double C2 = 2.0 / (4.0 * 3.141592653589793238);
       double v;
-      if (f < 12) v = __ldg(rec + f);
-      else if (f < 42) v = C2 * __ldg(rec + 18 + f);  // a_f from 30, g_e from 42
-      else if (f < 63) v = __ldg(g.trf + (size_t)un.z * RADB200_TRF_STRIDE + (f - 42));
-      else v = __ldg(g.poly + (size_t)un.y * RADB200_POLY_STRIDE + 3 + (f - 63));
-      sd[e] = v;
-    }
-    for (int e = tid; e < cnt * T32_F; e += 128) {
-      const int k = e / T32_F, f = e - k * T32_F;
-      const int4 un = __ldg(g.units + base + k);
-      const double *rec = g.tetrec + (size_t)__ldg(g.tetidx + un.y) * TET_REC_FIELD + 12;  // lengths, then normals
+      if (f < 12) v = t[f];
+      else if (f < 42) v = C2 * t[18 + f];  // a_f from 30, g_e from 42
+      else if (f < 63) v = T[f - 42];
+      else v = g.poly[(size_t)un.y * RADB200_POLY_STRIDE + 3 + (f - 63)];
+      reinterpret_cast<double *>(o)[f] = v;
+    } else {
+      const int q = f - T32_D;
       float v;
-      if (f < 18) v = (float)__ldg(rec + f);
-      else if (f == 18) {
+      if (q < 18) v = (float)t[12 + q];  // lengths, then normals
+      else if (q == 18) {
         double m = 0.0;
-        for (int q = 0; q < 6; q++) m = fmax(m, __ldg(rec + q));
+        for (int c = 0; c < 6; c++) m = fmax(m, t[12 + c]);
         v = (float)(16.0 * m * m);
       } else {
-        const double *F = g.trf + (size_t)un.z * RADB200_TRF_STRIDE + 12;
+        const double *F = T + 12;
         v = un.w && F[1] == 0.0 && F[2] == 0.0 && F[3] == 0.0 && F[5] == 0.0 && F[6] == 0.0 && F[7] == 0.0 ? 1.f : 0.f;
       }
-      sf[e] = v;
+      reinterpret_cast<float *>(o + T32_D * 8)[q] = v;
     }
-    __syncthreads();
-    for (int k = 0; k < cnt; k++)
-#pragma unroll
-      for (int p = 0; p < PPT; p++) tet32_pair(sd + k * T32_D, sf + k * T32_F, P[p], what, acc[p]);
   }
-#pragma unroll
-  for (int p = 0; p < PPT; p++)
-    if (idx[p] >= 0) {
-      double *o = out + ((size_t)blockIdx.y * npts + idx[p]) * 3;
-#pragma unroll
-      for (int c = 0; c < 3; c++) o[c] = accumulate ? o[c] + acc[p][c] : acc[p][c];
+}
+
+// perm: the order of the points (null: as they are).  Records come in through
+// two shared buffers, the next tile's copy under way while a tile is summed.
+__global__ void __launch_bounds__(T32_T) field_tet32_kernel(const unsigned char *__restrict__ rec,
+                                                            const double *__restrict__ pts, int64_t npts,
+                                                            const unsigned *__restrict__ perm, int what,
+                                                            double *__restrict__ out, int nu, int chunk, int accumulate)
+{
+  __shared__ __align__(16) unsigned char buf[2][T32_TILE * T32_REC];
+  const int tid = threadIdx.x;
+  const int u0 = blockIdx.y * chunk, u1 = min(nu, u0 + chunk);
+  const int64_t i = (int64_t)blockIdx.x * T32_T + tid;
+  const int64_t idx = i < npts ? (perm ? (int64_t)perm[i] : i) : -1;
+  D3 P{0, 0, 0};
+  if (idx >= 0) P = D3{pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]};
+  double acc[3] = {0, 0, 0};
+  auto fetch = [&](int base, int b) {
+    const int n16 = min(T32_TILE, u1 - base) * (T32_REC / 16);
+    const unsigned char *src = rec + (size_t)base * T32_REC;
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(buf[b]);
+    for (int e = tid; e < n16; e += T32_T)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src + 16 * (size_t)e) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(u0, 0);
+  for (int base = u0, b = 0; base < u1; base += T32_TILE, b ^= 1) {
+    if (base + T32_TILE < u1) {
+      fetch(base + T32_TILE, b ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int cnt = min(T32_TILE, u1 - base);
+    for (int k = 0; k < cnt; k++) {
+      const unsigned char *r = buf[b] + k * T32_REC;
+      tet32_pair(reinterpret_cast<const double *>(r), reinterpret_cast<const float *>(r + T32_D * 8), P, what, acc);
     }
+    __syncthreads();  // before the tile after next is copied over this one
+  }
+  if (idx >= 0) {
+    double *o = out + ((size_t)blockIdx.y * npts + idx) * 3;
+#pragma unroll
+    for (int c = 0; c < 3; c++) o[c] = accumulate ? o[c] + acc[c] : acc[c];
+  }
 }
 
 // floats in an order that unsigned integers share
@@ -314,14 +328,21 @@ struct PointOrder {
   }
 };
 
-template <int PPT>
-int launch_ppt(const GeomView &g, const double *d_pts, int64_t npts, const unsigned *perm, int what, double *d_out, int ub,
-               int ue, int accumulate, DBuf &scratch, cudaStream_t st)
+}  // namespace
+
+int launch_tet32_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int ub, int ue,
+                       int accumulate, DBuf &scratch, cudaStream_t st)
 {
-  const int64_t nblk = (npts + 128 * PPT - 1) / (128 * PPT);
+  PointOrder order;
+  if (npts >= T32_SORT_MIN && npts <= INT32_MAX) RB_TRY(order.build(d_pts, npts, st));
+  const int64_t nblk = (npts + T32_T - 1) / T32_T;
   const int nu = ue - ub;
+  DBuf rec;
+  RB_TRY(rec.alloc((size_t)nu * T32_REC));
+  tet32_record_kernel<<<std::min((nu * (T32_D + T32_F) + 255) / 256, 148 * 8), 256, 0, st>>>(g, ub, nu, rec.as<unsigned char>());
+  RB_TRY(check_launch("tet32_record_kernel"));
   // too few points for the GPU: split the tetrahedra as well
-  const int64_t target = 148 * 6;
+  const int64_t target = 148 * 8;
   int nchunk = nblk < target ? (int)((target + nblk - 1) / nblk) : 1;
   nchunk = std::min(std::min(nchunk, nu), 65535);
   const int chunk = (nu + nchunk - 1) / nchunk;
@@ -331,26 +352,13 @@ int launch_ppt(const GeomView &g, const double *d_pts, int64_t npts, const unsig
     RB_TRY(scratch.alloc((size_t)nchunk * npts * 3 * sizeof(double)));
     dst = scratch.as<double>();
   }
-  field_tet32_kernel<PPT><<<dim3((unsigned)nblk, (unsigned)nchunk), 128, 0, st>>>(g, d_pts, npts, perm, what, dst, ub, ue, chunk,
-                                                                                 nchunk > 1 ? 0 : accumulate);
+  field_tet32_kernel<<<dim3((unsigned)nblk, (unsigned)nchunk), T32_T, 0, st>>>(rec.as<unsigned char>(), d_pts, npts, order.perm,
+                                                                              what, dst, nu, chunk, nchunk > 1 ? 0 : accumulate);
   RB_TRY(check_launch("field_tet32_kernel"));
   if (nchunk == 1) return 0;
   const int64_t n3 = npts * 3;
   tet32_reduce_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(scratch.as<double>(), nchunk, n3, d_out, accumulate);
   return check_launch("tet32_reduce_kernel");
-}
-
-}  // namespace
-
-#ifndef T32_PPT
-#define T32_PPT 1
-#endif
-int launch_tet32_field(const GeomView &g, const double *d_pts, int64_t npts, int what, double *d_out, int ub, int ue,
-                       int accumulate, DBuf &scratch, cudaStream_t st)
-{
-  PointOrder order;
-  if (npts >= T32_SORT_MIN && npts <= INT32_MAX) RB_TRY(order.build(d_pts, npts, st));
-  return launch_ppt<T32_PPT>(g, d_pts, npts, order.perm, what, d_out, ub, ue, accumulate, scratch, st);
 }
 
 }  // namespace rb

@@ -101,6 +101,26 @@ struct DBuf {
   template <typename T> T *as() const { return (T *)p; }
 };
 
+// A part of a block that several host arrays were brought into together.
+struct DRef {
+  void *p = nullptr;
+  template <typename T> T *as() const { return (T *)p; }
+};
+// Host arrays for one block: parts up to STAGE_MAX go through one buffer and one
+// copy (a copy from pageable memory costs about 8 us whatever its size, and a
+// small geometry has a dozen arrays), larger ones are copied from where they are.
+struct Staging {
+  static constexpr size_t STAGE_MAX = 256 << 10;
+  struct Part {
+    DRef *ref;
+    const void *src;
+    size_t bytes, off;
+  };
+  std::vector<Part> parts;
+  void add(DRef &ref, const void *src, size_t bytes) { parts.push_back({&ref, src, bytes, 0}); }
+  int upload(DBuf &blob);
+};
+
 // ---- tetrahedral meshes by their unique vertices, edges and faces -----------
 // The vertex/edge form sums, per tetrahedron, a logarithm per edge and a
 // solid angle per face.  Tetrahedra of a mesh share vertices, edges and
@@ -157,13 +177,16 @@ struct GeomView {
 };
 
 struct DevGeom {
-  DBuf trf, rec, rec_img, poly, poly_info, face, face_vtx, vtx2d, edge, arc, bkg, units;
+  DBuf blob, topo_blob;  // hold the arrays that came from the host
+  DRef trf, rec, rec_img, poly, poly_info, face, face_vtx, vtx2d, arc, bkg, units;
+  DBuf edge;
   // polyhedron topology (vertex/edge form), see TopoView in formulas.cuh
-  DBuf tinfo, tinfo2, tv, te, tel, teg, teG, tt, ttm, tfn, tfa;
+  DRef tinfo, tinfo2, tv, te, tel, teg, teG, tt, ttm, tfn, tfa;
   DBuf tri;             // triangle faces of the face form (tri_face)
   int all_tri = 0;
-  DBuf tetidx, tetrec;  // fixed-topology tetrahedron records (tet_fast)
-  DBuf m_tile, m_v, m_e, m_f, m_group, m_gbox, m_gtet;  // mesh form (MeshView)
+  DRef tetidx, tetrec;  // fixed-topology tetrahedron records (tet_fast)
+  DBuf mesh_blob;
+  DRef m_tile, m_v, m_e, m_f, m_group, m_gbox, m_gtet;  // mesh form (MeshView)
   int m_tiles = 0, m_groups = 0;
   int n_units = 0, n_rec = 0, n_poly = 0;
   int ustart[5] = {0, 0, 0, 0, 0};
@@ -174,6 +197,7 @@ struct DevGeom {
   // coefficients
   enum Form { FACES, FIELD, MESH, TENSOR };
   int upload(const RadB200Geom *G, Form form);
+  int upload_topo(const RadB200Geom *G, Form form);
   GeomView view(int fast = 0) const;
 };
 
@@ -202,7 +226,8 @@ struct Intrc {
   int fast = 0;     // polyhedra in the vertex/edge form
   int geom_ok = 1;  // 0: loaded from a matrix assembled elsewhere (no element geometry)
   DevGeom geom;     // relaxable elements (object frames, images)
-  DBuf elem_src, obs, rowT;           // [2n] int, [3n] obs points, [9n] s*Minv of main image
+  DBuf elem_blob;
+  DRef elem_src, obs, rowT;           // [2n] int, [3n] obs points, [9n] s*Minv of main image
   DBuf N32, N64;                      // [n3 x ld]
   DBuf near_ptr, near_row, near_col, near_D, near_tptr, near_tidx;  // mixed storage: FP64 residue of near pairs
   int64_t near_nnz = 0;
@@ -233,7 +258,11 @@ struct Intrc {
   double lu_shift = 0.0;              // sigma when the factors are of A + sigma I (a pivot fell below the threshold)
   int lu_solve_id = -1;
   int solve_id = 0;                   // counts relaxations / direct solves on this interaction
-  uint64_t stamp = 0;                 // hash of the element records, frames and materials
+  // hash of the element records, frames and materials as created, for saved
+  // states (intrc_stamp): formed at the first save or restore
+  uint64_t stamp = 0;
+  bool has_stamp = false;
+  std::vector<double> h_obs, h_rowT;
   DBuf lastM, lastH;                  // converged state of the last solve
   int last_kind = -1;                 // 0 relax, 1 direct
   // adjoint: external sources (kept for the gradient of H_ext at the centres),

@@ -28,8 +28,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <map>
-#include <tuple>
-#include <unordered_map>
+#include <vector>
 
 #include "internal.cuh"
 
@@ -37,16 +36,46 @@ namespace rb {
 
 namespace {
 
-struct KeyHash {
-  size_t operator()(const std::tuple<long long, long long, long long> &k) const
+// Numbers 0, 1, .. for keys of K words in order of first sight: open addressing
+// in one table sized for all keys at most half full (the node-based map of the
+// standard library took two thirds of the mesh form's 7 ms for 6,000
+// tetrahedra).
+template <int K> class KeyIndex {
+ public:
+  explicit KeyIndex(size_t most)
   {
-    uint64_t h = 1469598103934665603ULL;
-    for (long long v : {std::get<0>(k), std::get<1>(k), std::get<2>(k)}) {
-      h ^= (uint64_t)v;
-      h *= 1099511628211ULL;
-    }
-    return (size_t)h;
+    size_t n = 16;
+    while (n < 2 * most) n <<= 1;
+    slot.assign(n, -1);
+    keys.reserve(K * most);
   }
+  // the key's number; fresh says whether it is new
+  int number(const uint64_t *k, bool &fresh)
+  {
+    uint64_t h = 0x9e3779b97f4a7c15ULL;
+    for (int w = 0; w < K; w++) {
+      h = (h ^ k[w]) * 0xff51afd7ed558ccdULL;
+      h ^= h >> 32;
+    }
+    const size_t mask = slot.size() - 1;
+    for (size_t q = h & mask;; q = (q + 1) & mask) {
+      const int id = slot[q];
+      if (id < 0) {
+        slot[q] = (int)(keys.size() / K);
+        keys.insert(keys.end(), k, k + K);
+        fresh = true;
+        return slot[q];
+      }
+      if (std::equal(k, k + K, &keys[(size_t)K * id])) {
+        fresh = false;
+        return id;
+      }
+    }
+  }
+
+ private:
+  std::vector<int> slot;
+  std::vector<uint64_t> keys;
 };
 
 uint32_t spread10(uint32_t x)
@@ -95,24 +124,20 @@ void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, 
   // unique vertices: copies of one vertex in different tetrahedra are
   // reconstructed from different face frames, so they are merged on a grid of
   // 1e-12 of the mesh's extent (a vertex not merged is only evaluated twice)
-  std::unordered_map<std::tuple<long long, long long, long long>, int, KeyHash> vid;
+  KeyIndex<3> vid((size_t)nt * 4);
   std::vector<double> V;
   std::vector<int> tv((size_t)nt * 4);
   for (int k = 0; k < nt; k++)
     for (int v = 0; v < 4; v++) {
       const double *p = rec(k) + 3 * v;
-      auto key = std::make_tuple(llround((p[0] - lo[0]) / tol), llround((p[1] - lo[1]) / tol), llround((p[2] - lo[2]) / tol));
-      auto it = vid.find(key);
-      int id;
-      if (it == vid.end()) {
-        id = (int)(V.size() / 3);
-        vid.emplace(key, id);
-        V.insert(V.end(), p, p + 3);
-      } else id = it->second;
-      tv[4 * (size_t)k + v] = id;
+      const uint64_t key[3] = {(uint64_t)llround((p[0] - lo[0]) / tol), (uint64_t)llround((p[1] - lo[1]) / tol),
+                               (uint64_t)llround((p[2] - lo[2]) / tol)};
+      bool fresh;
+      tv[4 * (size_t)k + v] = vid.number(key, fresh);
+      if (fresh) V.insert(V.end(), p, p + 3);
     }
   // unique edges and faces with their summed coefficients
-  std::unordered_map<uint64_t, int> eid, fid;
+  KeyIndex<1> eid((size_t)nt * 6), fid((size_t)nt * 4);
   std::vector<double> G;             // 3 per edge
   std::vector<int> ev;               // 2 per edge
   std::vector<double> A, M;          // 3 per face: coefficient, unnormalized normal (own orientation)
@@ -123,15 +148,13 @@ void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, 
     for (int e = 0; e < 6; e++) {
       int a = tv[4 * k + tet_edge_a(e)], b = tv[4 * k + tet_edge_b(e)];
       uint64_t key = ((uint64_t)std::min(a, b) << 32) | (uint32_t)std::max(a, b);
-      auto it = eid.find(key);
-      int id;
-      if (it == eid.end()) {
-        id = (int)(ev.size() / 2);
-        eid.emplace(key, id);
+      bool fresh;
+      const int id = eid.number(&key, fresh);
+      if (fresh) {
         ev.push_back(a);
         ev.push_back(b);
         G.insert(G.end(), 3, 0.0);
-      } else id = it->second;
+      }
       for (int c = 0; c < 3; c++) G[3 * (size_t)id + c] += r[42 + 3 * e + c];
       te[6 * (size_t)k + e] = id;
     }
@@ -139,12 +162,10 @@ void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, 
       int a = tv[4 * k + tet_face_a(f)], b = tv[4 * k + tet_face_b(f)], c = tv[4 * k + tet_face_c(f)];
       int s0 = std::min(a, std::min(b, c)), s2 = std::max(a, std::max(b, c)), s1 = a + b + c - s0 - s2;
       uint64_t key = ((uint64_t)s0 << 42) | ((uint64_t)s1 << 21) | (uint64_t)s2;
-      auto it = fid.find(key);
-      int id;
       const double *m = r + 18 + 3 * f;
-      if (it == fid.end()) {
-        id = (int)(fv.size() / 3);
-        fid.emplace(key, id);
+      bool fresh;
+      const int id = fid.number(&key, fresh);
+      if (fresh) {
         fv.push_back(a);
         fv.push_back(b);
         fv.push_back(c);
@@ -155,7 +176,7 @@ void build_group(const std::vector<int> &polys, const std::vector<int> &tetidx, 
         if (mm[0] * m[0] + mm[1] * m[1] + mm[2] * m[2] < 0) { mm[0] = -mm[0]; mm[1] = -mm[1]; mm[2] = -mm[2]; }
         M.insert(M.end(), mm, mm + 3);
         A.insert(A.end(), 3, 0.0);
-      } else id = it->second;
+      }
       const double *mm = &M[3 * (size_t)id];
       const double s = (mm[0] * m[0] + mm[1] * m[1] + mm[2] * m[2] < 0) ? -1.0 : 1.0;
       for (int c2 = 0; c2 < 3; c2++) A[3 * (size_t)id + c2] += s * r[30 + 3 * f + c2];
@@ -251,13 +272,15 @@ int build_mesh(const RadB200Geom *G, const std::vector<int> &tetidx, const std::
   }
   MeshHost h;
   for (auto &g : groups) build_group(g.second, tetidx, tetrec, g.first, h);
-  RB_TRY(dg.m_tile.upload(h.tile.data(), h.tile.size() * sizeof(int4)));
-  RB_TRY(dg.m_v.upload(h.v.data(), h.v.size() * sizeof(double)));
-  RB_TRY(dg.m_e.upload(h.e.data(), h.e.size() * sizeof(double)));
-  RB_TRY(dg.m_f.upload(h.f.data(), h.f.size() * sizeof(double)));
-  RB_TRY(dg.m_group.upload(h.group.data(), h.group.size() * sizeof(int4)));
-  RB_TRY(dg.m_gbox.upload(h.gbox.data(), h.gbox.size() * sizeof(double)));
-  RB_TRY(dg.m_gtet.upload(h.gtet.data(), h.gtet.size() * sizeof(int)));
+  Staging st;
+  st.add(dg.m_tile, h.tile.data(), h.tile.size() * sizeof(int4));
+  st.add(dg.m_v, h.v.data(), h.v.size() * sizeof(double));
+  st.add(dg.m_e, h.e.data(), h.e.size() * sizeof(double));
+  st.add(dg.m_f, h.f.data(), h.f.size() * sizeof(double));
+  st.add(dg.m_group, h.group.data(), h.group.size() * sizeof(int4));
+  st.add(dg.m_gbox, h.gbox.data(), h.gbox.size() * sizeof(double));
+  st.add(dg.m_gtet, h.gtet.data(), h.gtet.size() * sizeof(int));
+  RB_TRY(st.upload(dg.mesh_blob));
   dg.m_tiles = (int)(h.tile.size() / 2);
   dg.m_groups = (int)h.group.size();
   return 0;

@@ -31,7 +31,7 @@ __device__ __forceinline__ void elem_tensor(const GeomView &g, int kind, int idx
     cuboid_tensor(g, idx, q, Q);
     return;
   }
-  if (g.fast && __ldg(&g.tp.tinfo[idx].y) >= 0) {  // vertex/edge form
+  if (g.fast && (g.all_tets || __ldg(&g.tp.tinfo[idx].y) >= 0)) {  // vertex/edge form
     int ti = __ldg(g.tetidx + idx);
     if (ti >= 0) tet_fast<double, true>(g.tetrec + (size_t)ti * TET_REC_TENSOR, q, Q);
     else poly_fast<double, true>(g.tp, idx, q, Q);

@@ -804,8 +804,8 @@ class Interaction:
         self.last_status = None
 
     def writeback(self, M: np.ndarray):
-        for e, lf in enumerate(self.pack.leaves):
-            lf.obj.m = M[3 * e:3 * e + 3].copy()
+        for lf, m in zip(self.pack.leaves, M.reshape(-1, 3).copy()):
+            lf.obj.m = m
         self.M = M
 
 

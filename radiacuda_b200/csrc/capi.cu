@@ -1041,7 +1041,6 @@ int radb200_intrc_set_materials(int64_t handle, const RadB200Relax *r)
   intrc_stamp(*I);  // of the materials it was created with
   RB_TRY(upload_materials(*I, r));
   // factors and the converged state belong to the old materials
-  I->drop_lu_graphs();
   I->lu_mode = -1;
   I->lu_of_d = 0;
   I->last_kind = -1;

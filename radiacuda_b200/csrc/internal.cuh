@@ -250,7 +250,7 @@ struct Intrc {
   // LU factors (row-major [n3 x ld]) and solve state
   DBuf LU32, LU64, lu_scratch;
   DBuf LUinv;                         // [2][3N x 128] inverses of the diagonal blocks (L, then U)
-  DBuf tri_sync;                      // counters and flags of the one-launch triangular sweeps
+  DBuf tri_sync;                      // vectors and counters of the triangular sweeps
   DBuf sweep_m;                       // FP32 factors: per block Linv_k L_{k,k-1}, then Uinv_k U_{k,k+1} (128 x 128 each)
   int lu_tc = 0;                      // the factorization ran on the tensor cores
   int lu_mode = -1;                   // factors valid for this mode (-1 none)
@@ -271,17 +271,6 @@ struct Intrc {
   int has_ext = 0;
   std::vector<int> h_elem_src;        // [2n]
   std::vector<double> h_obsJ;         // [9n] row-major
-  // the triangular solves with the current factors, captured once as CUDA
-  // graphs ([0] A^-1, [1] A^-T) acting on lu_gx; dropped when the factors change
-  cudaGraphExec_t lu_graph[2] = {nullptr, nullptr};
-  long long lu_graph_kernels[2] = {0, 0};  // kernels per replay (launch counter)
-  DBuf lu_gx;
-  void drop_lu_graphs()
-  {
-    for (auto &g : lu_graph)
-      if (g) { cudaGraphExecDestroy(g); g = nullptr; }
-  }
-  ~Intrc() { drop_lu_graphs(); }
 };
 
 // ---- small vector helpers (relax.cu) ---------------------------------------
@@ -314,6 +303,7 @@ int gmres(Op &op, int n3, int ld, const double *b, double *x, double rtol, int m
 int lu_precond(Intrc &I, double *x, cudaStream_t st);
 int relax_jacobi(Intrc &I, double prec, int max_iter, double omega0, double *status);
 int lu_precond_transposed(Intrc &I, double *x, cudaStream_t st);
+int tri_sweep_error(int *flag);  // 1 when a wait of the sweeps ran out
 // factor A = I - X N with X [n x RADB200_MAT_STRIDE] (3x3 in the first 9
 // slots) into the interaction's LU buffers; of_d marks factors of I - D N
 int lu_build_x(Intrc &I, int mode, const double *X, int of_d, double *factor_seconds);

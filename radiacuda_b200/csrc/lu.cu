@@ -27,7 +27,7 @@
 //               gemm_tc.cu), then right-preconditioned FP64 GMRES on A with
 //               the FP64 residual (GMRES-IR).
 // Triangular solves with the factors use the stored diagonal-block inverses
-// (one persistent launch per sweep, tri_sweep_kernel).
+// (one persistent launch per sweep, lu_sweep.cuh).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -35,6 +35,7 @@
 
 #include "internal.cuh"
 #include "lu_diag.cuh"
+#include "lu_sweep.cuh"
 
 namespace rb {
 
@@ -80,6 +81,7 @@ __global__ void apply_A_kernel(const double *__restrict__ x, const double *__res
 
 // ---- diagonal block: factor (unpivoted) and invert both triangles: one CTA,
 // blocked by 32 in shared memory (lu_diag.cuh)
+static_assert(SW_NB == LU_NB, "the sweeps work on LU_NB blocks");
 static_assert(DG_N == LU_NB, "the diagonal-block kernel works on LU_NB x LU_NB blocks");
 
 // ---- CUDA-core GEMM: C[m x n] (=|-=) A[m x k] B[k x n]; 64x64 tile, k-slices of 16
@@ -205,122 +207,6 @@ static int gemm_to(T *dst, int ldd, int m, int n, int k, T *A, int lda, const T 
   }
   RB_TRY(gemm<T>(tmp, ldt, m, n, k, A, lda, B, ldb, 1, st, tc_used));
   return copy2d<T>(dst, ldd, tmp, ldt, m, n, st);
-}
-
-// ---- triangular solves with the factors (in place on x, FP64) ----
-// dot of a 128-wide row (16-byte aligned, zero beyond nb) with xs, across a warp
-__device__ __forceinline__ double row128_dot(const float *row, const double *xs, int lane)
-{
-  float4 v = __ldg(reinterpret_cast<const float4 *>(row) + lane);
-  const double *xp = xs + 4 * lane;
-  return (double)v.x * xp[0] + (double)v.y * xp[1] + (double)v.z * xp[2] + (double)v.w * xp[3];
-}
-__device__ __forceinline__ double row128_dot(const double *row, const double *xs, int lane)
-{
-  double2 v0 = __ldg(reinterpret_cast<const double2 *>(row) + lane);
-  double2 v1 = __ldg(reinterpret_cast<const double2 *>(row) + 32 + lane);
-  return v0.x * xs[2 * lane] + v0.y * xs[2 * lane + 1] + v1.x * xs[64 + 2 * lane] + v1.y * xs[64 + 2 * lane + 1];
-}
-__device__ __forceinline__ double warp_sum(double s)
-{
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  return s;
-}
-
-// x[k0:k0+nb] <- Inv_k x[k0:k0+nb]   (Inv = L^-1 or U^-1 of diagonal block k,
-// pitch 128 with zero columns beyond nb); warp per row
-template <typename T>
-__global__ void __launch_bounds__(256) block_matvec_kernel(const T *__restrict__ Inv, int k0, int nb, double *__restrict__ x)
-{
-  __shared__ double xs[LU_NB];
-  if (threadIdx.x < LU_NB) xs[threadIdx.x] = threadIdx.x < nb ? x[k0 + threadIdx.x] : 0.0;
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = warp; r < nb; r += 8) {
-    double s = warp_sum(row128_dot(Inv + (size_t)(k0 + r) * LU_NB, xs, lane));
-    if (lane == 0) x[k0 + r] = s;
-  }
-}
-
-// x[rows r0..r1) -= A[rows, k0:k0+nb] x[k0:k0+nb] (warp per row, 16-byte loads
-// when the panel is a full 128 wide)
-template <typename T>
-__global__ void __launch_bounds__(256) panel_gemv_kernel(const T *__restrict__ A, int ld, int k0, int nb, int r0, int r1,
-                                                         double *__restrict__ x)
-{
-  __shared__ double xs[LU_NB];
-  for (int r = threadIdx.x; r < LU_NB; r += blockDim.x) xs[r] = r < nb ? x[k0 + r] : 0.0;
-  __syncthreads();
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int row = r0 + blockIdx.x * 8 + warp;
-  if (row >= r1) return;
-  const T *a = A + (size_t)row * ld + k0;
-  double s = 0.0;
-  if (nb == LU_NB) s = row128_dot(a, xs, lane);
-  else
-    for (int j = lane; j < nb; j += 32) s += (double)a[j] * xs[j];
-  s = warp_sum(s);
-  if (lane == 0) x[row] -= s;
-}
-
-// ---- transposed solves, A^T = U^T L^T (adjoint) ----
-// x[k0:k0+nb] <- Inv_k^T x[k0:k0+nb]
-template <typename T>
-__global__ void __launch_bounds__(LU_NB) block_matvec_t_kernel(const T *__restrict__ Inv, int k0, int nb, double *__restrict__ x)
-{
-  __shared__ double xs[LU_NB];
-  int r = threadIdx.x;
-  if (r < nb) xs[r] = x[k0 + r];
-  __syncthreads();
-  if (r < nb) {
-    double s = 0.0;
-    for (int j = 0; j < nb; j++) s += (double)Inv[(size_t)(k0 + j) * LU_NB + r] * xs[j];
-    x[k0 + r] = s;
-  }
-}
-
-// x[c0..c1) -= A[k0:k0+nb, c0..c1)^T x[k0:k0+nb] (thread per column, coalesced rows)
-template <typename T>
-__global__ void __launch_bounds__(256) panel_gemv_t_kernel(const T *__restrict__ A, int ld, int k0, int nb, int c0, int c1,
-                                                           double *__restrict__ x)
-{
-  __shared__ double xs[LU_NB];
-  for (int r = threadIdx.x; r < nb; r += blockDim.x) xs[r] = x[k0 + r];
-  __syncthreads();
-  int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= c1) return;
-  const T *a = A + (size_t)k0 * ld + c;
-  double s = 0.0;
-  for (int r = 0; r < nb; r++) s += (double)a[(size_t)r * ld] * xs[r];
-  x[c] -= s;
-}
-
-template <typename T>
-static int lu_solve_t(const T *A, const T *Linv, const T *Uinv, int n3, int ld, double *x, cudaStream_t st)
-{
-  // U^T y = x, forward over the block rows of U
-  for (int k0 = 0; k0 < n3; k0 += LU_NB) {
-    int nb = std::min(LU_NB, n3 - k0);
-    block_matvec_t_kernel<T><<<1, LU_NB, 0, st>>>(Uinv, k0, nb, x);
-    RB_TRY(check_launch("block_matvec_t_kernel"));
-    int rest = k0 + nb;
-    if (rest < n3) {
-      panel_gemv_t_kernel<T><<<(n3 - rest + 255) / 256, 256, 0, st>>>(A, ld, k0, nb, rest, n3, x);
-      RB_TRY(check_launch("panel_gemv_t_kernel"));
-    }
-  }
-  // L^T z = y, backward over the block rows of L
-  int last = ((n3 - 1) / LU_NB) * LU_NB;
-  for (int k0 = last; k0 >= 0; k0 -= LU_NB) {
-    int nb = std::min(LU_NB, n3 - k0);
-    block_matvec_t_kernel<T><<<1, LU_NB, 0, st>>>(Linv, k0, nb, x);
-    RB_TRY(check_launch("block_matvec_t_kernel"));
-    if (k0 > 0) {
-      panel_gemv_t_kernel<T><<<(k0 + 255) / 256, 256, 0, st>>>(A, ld, k0, nb, 0, k0, x);
-      RB_TRY(check_launch("panel_gemv_t_kernel"));
-    }
-  }
-  return 0;
 }
 
 // Optional CUDA-event timing of the trailing updates (A22 -= L21 U12) on the
@@ -608,244 +494,6 @@ static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, doubl
   return 0;
 }
 
-// ---- triangular sweeps in one launch per factor ---------------------------------
-// Forward with the unit-lower factor: x_k = Linv_k (b_k - sum_{j<k} L_kj x_j);
-// backward with U: x_k = Uinv_k (b_k - sum_{j>k} U_kj x_j), blocks of 128.
-// One persistent launch per sweep: each CTA takes the next block in sweep
-// order from an atomic counter, subtracts the products with the blocks already
-// solved as their flags appear (streaming its row panel of the factor while
-// the chain of blocks advances), applies the diagonal block's inverse, and
-// publishes x_k and its flag (release; readers acquire, then read x_j through
-// L2).  A CTA waits only on blocks taken before its own by CTAs that are
-// running, so every wait ends; each is also bounded by TRI_SPIN polls, after
-// which the launch records an error in *err and every CTA returns.
-// sync layout: [counter, flags of the blocks]; zeroed before each sweep.
-constexpr long long TRI_SPIN = 1ll << 24;
-
-__device__ __forceinline__ int ld_acquire_s32(const int *p)
-{
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_s32(int *p, int v)
-{
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// One lane's slice of a 128-wide row of the factor (or of a diagonal-block
-// inverse), loaded ahead of use, and its dot product with xs.
-template <typename T> struct RowSlice;
-template <> struct RowSlice<float> {
-  float4 v;
-  __device__ __forceinline__ void set(float4 q) { v = q; }
-  __device__ __forceinline__ void load(const float *row, int lane) { v = __ldg(reinterpret_cast<const float4 *>(row) + lane); }
-  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ double dot(const double *xs, int lane) const
-  {
-    const double *xp = xs + 4 * lane;
-    return (double)v.x * xp[0] + (double)v.y * xp[1] + (double)v.z * xp[2] + (double)v.w * xp[3];
-  }
-};
-template <> struct RowSlice<double> {
-  double2 a, b;
-  __device__ __forceinline__ void set(float4) {}  // unused: inverses are staged for float factors only
-  __device__ __forceinline__ void load(const double *row, int lane)
-  {
-    a = __ldg(reinterpret_cast<const double2 *>(row) + lane);
-    b = __ldg(reinterpret_cast<const double2 *>(row) + 32 + lane);
-  }
-  __device__ __forceinline__ void zero() { a = b = make_double2(0.0, 0.0); }
-  __device__ __forceinline__ double dot(const double *xs, int lane) const
-  {
-    return a.x * xs[2 * lane] + a.y * xs[2 * lane + 1] + b.x * xs[64 + 2 * lane] + b.y * xs[64 + 2 * lane + 1];
-  }
-};
-
-// rows per warp per batch: 8 warps x TRI_ROWS<T> x TRI_BATCH<T> = 128 rows
-template <typename T> constexpr int tri_rows() { return sizeof(T) == 4 ? 16 : 8; }
-
-template <typename T, bool UPPER>
-__global__ void __launch_bounds__(256, 2) tri_sweep_kernel(const T *__restrict__ A, int ld, const T *__restrict__ Inv, int n3,
-                                                        double *x, int *sync, int *err, const float *__restrict__ Msub)
-{
-  constexpr int NR = tri_rows<T>(), NB = LU_NB / (8 * NR);  // rows per batch, batches
-  constexpr bool STAGE_INV = sizeof(T) == 4;  // Inv_k in shared memory (dynamic, LU_NB^2 floats)
-  extern __shared__ float4 sinv4[];
-  __shared__ double xs[LU_NB], acc_s[LU_NB];
-  __shared__ int s_t, s_bad;
-  const int nblk = (n3 + LU_NB - 1) / LU_NB;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int *flags = sync + 1;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) { s_t = atomicAdd(sync, 1); s_bad = 0; }
-    __syncthreads();
-    const int t = s_t;
-    if (t >= nblk) return;
-    const int k = UPPER ? nblk - 1 - t : t;
-    const int k0 = k * LU_NB, nb = min(LU_NB, n3 - k0);
-    // this warp's rows: (warp * NB + batch) * NR + i, accumulated in shared
-    // memory by the warp's lane 0 (every row belongs to one warp)
-    if (threadIdx.x < LU_NB) acc_s[threadIdx.x] = threadIdx.x < nb ? x[k0 + threadIdx.x] : 0.0;
-    // with coupling blocks (FP32 factors, Msub): everything but the block
-    // before this one in sweep order is done first and multiplied by the
-    // inverse while that block is solved; x_k = y_k - M_k x_j then remains
-    const bool use_m = STAGE_INV && Msub != nullptr && t > 0;
-    // the matrix needed last, on the chain's critical path (M_k, or the
-    // diagonal block's inverse): staged now (visible after the barriers
-    // below), while the chain is still far from this block
-    if constexpr (STAGE_INV) {
-      const float *src = use_m ? Msub + (size_t)k * LU_NB * LU_NB : Inv + (size_t)k0 * LU_NB;
-      for (int e = threadIdx.x; e < LU_NB * LU_NB / 4; e += blockDim.x) {
-        const int r = e / (LU_NB / 4);
-        sinv4[e] = (use_m || r < nb) ? __ldg(reinterpret_cast<const float4 *>(src + (size_t)r * LU_NB) + (e % (LU_NB / 4)))
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    const int s_end = use_m ? t - 1 : t;
-    for (int s = 0; s < s_end; s++) {
-      const int j = UPPER ? nblk - 1 - s : s;
-      const int j0 = j * LU_NB, nbj = min(LU_NB, n3 - j0);
-      const bool full = (nbj == LU_NB);
-      // the tile's first batch is loaded before the wait: it does not depend on x_j
-      RowSlice<T> v[NR];
-      if (full) {
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-          const int r = warp * NB * NR + i;
-          if (r < nb) v[i].load(A + (size_t)(k0 + r) * ld + j0, lane);
-          else v[i].zero();
-        }
-      }
-      if (threadIdx.x == 0) {
-        long long it = 0;
-        while (ld_acquire_s32(flags + j) == 0) {
-          if (++it > TRI_SPIN || ld_acquire_s32(err) != 0) { s_bad = 1; atomicExch(err, 1); break; }
-        }
-      }
-      __syncthreads();  // the flag seen; every warp done with the previous xs
-      if (s_bad) return;
-      if (threadIdx.x < LU_NB) xs[threadIdx.x] = threadIdx.x < nbj ? __ldcg(x + j0 + threadIdx.x) : 0.0;
-      __syncthreads();
-      if (full) {
-#pragma unroll
-        for (int b = 0; b < NB; b++) {
-          if (b > 0) {
-#pragma unroll
-            for (int i = 0; i < NR; i++) {
-              const int r = (warp * NB + b) * NR + i;
-              if (r < nb) v[i].load(A + (size_t)(k0 + r) * ld + j0, lane);
-              else v[i].zero();
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < NR; i++) {
-            const double w = warp_sum(v[i].dot(xs, lane));
-            if (lane == 0) acc_s[(warp * NB + b) * NR + i] -= w;
-          }
-        }
-      } else {
-        // the last, partial block: masked columns
-#pragma unroll
-        for (int b = 0; b < NB; b++)
-#pragma unroll
-          for (int i = 0; i < NR; i++) {
-            const int r = (warp * NB + b) * NR + i;
-            double w = 0.0;
-            if (r < nb) {
-              const T *a = A + (size_t)(k0 + r) * ld + j0;
-              for (int c = lane; c < nbj; c += 32) w += (double)a[c] * xs[c];
-            }
-            w = warp_sum(w);
-            if (lane == 0) acc_s[r] -= w;
-          }
-      }
-    }
-    if (use_m) {
-      // y_k = Inv_k acc into acc_s (Inv_k through L2: off the chain)
-      __syncthreads();
-      if (threadIdx.x < LU_NB) xs[threadIdx.x] = threadIdx.x < nb ? acc_s[threadIdx.x] : 0.0;
-      __syncthreads();
-#pragma unroll
-      for (int b = 0; b < NB; b++) {
-        RowSlice<T> v[NR];
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-          const int r = (warp * NB + b) * NR + i;
-          if (r < nb) v[i].load(Inv + (size_t)(k0 + r) * LU_NB, lane);
-          else v[i].zero();
-        }
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-          const int r = (warp * NB + b) * NR + i;
-          const double w = warp_sum(v[i].dot(xs, lane));
-          if (lane == 0) acc_s[r] = w;
-        }
-      }
-      // the block before this one in sweep order
-      const int j = UPPER ? k + 1 : k - 1;
-      const int j0 = j * LU_NB, nbj = min(LU_NB, n3 - j0);
-      if (threadIdx.x == 0) {
-        long long it = 0;
-        while (ld_acquire_s32(flags + j) == 0) {
-          if (++it > TRI_SPIN || ld_acquire_s32(err) != 0) { s_bad = 1; atomicExch(err, 1); break; }
-        }
-      }
-      __syncthreads();  // the flag seen; every warp done with xs
-      if (s_bad) return;
-      if (threadIdx.x < LU_NB) xs[threadIdx.x] = threadIdx.x < nbj ? __ldcg(x + j0 + threadIdx.x) : 0.0;
-      __syncthreads();
-#pragma unroll
-      for (int b = 0; b < NB; b++) {
-        RowSlice<T> v[NR];
-#pragma unroll
-        for (int i = 0; i < NR; i++) v[i].set(sinv4[((warp * NB + b) * NR + i) * (LU_NB / 4) + lane]);
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-          const int r = (warp * NB + b) * NR + i;
-          const double w = warp_sum(v[i].dot(xs, lane));
-          if (lane == 0 && r < nb) x[k0 + r] = acc_s[r] - w;
-        }
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        __threadfence();
-        st_release_s32(flags + k, 1);
-      }
-      continue;
-    }
-    // x_k = Inv_k acc (rows of Inv beyond nb hold zero columns)
-    __syncthreads();
-    if (threadIdx.x < LU_NB) xs[threadIdx.x] = threadIdx.x < nb ? acc_s[threadIdx.x] : 0.0;
-    __syncthreads();
-#pragma unroll
-    for (int b = 0; b < NB; b++) {
-      RowSlice<T> v[NR];
-#pragma unroll
-      for (int i = 0; i < NR; i++) {
-        const int r = (warp * NB + b) * NR + i;
-        if (STAGE_INV) {
-          const float4 q = sinv4[r * (LU_NB / 4) + lane];
-          v[i].set(q);
-        } else if (r < nb) v[i].load(Inv + (size_t)(k0 + r) * LU_NB, lane);
-        else v[i].zero();
-      }
-#pragma unroll
-      for (int i = 0; i < NR; i++) {
-        const int r = (warp * NB + b) * NR + i;
-        const double w = warp_sum(v[i].dot(xs, lane));
-        if (lane == 0 && r < nb) x[k0 + r] = w;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      st_release_s32(flags + k, 1);
-    }
-  }
-}
-
 // Coupling blocks of FP32 factors for the sweeps: Mf[k] = Linv_k L_{k,k-1}
 // (k >= 1) and Mb[k] = Uinv_k U_{k,k+1} (k < nblk - 1), 128 x 128 each, rows
 // beyond block k's size and columns beyond its neighbour's zero.  With them a
@@ -900,66 +548,7 @@ __global__ void __launch_bounds__(256) sweep_m_kernel(const float *__restrict__ 
     for (int c = 0; c < 8; c++) out[(size_t)(tr * 8 + i) * LU_NB + tc * 8 + c] = acc[i][c];
 }
 
-// RADB200_TRI_SWEEP=0: the per-block launches below instead (A/B comparisons)
-static bool tri_sweep_enabled()
-{
-  static int on = -1;
-  if (on < 0) {
-    const char *e = getenv("RADB200_TRI_SWEEP");
-    on = (e && atoi(e) == 0) ? 0 : 1;
-  }
-  return on == 1;
-}
-
-// RADB200_SWEEP_M=0: FP32 sweeps without coupling blocks (A/B comparisons)
-static bool sweep_m_enabled()
-{
-  static int on = -1;
-  if (on < 0) {
-    const char *e = getenv("RADB200_SWEEP_M");
-    on = (e && atoi(e) == 0) ? 0 : 1;
-  }
-  return on == 1;
-}
-
-static DBuf g_tri_err;  // allocated with the first factors, before any capture
-
-// the sweeps' counters and flags of an interaction (allocated with its factors,
-// so that a captured solve never sees the buffer move)
-static int tri_sync_alloc(Intrc &I)
-{
-  const size_t per = (size_t)(I.n3 + LU_NB - 1) / LU_NB + 1;
-  RB_TRY(I.tri_sync.alloc(2 * per * sizeof(int)));
-  static bool attr = false;
-  if (!attr) {
-    const int dyn = LU_NB * LU_NB * (int)sizeof(float);
-    RB_CUDA(cudaFuncSetAttribute(tri_sweep_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    RB_CUDA(cudaFuncSetAttribute(tri_sweep_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
-    attr = true;
-  }
-  if (!g_tri_err.p) {
-    RB_TRY(g_tri_err.alloc(sizeof(int)));
-    RB_CUDA(cudaMemset(g_tri_err.p, 0, sizeof(int)));
-  }
-  return 0;
-}
-
-template <typename T>
-static int lu_solve_sweeps(const T *A, const T *Linv, const T *Uinv, int n3, int ld, double *x, int *sync,
-                           const float *Mf, const float *Mb, cudaStream_t st)
-{
-  const int nblk = (n3 + LU_NB - 1) / LU_NB;
-  const size_t per = (size_t)nblk + 1;
-  RB_CUDA(cudaMemsetAsync(sync, 0, 2 * per * sizeof(int), st));
-  const int grid = std::min(nblk, 148 * 4);
-  // FP32 factors: the inverses staged in dynamic shared memory (the limit is
-  // raised in tri_sync_alloc, before any capture)
-  const size_t dyn = sizeof(T) == 4 ? (size_t)LU_NB * LU_NB * sizeof(float) : 0;
-  tri_sweep_kernel<T, false><<<grid, 256, dyn, st>>>(A, ld, Linv, n3, x, sync, g_tri_err.as<int>(), Mf);
-  RB_TRY(check_launch("tri_sweep_kernel"));
-  tri_sweep_kernel<T, true><<<grid, 256, dyn, st>>>(A, ld, Uinv, n3, x, sync + per, g_tri_err.as<int>(), Mb);
-  return check_launch("tri_sweep_kernel");
-}
+static DBuf g_tri_err;  // error flag of the sweeps
 
 // error flag of the sweeps: 0, or 1 when a wait ran out (then cleared)
 int tri_sweep_error(int *flag)
@@ -971,107 +560,67 @@ int tri_sweep_error(int *flag)
   return 0;
 }
 
-template <typename T>
-static int lu_solve(const T *A, const T *Linv, const T *Uinv, int n3, int ld, double *x, int *sync, cudaStream_t st,
-                    const float *Mf = nullptr, const float *Mb = nullptr)
+// Buffers of the sweeps for the current factors (also factors that came with a
+// restored state): two vectors, two counters; FP32 factors: coupling blocks.
+static int sweep_prepare(Intrc &I, int mode)
 {
-  if (sync && tri_sweep_enabled()) return lu_solve_sweeps<T>(A, Linv, Uinv, n3, ld, x, sync, Mf, Mb, st);
-  for (int k0 = 0; k0 < n3; k0 += LU_NB) {
-    int nb = std::min(LU_NB, n3 - k0);
-    block_matvec_kernel<T><<<1, 256, 0, st>>>(Linv, k0, nb, x);
-    RB_TRY(check_launch("block_matvec_kernel"));
-    int rest = k0 + nb;
-    if (rest < n3) {
-      panel_gemv_kernel<T><<<(n3 - rest + 7) / 8, 256, 0, st>>>(A, ld, k0, nb, rest, n3, x);
-      RB_TRY(check_launch("panel_gemv_kernel"));
-    }
+  RB_TRY(I.tri_sync.alloc(2 * (size_t)I.ld * sizeof(double) + 2 * sizeof(int)));
+  if (!g_tri_err.p) {
+    RB_TRY(g_tri_err.alloc(sizeof(int)));
+    RB_CUDA(cudaMemset(g_tri_err.p, 0, sizeof(int)));
   }
-  int last = ((n3 - 1) / LU_NB) * LU_NB;
-  for (int k0 = last; k0 >= 0; k0 -= LU_NB) {
-    int nb = std::min(LU_NB, n3 - k0);
-    block_matvec_kernel<T><<<1, 256, 0, st>>>(Uinv, k0, nb, x);
-    RB_TRY(check_launch("block_matvec_kernel"));
-    if (k0 > 0) {
-      panel_gemv_kernel<T><<<(k0 + 7) / 8, 256, 0, st>>>(A, ld, k0, nb, 0, k0, x);
-      RB_TRY(check_launch("panel_gemv_kernel"));
-    }
+  if (mode == RADB200_LU_TF32 && !I.sweep_m.p && I.n3 > LU_NB) {
+    const int nblk = (I.n3 + LU_NB - 1) / LU_NB;
+    RB_TRY(I.sweep_m.alloc(2 * (size_t)nblk * LU_NB * LU_NB * sizeof(float)));
+    const float *inv = I.LUinv.as<float>();
+    float *Mf = I.sweep_m.as<float>(), *Mb = Mf + (size_t)nblk * LU_NB * LU_NB;
+    sweep_m_kernel<<<2 * nblk, 256>>>(I.LU32.as<float>(), I.ld, inv, inv + (size_t)I.n3 * LU_NB, I.n3, Mf, Mb);
+    RB_TRY(check_launch("sweep_m_kernel"));
   }
   return 0;
 }
 
-static int lu_solve_direct(Intrc &I, int transposed, double *x, cudaStream_t st)
+template <typename T> static int sweeps(Intrc &I, const T *A, int transposed, double *x, cudaStream_t st)
 {
-  const int n3 = I.n3, ld = I.ld;
-  if (I.lu_mode == RADB200_LU_F64) {
-    const double *L = I.LUinv.as<double>(), *U = L + (size_t)n3 * LU_NB;
-    return transposed ? lu_solve_t<double>(I.LU64.as<double>(), L, U, n3, ld, x, st)
-                      : lu_solve<double>(I.LU64.as<double>(), L, U, n3, ld, x, I.tri_sync.as<int>(), st);
+  const int n3 = I.n3, ld = I.ld, nblk = (n3 + LU_NB - 1) / LU_NB;
+  double *y = I.tri_sync.as<double>(), *z = y + ld;
+  int *count = reinterpret_cast<int *>(z + ld), *err = g_tri_err.as<int>();
+  const T *L = I.LUinv.as<T>(), *U = L + (size_t)n3 * LU_NB;
+  RB_CUDA(cudaMemsetAsync(y, 0xff, 2 * (size_t)ld * sizeof(double), st));  // SWEEP_EMPTY
+  RB_CUDA(cudaMemsetAsync(count, 0, 2 * sizeof(int), st));
+  int dev = 0, nsm = 0;
+  RB_CUDA(cudaGetDevice(&dev));
+  RB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int grid = std::min(nblk, nsm);
+  auto run = [&](auto kernel, int blocks, auto... args) -> int {
+    const size_t smem = sweep_smem<T>(blocks);
+    RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, SW_T, smem, st>>>(args...);
+    return check_launch("sweep_kernel");
+  };
+  if (transposed) {
+    RB_TRY(run(sweep_t_kernel<T, false>, 1, A, ld, U, n3, x, y, count, err));
+    RB_TRY(run(sweep_t_kernel<T, true>, 1, A, ld, L, n3, y, z, count + 1, err));
+  } else {
+    // (FP64 factors: no coupling blocks)
+    const T *Mf = sizeof(T) == 4 ? I.sweep_m.as<T>() : nullptr, *Mb = Mf ? Mf + (size_t)nblk * LU_NB * LU_NB : nullptr;
+    RB_TRY(run(sweep_kernel<T, false>, Mf ? 2 : 1, A, ld, L, n3, x, y, count, err, Mf));
+    RB_TRY(run(sweep_kernel<T, true>, Mf ? 2 : 1, A, ld, U, n3, y, z, count + 1, err, Mb));
   }
-  if (I.lu_mode == RADB200_LU_TF32) {
-    const float *L = I.LUinv.as<float>(), *U = L + (size_t)n3 * LU_NB;
-    return transposed ? lu_solve_t<float>(I.LU32.as<float>(), L, U, n3, ld, x, st)
-                      : lu_solve<float>(I.LU32.as<float>(), L, U, n3, ld, x, I.tri_sync.as<int>(), st,
-                                        I.sweep_m.p ? I.sweep_m.as<float>() : nullptr,
-                                        I.sweep_m.p ? I.sweep_m.as<float>() + (size_t)((n3 + LU_NB - 1) / LU_NB) * LU_NB * LU_NB
-                                                    : nullptr);
-  }
-  set_error("no LU factors on this interaction");
-  return RADB200_E_ARG;
+  RB_CUDA(cudaMemcpyAsync(x, z, (size_t)n3 * sizeof(double), cudaMemcpyDeviceToDevice, st));
+  return 0;
 }
 
-// x <- A^-1 x (or A^-T x) with the kept factors.  For systems of 64 blocks
-// and more, the ~4 n / 128 small launches of the block sweeps are captured
-// once per factorization into a CUDA graph on a fixed buffer and replayed:
-// one launch per application.
-// RADB200_LU_GRAPH=0 launches the sweeps directly, never capturing them: a
-// per-kernel profiler cannot run a launch made into a capturing stream (the
-// kernel only becomes a graph node there), so launch lists are taken with it.
-static bool lu_graph_enabled()
-{
-  static int on = -1;
-  if (on < 0) {
-    const char *e = getenv("RADB200_LU_GRAPH");
-    on = (e && atoi(e) == 0) ? 0 : 1;
-  }
-  return on == 1;
-}
-
+// x <- A^-1 x (or A^-T x) with the kept factors
 static int lu_apply(Intrc &I, int transposed, double *x, cudaStream_t st)
 {
-  // small systems: a few applications per factorization do not repay a capture
-  if (I.n3 < 64 * LU_NB || !lu_graph_enabled()) return lu_solve_direct(I, transposed, x, st);
-  cudaGraphExec_t &ex = I.lu_graph[transposed];
-  if (!ex) {
-    RB_TRY(I.lu_gx.alloc((size_t)I.ld * sizeof(double)));
-    cudaStream_t cs;
-    RB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaGraph_t graph = nullptr;
-    int rc = 0;
-    cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
-    if (e == cudaSuccess) {
-      const long long before = g_launches;
-      rc = lu_solve_direct(I, transposed, I.lu_gx.as<double>(), cs);
-      I.lu_graph_kernels[transposed] = g_launches - before;
-      g_launches = before;  // captured, not launched
-      e = cudaStreamEndCapture(cs, &graph);
-      if (e == cudaSuccess && rc == 0) e = cudaGraphInstantiate(&ex, graph, 0);
-    }
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cs);
-    if (rc) return rc;
-    if (e != cudaSuccess) {
-      // no graph: run the sweeps directly (same kernels, launched one by one)
-      cudaGetLastError();
-      ex = nullptr;
-      return lu_solve_direct(I, transposed, x, st);
-    }
+  if (I.lu_mode != RADB200_LU_F64 && I.lu_mode != RADB200_LU_TF32) {
+    set_error("no LU factors on this interaction");
+    return RADB200_E_ARG;
   }
-  const size_t bytes = (size_t)I.n3 * sizeof(double);
-  RB_CUDA(cudaMemcpyAsync(I.lu_gx.p, x, bytes, cudaMemcpyDeviceToDevice, st));
-  RB_CUDA(cudaGraphLaunch(ex, st));
-  g_launches += I.lu_graph_kernels[transposed];
-  RB_CUDA(cudaMemcpyAsync(x, I.lu_gx.p, bytes, cudaMemcpyDeviceToDevice, st));
-  return 0;
+  RB_TRY(sweep_prepare(I, I.lu_mode));
+  return I.lu_mode == RADB200_LU_F64 ? sweeps<double>(I, I.LU64.as<double>(), transposed, x, st)
+                                     : sweeps<float>(I, I.LU32.as<float>(), transposed, x, st);
 }
 
 int lu_precond(Intrc &I, double *x, cudaStream_t st) { return lu_apply(I, 0, x, st); }
@@ -1141,7 +690,6 @@ int lu_build_x(Intrc &I, int mode, const double *X, int of_d, double *factor_sec
   auto t0 = std::chrono::steady_clock::now();
   const int n3 = I.n3, ld = I.ld;
   I.lu_mode = -1;
-  I.drop_lu_graphs();
   DBuf err;  // [pivot flag, max |A_ii| as float bits]
   dim3 bgrid((ld + 255) / 256 > 64 ? 64 : (ld + 255) / 256, n3);
   int tc_used = 0;
@@ -1208,16 +756,8 @@ int lu_build_x(Intrc &I, int mode, const double *X, int of_d, double *factor_sec
     set_error("LU: vanishing pivot (A and A + sigma I not factorable without pivoting)");
     return RADB200_E_NUMERIC;
   }
-  RB_TRY(tri_sync_alloc(I));
   I.sweep_m.release();
-  if (mode != RADB200_LU_F64 && sweep_m_enabled() && n3 > LU_NB) {
-    const int nblk = (n3 + LU_NB - 1) / LU_NB;
-    RB_TRY(I.sweep_m.alloc(2 * (size_t)nblk * LU_NB * LU_NB * sizeof(float)));
-    const float *inv = I.LUinv.as<float>();
-    float *Mf = I.sweep_m.as<float>(), *Mb = Mf + (size_t)nblk * LU_NB * LU_NB;
-    sweep_m_kernel<<<2 * nblk, 256>>>(I.LU32.as<float>(), ld, inv, inv + (size_t)n3 * LU_NB, n3, Mf, Mb);
-    RB_TRY(check_launch("sweep_m_kernel"));
-  }
+  RB_TRY(sweep_prepare(I, mode));
   I.lu_mode = mode;
   I.lu_of_d = of_d;
   I.lu_solve_id = I.solve_id;

@@ -1,6 +1,6 @@
-"""The device-resident Anderson iteration and the fused Arnoldi steps at sizes
-around their tiles (128 rows of a basis slice, 256 threads), against dense
-solves of the same matrix."""
+"""The device-resident Anderson iteration, the fused Arnoldi steps and the
+triangular sweeps at sizes around their tiles (128 rows of a block or a basis
+slice, 256 threads), against dense solves of the same matrix."""
 import numpy as np
 import pytest
 
@@ -81,3 +81,38 @@ def test_adjoint_gmres_restarts(cuda, rad):
         nat.free()
     assert st[0] <= 1e-11
     assert rel_err(M, exp) < 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [1, 42, 43, 85, 86, 128, 171])
+def test_triangular_sweeps(cuda, rad, n, mode):
+    """FP64 factors solve to their rounding in one application, FP32 ones in a
+    few refinements, forward and transposed; a restored interaction forms the
+    sweeps' buffers again and gives the same bits."""
+    h = _blocks(rad, n)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    exp = O.linear_direct(pack, O.assemble(pack), O.extfield(pack))
+    g = np.random.default_rng(n + 1).normal(size=3 * n)
+    nat = _native.NativeInteraction(pack, 1)
+    try:
+        nat.relax(1, 1e-13, 500, True, 1.0, np.zeros(3 * n))
+        lam0, st0 = nat.adjoint_solve(g, 1e-13, 200)   # factors of I - D N
+        M, st = nat.direct(mode, 1e-13, 60)
+        lam, sa = nat.adjoint_solve(g, 1e-13, 60)      # the direct solve's own
+        state = nat.save()
+    finally:
+        nat.free()
+    # FP64 factors of these well conditioned matrices leave a residual near
+    # 1e-16, so at most one refinement; FP32 ones gain at least 1e4 per step
+    most = 1 if mode == 0 else 4
+    assert st[0] <= 1e-13 and st[1] <= most
+    assert rel_err(M, exp) < 1e-11
+    assert sa[0] <= 1e-13 and sa[1] <= most + 1 and sa[2] == 1.0
+    assert st0[0] <= 1e-13 and rel_err(lam, lam0) < 1e-11
+    again = _native.NativeInteraction(pack, 1, state)
+    try:
+        lam2, _ = again.adjoint_solve(g, 1e-13, 60)
+    finally:
+        again.free()
+    assert np.array_equal(lam2, lam)

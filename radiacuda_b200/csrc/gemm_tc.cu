@@ -312,16 +312,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_update_kernel(float *__restr
 }
 
 // ---- TMA variant ---------------------------------------------------------------
-// Same tiles and epilogue, but the operands come in by TMA: per K chunk of 32
-// one 2-D bulk tensor load of A (32 x 128) and one of B^T (32 x 256), written
-// by the copy engine in the 128-byte-swizzled K-major layout (8-row x 128-byte
+// Same tiles, but the operands come in by TMA: per K chunk of 128 bytes one
+// 2-D bulk tensor load of A (128 rows) and one of B^T (256 rows), written by
+// the copy engine in the 128-byte-swizzled K-major layout (8-row x 128-byte
 // atoms, 1024-byte aligned) and completed on the stage's "full" mbarrier with
-// a transaction count.  One lane of a producer warp issues the loads and the
-// MMAs through TM_NST stages (loads run TM_NST - 1 chunks ahead; a stage is
-// refilled once the MMAs that read it have committed to its "empty"
-// mbarrier) into two alternating TMEM accumulators; 8 epilogue warps load C
-// and write the results.  Descriptors: start address of the atom + 32 bytes
-// per K=8 step, SBO 1024, layout 128B swizzle.
+// a transaction count.  Descriptors: start address of the atom + 32 bytes per
+// MMA step, SBO 1024, layout 128B swizzle.
 constexpr int TM_KC = 32;
 constexpr int TM_NST = 4;
 constexpr int TM_STAGE_A = TC_BM * TM_KC * 4;   // 16 KB
@@ -369,15 +365,28 @@ __device__ __forceinline__ int tm_wait(uint32_t bar, uint32_t parity)
   return 1;
 }
 
-constexpr int TM_THREADS = 288;  // warps 0-7: epilogue; warp 8: TMA loads and MMAs
+constexpr int TM_THREADS = 320;  // warps 0-7: epilogue; warp 8: TMA loads; warp 9: MMAs
 
-
-// Warp-specialised: warp 8 (one lane) streams the chunks of all of the CTA's
-// tiles through the operand stages into two TMEM accumulators (columns
-// 0-255 and 256-511, alternating per tile) and commits each finished tile to
-// that buffer's "full" barrier; warps 0-7 drain a finished buffer (C loaded
-// beforehand, C - AB stored) and arrive on its "empty" barrier, so the MMAs
-// of tile i+1 run while tile i is written back.  Every wait is bounded.
+// Warp-specialised: one lane of warp 8 keeps the TM_NST operand stages filled
+// (a stage again once the MMAs that read it have committed to its "empty"
+// barrier), one lane of warp 9 issues the MMAs into two alternating TMEM
+// accumulators (columns 0-255 and 256-511) and commits each finished tile to
+// that buffer's "full" barrier; warps 0-7 write a finished buffer back and
+// arrive on its "empty" barrier, so the MMAs of tile i+1 run meanwhile.  Every
+// wait is bounded.
+// What bounds it: up to K of about 1024 the traffic of C (8 bytes an element),
+// above that the operand stream.  Random data, 24,576^2, 148 CTAs:
+//   K                                  128    512    1024   2048
+//   C through registers, one lane for
+//   loads and MMAs                     1.50   1.40   1.61   2.47 ms
+//   this kernel                        1.11   1.12   1.47   2.41 ms
+// (1026 TFLOP/s at K = 2048; C at 4.3 TB/s at K = 128).  Before, a thread held
+// 2 of its 4 slices of C ahead and subtracted in registers: with loads and
+// stores in the epilogue's own chain a tile took 11 us whatever its K.  Now C
+// is never read by the SM: -AB goes to L2 as an FP32 addition of the copy
+// engine (one rounding, as before).  Holding all 4 slices ahead spilled (1.8
+// ms).  The TMA and MMA lanes are two because the divisions and waits of one
+// lane doing both were serial with every chunk.
 // F16: the operands are FP16 copies scaled by powers of two (*scale holds
 // 1 / (sA sB), applied to the accumulator in the epilogue): kind::f16 MMAs of
 // K = 16 (32 bytes of a 128-byte row, as the TF32 K = 8 step), 64 elements
@@ -385,6 +394,7 @@ constexpr int TM_THREADS = 288;  // warps 0-7: epilogue; warp 8: TMA loads and M
 template <bool F16>
 __global__ void __launch_bounds__(TM_THREADS, 1) tc_update_tma_kernel(const __grid_constant__ CUtensorMap tmA,
                                                                       const __grid_constant__ CUtensorMap tmB,
+                                                                      const __grid_constant__ CUtensorMap tmC,
                                                                       float *__restrict__ C, int ldc, int m, int n, int k,
                                                                       int *__restrict__ err, int overwrite,
                                                                       const float *__restrict__ row_scale,
@@ -430,21 +440,37 @@ __global__ void __launch_bounds__(TM_THREADS, 1) tc_update_tma_kernel(const __gr
   const int my_tiles = (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
 
   if (warp == 8) {
-    // ---------------- producer: TMA loads and MMAs (lane 0) ----------------
-    int issued = 0, consumed = 0;
+    // ---------------- TMA loads (one lane) ----------------
     if (lane == 0) {
-      const int G = my_tiles * nch;
-      auto issue = [&](int gg) {
-        const int ii = gg / nch, cc = gg - ii * nch;
-        const int tt = blockIdx.x + ii * gridDim.x;
-        const uint32_t so = s0 + (gg % TM_NST) * TM_STAGE, fb = smem_u32(&full[gg % TM_NST]);
-        mbar_expect_tx(fb, (uint32_t)TM_STAGE);
-        int rr, ccol;
-        tile_rc(tt, tiles_m, tiles_n, rr, ccol);
-        tma_load_2d(so, &tmA, cc * KC, rr, fb);
-        tma_load_2d(so + TM_STAGE_A, &tmB, cc * KC, ccol, fb);
-      };
-      for (; issued < TM_NST - 1 && issued < G; issued++) issue(issued);
+      int st = 0;
+      uint32_t round = 0;
+      for (int i = 0; i < my_tiles && !timed_out; i++) {
+        int row0, col0;
+        tile_rc(blockIdx.x + i * gridDim.x, tiles_m, tiles_n, row0, col0);
+        for (int c = 0; c < nch; c++) {
+          const uint32_t so = s0 + st * TM_STAGE, fb = smem_u32(&full[st]);
+          // the MMAs of the stage's previous chunk are done
+          if (round > 0 && !tm_wait(smem_u32(&empty[st]), (round - 1) & 1)) { timed_out = 1; break; }
+          mbar_expect_tx(fb, (uint32_t)TM_STAGE);
+          tma_load_2d(so, &tmA, c * KC, row0, fb);
+          tma_load_2d(so + TM_STAGE_A, &tmB, c * KC, col0, fb);
+          if (++st == TM_NST) { st = 0; round++; }
+        }
+      }
+      // after a timeout: wait (bounded) for the copies still in flight, the
+      // last one of each stage
+      if (timed_out)
+        for (int j = 0; j < TM_NST; j++) {
+          const uint32_t last = j < st ? round : round - 1;  // round 0: nothing issued
+          if (j < st || round > 0) tm_wait(smem_u32(&full[j]), last & 1);
+        }
+    }
+    __syncwarp();
+  } else if (warp == 9) {
+    // ---------------- MMAs (one lane) ----------------
+    if (lane == 0) {
+      int st = 0;
+      uint32_t round = 0;
       // F16: A and B formats 0 (f16); TF32: 2 (tf32)
       const uint32_t idesc = F16 ? (umma_idesc(0) & ~((7u << 7) | (7u << 10))) : umma_idesc(0);
       for (int i = 0; i < my_tiles && !timed_out; i++) {
@@ -454,37 +480,26 @@ __global__ void __launch_bounds__(TM_THREADS, 1) tc_update_tma_kernel(const __gr
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t dacc = tmem + (uint32_t)(buf * TC_BN);
         for (int c = 0; c < nch; c++) {
-          const int g = i * nch + c, st = g % TM_NST;
-          if (!tm_wait(smem_u32(&full[st]), (uint32_t)((g / TM_NST) & 1))) { timed_out = 1; break; }
-          consumed++;
-          const uint32_t ua = s0 + st * TM_STAGE, ub = ua + TM_STAGE_A;
+          if (!tm_wait(smem_u32(&full[st]), round & 1)) { timed_out = 1; break; }
+          const uint64_t da = umma_desc_sw128(s0 + st * TM_STAGE), db = umma_desc_sw128(s0 + st * TM_STAGE + TM_STAGE_A);
 #pragma unroll
-          for (int s = 0; s < TM_KC / 8; s++) {
-            uint64_t da = umma_desc_sw128(ua + 32u * s);
-            uint64_t db = umma_desc_sw128(ub + 32u * s);
-            uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
+          for (int s = 0; s < TM_KC / 8; s++) {  // 32 bytes of K further each: 2 in the address field
+            const uint32_t acc = (c > 0 || s > 0) ? 1u : 0u;
             if (F16)
               asm volatile(
                   "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                   "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dacc),
-                  "l"(da), "l"(db), "r"(idesc), "r"(acc));
+                  "l"(da + 2 * s), "l"(db + 2 * s), "r"(idesc), "r"(acc));
             else
               asm volatile(
                   "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                   "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dacc),
-                  "l"(da), "l"(db), "r"(idesc), "r"(acc));
+                  "l"(da + 2 * s), "l"(db + 2 * s), "r"(idesc), "r"(acc));
           }
           asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                            smem_u32(&empty[st]))
                        : "memory");
-          if (issued < G) {
-            const int old = issued - TM_NST;  // the chunk whose stage is refilled
-            if (old >= 0 && !tm_wait(smem_u32(&empty[old % TM_NST]), (uint32_t)((old / TM_NST) & 1))) {
-              timed_out = 1;
-              break;
-            }
-            issue(issued++);
-          }
+          if (++st == TM_NST) { st = 0; round++; }
         }
         if (timed_out) break;
         // the tile's accumulators are complete once everything issued so far is
@@ -492,114 +507,86 @@ __global__ void __launch_bounds__(TM_THREADS, 1) tc_update_tma_kernel(const __gr
                          smem_u32(&accf[buf]))
                      : "memory");
       }
-      // after a timeout: wait (bounded) for bulk copies still in flight
-      for (int j = consumed; j < issued; j++) tm_wait(smem_u32(&full[j % TM_NST]), (uint32_t)((j / TM_NST) & 1));
     }
     __syncwarp();
   } else {
     // ---------------- epilogue: warps 0-7 ----------------
     // Warp (q, hc) owns rows q*32.. of the tile (its TMEM lane quarter) and
-    // the column half hc*128.., in four 32-column slices.  C is read and
-    // written row-contiguous: lane l takes 4 columns, (l % 8) * 4.., of row
-    // (l / 8) of every group of 4 rows, so a warp instruction covers four
-    // full 128-byte lines.  The accumulator rows arrive lane = row
-    // (tcgen05.ld 32x32b) and are turned around through a 32 x 32 shared
-    // buffer per warp in 16-byte groups: group g of row r sits at group
-    // position g ^ (r % 8), so the row-wise group writes and the column-wise
-    // group reads of each 8-lane phase hit all 32 banks once.  The tile's C values are loaded before its
-    // accumulator is waited on.
-    const int q = warp & 3, hc = warp >> 2;
+    // the column half hc*128.., in four 32-column slices: accumulators to
+    // registers (lane = row), -AB or AB to the warp's 32 x 32 shared buffer in
+    // the 128-byte-swizzled layout (16-byte group g of row r at g ^ (r % 8):
+    // no bank conflicts), from there by one bulk tensor copy, added to C in L2
+    // (or stored) and clipped at C's edges by the copy engine.  Its rows end at
+    // a multiple of 4 columns (a copy writes 16 bytes at a time); the up to
+    // three columns after that go by plain accesses.
+    const int q = warp & 3, hc = warp >> 2, n4 = n & ~3;
     float *W = reinterpret_cast<float *>(sbase + TM_NST * TM_STAGE) + warp * 32 * 32;
-    const int lr = lane >> 3, lc = (lane & 7) * 4;
     for (int i = 0; i < my_tiles; i++) {
       const int tile = blockIdx.x + i * gridDim.x;
       int row0, col0;
       tile_rc(tile, tiles_m, tiles_n, row0, col0);
       const int buf = i & 1;
       const int rbase = row0 + q * 32, cbase = col0 + hc * 128;
-      // C slice sl (8 float4 per thread) for rows rbase + 4 rr + lr, columns cbase + 32 sl + lc ..:
-      // slices 0 and 1 are loaded before the accumulator wait, slice sl + 2
-      // while slice sl is written back
-      auto load_slice = [&](float4 *cs, int sl) {
-#pragma unroll
-        for (int rr = 0; rr < 8; rr++) {
-          const int gr = rbase + 4 * rr + lr, gc = cbase + 32 * sl + lc;
-          cs[rr] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!overwrite && gr < m) {
-            const float *src = C + (size_t)gr * ldc + gc;
-            if (gc + 3 < n) cs[rr] = *reinterpret_cast<const float4 *>(src);
-            else if (gc < n) {
-              cs[rr].x = src[0];
-              if (gc + 1 < n) cs[rr].y = src[1];
-              if (gc + 2 < n) cs[rr].z = src[2];
-            }
-          }
-        }
-      };
-      auto store_slice = [&](const float4 *cs, int sl) {
-        // FP16 operands: the accumulator carries the row and column factors
-        // (read only for columns inside C: the factors hold n + 8 entries)
-        const int gcs = cbase + 32 * sl + lc;
-        const float4 csc = (F16 && gcs < n) ? __ldg(reinterpret_cast<const float4 *>(col_scale + gcs))
-                                            : make_float4(1.f, 1.f, 1.f, 1.f);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          uint32_t v[16];
-          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TC_BN + hc * 128 + sl * 32 + h * 16);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-              : "r"(taddr));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int c4 = 0; c4 < 4; c4++)
-            *reinterpret_cast<float4 *>(W + lane * 32 + (((h * 4 + c4) ^ (lane & 7)) << 2)) =
-                make_float4(__uint_as_float(v[4 * c4]), __uint_as_float(v[4 * c4 + 1]), __uint_as_float(v[4 * c4 + 2]),
-                            __uint_as_float(v[4 * c4 + 3]));
-        }
-        __syncwarp();
-#pragma unroll
-        for (int rr = 0; rr < 8; rr++) {
-          const int rl = 4 * rr + lr;
-          float4 t = *reinterpret_cast<const float4 *>(W + rl * 32 + (((lane & 7) ^ (rl & 7)) << 2));
-          const int gr = rbase + rl, gc = cbase + 32 * sl + lc;
-          if (gr < m) {
-            if (F16) {
-              const float rsc = __ldg(row_scale + gr);
-              t.x *= rsc * csc.x;
-              t.y *= rsc * csc.y;
-              t.z *= rsc * csc.z;
-              t.w *= rsc * csc.w;
-            }
-            const float4 c4 = cs[rr];
-            const float4 o = overwrite ? t : make_float4(c4.x - t.x, c4.y - t.y, c4.z - t.z, c4.w - t.w);
-            float *dst = C + (size_t)gr * ldc + gc;
-            if (gc + 3 < n) *reinterpret_cast<float4 *>(dst) = o;
-            else if (gc < n) {
-              dst[0] = o.x;
-              if (gc + 1 < n) dst[1] = o.y;
-              if (gc + 2 < n) dst[2] = o.z;
-            }
-          }
-        }
-        __syncwarp();  // the next slice overwrites W
-      };
-      float4 c0[8], c1[8], c2[8], c3[8];
-      load_slice(c0, 0);
-      load_slice(c1, 1);
+      const float sign = overwrite ? 1.f : -1.f;
+      const float rsc = F16 && rbase + lane < m ? sign * __ldg(row_scale + rbase + lane) : sign;
       if (!tm_wait(smem_u32(&accf[buf]), (uint32_t)((i / 2) & 1))) { timed_out = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      store_slice(c0, 0);
-      load_slice(c2, 2);
-      store_slice(c1, 1);
-      load_slice(c3, 3);
-      store_slice(c2, 2);
-      store_slice(c3, 3);
-      // this thread's reads of the buffer are done: release it to the producer
+#pragma unroll
+      for (int sl = 0; sl < 4; sl++) {
+        const int col = cbase + 32 * sl;
+        uint32_t v[32];
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * TC_BN + hc * 128 + sl * 32);
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+            "tcgen05.wait::ld.sync.aligned;\n"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
+              "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
+              "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+            : "r"(taddr)
+            : "memory");
+        // the previous copy has read the buffer
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+          // FP16 operands: the accumulator carries the row and column factors
+          // (read only for columns inside C: the factors hold n + 8 entries)
+          const float4 cs = (F16 && col + 4 * g < n) ? __ldg(reinterpret_cast<const float4 *>(col_scale + col) + g)
+                                                     : make_float4(1.f, 1.f, 1.f, 1.f);
+          *reinterpret_cast<float4 *>(W + lane * 32 + ((g ^ (lane & 7)) << 2)) =
+              make_float4(rsc * cs.x * __uint_as_float(v[4 * g]), rsc * cs.y * __uint_as_float(v[4 * g + 1]),
+                          rsc * cs.z * __uint_as_float(v[4 * g + 2]), rsc * cs.w * __uint_as_float(v[4 * g + 3]));
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          if (col < n4 && rbase < m) {
+            if (overwrite)
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                               (uint64_t)&tmC), "r"(col), "r"(rbase), "r"(smem_u32(W))
+                           : "memory");
+            else
+              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                               (uint64_t)&tmC), "r"(col), "r"(rbase), "r"(smem_u32(W))
+                           : "memory");
+          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        if (n4 < n && n4 >= col && n4 < col + 32 && rbase + lane < m)
+          for (int c = n4; c < n; c++) {
+            const float t = W[lane * 32 + ((((c - col) >> 2) ^ (lane & 7)) << 2) + ((c - col) & 3)];
+            float *dst = C + (size_t)(rbase + lane) * ldc + c;
+            *dst = overwrite ? t : *dst + t;
+          }
+      }
+      // this thread's reads of the buffer are done: release it to the MMAs
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acce[buf])) : "memory");
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
   }
   if (timed_out && tid == 0) atomicExch(err, 2);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -822,11 +809,12 @@ static int launch_tc(float *C, int ldc, int m, int n, int k, float *A, int lda, 
     RB_TRY(check_launch("tc_f16_rows_kernel"));
     tc_f16_transpose_kernel<<<(n + 31) / 32, dim3(32, 8), 0, st>>>(B, ldb, k, n, bh.as<__half>(), kp, cs.as<float>());
     RB_TRY(check_launch("tc_f16_transpose_kernel"));
-    CUtensorMap ma, mb;
+    CUtensorMap ma, mb, mc;
+    RB_TRY(encode_map(&mc, C, m, std::max(n & ~3, 4), ldc, 32));
     RB_TRY(encode_map(&ma, ah.p, m, k, kp, TC_BM, true));
     RB_TRY(encode_map(&mb, bh.p, n, k, kp, TC_BN, true));
     RB_TRY(set_smem_once(tc_update_tma_kernel<true>, TM_SMEM, 0));
-    tc_update_tma_kernel<true><<<grid, TM_THREADS, TM_SMEM, st>>>(ma, mb, C, ldc, m, n, k, g_tc_err_flag.as<int>(),
+    tc_update_tma_kernel<true><<<grid, TM_THREADS, TM_SMEM, st>>>(ma, mb, mc, C, ldc, m, n, k, g_tc_err_flag.as<int>(),
                                                                   overwrite, rs.as<float>(), cs.as<float>());
     return check_launch("tc_update_tma_kernel<f16>");
   }
@@ -840,11 +828,12 @@ static int launch_tc(float *C, int ldc, int m, int n, int k, float *A, int lda, 
   tc_transpose_kernel<<<dim3((n + 31) / 32, (k + 31) / 32), dim3(32, 8), 0, st>>>(B, ldb, k, n, g_tc_bt.as<float>(), ldbt);
   RB_TRY(check_launch("tc_transpose_kernel"));
   if (use_tma) {
-    CUtensorMap ma, mb;
+    CUtensorMap ma, mb, mc;
+    RB_TRY(encode_map(&mc, C, m, std::max(n & ~3, 4), ldc, 32));
     RB_TRY(encode_map(&ma, A, m, k, lda, TC_BM));
     RB_TRY(encode_map(&mb, g_tc_bt.as<float>(), n, k, ldbt, TC_BN));
     RB_TRY(set_smem_once(tc_update_tma_kernel<false>, TM_SMEM, 1));
-    tc_update_tma_kernel<false><<<grid, TM_THREADS, TM_SMEM, st>>>(ma, mb, C, ldc, m, n, k, g_tc_err_flag.as<int>(),
+    tc_update_tma_kernel<false><<<grid, TM_THREADS, TM_SMEM, st>>>(ma, mb, mc, C, ldc, m, n, k, g_tc_err_flag.as<int>(),
                                                                    overwrite, nullptr, nullptr);
     return check_launch("tc_update_tma_kernel");
   }

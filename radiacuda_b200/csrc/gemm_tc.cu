@@ -651,73 +651,140 @@ __device__ __forceinline__ float f16_scale(unsigned maxbits)
   return ldexpf(1.f, 14 - e);
 }
 
+// Four elements of a row from p on, those at or past column limit `left` zero
+// (p is 16-byte aligned inside rows of a multiple of 4 elements)
+__device__ __forceinline__ float4 load4(const float *p, int left)
+{
+  if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 v = *reinterpret_cast<const float4 *>(p);
+  if (left < 4) {
+    v.w = 0.f;
+    if (left < 3) v.z = 0.f;
+    if (left < 2) v.y = 0.f;
+  }
+  return v;
+}
+__device__ __forceinline__ float absmax4(float m, const float4 &v)
+{
+  return fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+__device__ __forceinline__ uint2 half4(const float4 &v, float s)
+{
+  const __half2 a = __floats2half2_rn(s * v.x, s * v.y), b = __floats2half2_rn(s * v.z, s * v.w);
+  return make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
+}
+
 // Ah[r][c] = FP16(s_r A[r][c]) for c < k, 0 for k <= c < kp, with s_r the
 // power of two that brings row r's largest magnitude to at most 2^14; irs[r] =
-// 1 / s_r (exact).  A warp per row: the maximum, then the conversion (the row
-// is read again from L1/L2).
-__global__ void tc_f16_rows_kernel(const float *__restrict__ A, int lda, int m, int k, __half *__restrict__ Ah, int kp,
-                                   float *__restrict__ irs)
+// 1 / s_r (exact).  A warp per row, the row's first 1024 elements kept in
+// registers between its maximum and its conversion; HBM bound.
+__global__ void __launch_bounds__(256) tc_f16_rows_kernel(const float *__restrict__ A, int lda, int m, int k,
+                                                          __half *__restrict__ Ah, int kp, float *__restrict__ irs)
 {
   const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < m; r += nw) {
-    const float *row = A + (size_t)r * lda;
-    float mx = 0.f;
-    for (int c = lane; c < k; c += 32) mx = fmaxf(mx, fabsf(row[c]));
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const float sr = f16_scale(__float_as_uint(mx));
-    if (lane == 0) irs[r] = 1.f / sr;
-    __half2 *dst = reinterpret_cast<__half2 *>(Ah + (size_t)r * kp);
-    for (int c2 = lane; c2 < kp / 2; c2 += 32) {
-      const int c = 2 * c2;
-      dst[c2] = __floats2half2_rn(c < k ? sr * row[c] : 0.f, c + 1 < k ? sr * row[c + 1] : 0.f);
-    }
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (r >= m) return;
+  const float *row = A + (size_t)r * lda;
+  float4 v[8];
+  float mx = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int c = 128 * i + 4 * lane;
+    v[i] = load4(row + c, k - c);
   }
+#pragma unroll
+  for (int i = 0; i < 8; i++) mx = absmax4(mx, v[i]);
+  for (int c = 1024 + 4 * lane; c < k; c += 128) mx = absmax4(mx, load4(row + c, k - c));
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const float sr = f16_scale(__float_as_uint(mx));
+  if (lane == 0) irs[r] = 1.f / sr;
+  __half *dst = Ah + (size_t)r * kp;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int c = 128 * i + 4 * lane;
+    if (c < kp) *reinterpret_cast<uint2 *>(dst + c) = half4(v[i], sr);
+  }
+  for (int c = 1024 + 4 * lane; c < kp; c += 128) *reinterpret_cast<uint2 *>(dst + c) = half4(load4(row + c, k - c), sr);
 }
 
 // Bth[c][r] = FP16(t_c B[r][c]) (n x kp, K contiguous), with t_c the power of
 // two that brings column c's largest magnitude to at most 2^14; ics[c] = 1 / t_c.
-// A block of 32 x 8 threads per 32 columns: the column maxima, then the
-// columns turned around 32 rows at a time through shared memory.
-__global__ void tc_f16_transpose_kernel(const float *__restrict__ B, int ldb, int k, int n, __half *__restrict__ Bth,
-                                        int kp, float *__restrict__ ics)
+// A block per 32 columns: the column maxima, then 128 rows at a time turned
+// around through shared memory (the second reading comes from L2).  What
+// bounds it is the latency of its few blocks' loads, so a thread has four
+// 16-byte loads in flight, the next rows' while it turns the present ones.
+constexpr int TR_K = 128, TR_P = TR_K + 8;  // rows per turn; pitch: 16-byte aligned
+__global__ void __launch_bounds__(256) tc_f16_transpose_kernel(const float *__restrict__ B, int ldb, int k, int n,
+                                                               __half *__restrict__ Bth, int kp, float *__restrict__ ics)
 {
-  __shared__ float t[32][33];
-  __shared__ float red[8][32];
+  __shared__ __align__(16) __half t[2][32][TR_P];
+  __shared__ float red[32][33];
   __shared__ float sc[32];
-  const int c0 = blockIdx.x * 32, tx = threadIdx.x, ty = threadIdx.y;
-  const int c = c0 + tx;
-  float mx = 0.f;
-  if (c < n)
-    for (int r = ty; r < k; r += 8) mx = fmaxf(mx, fabsf(B[(size_t)r * ldb + c]));
-  red[ty][tx] = mx;
+  const int tid = threadIdx.x, g = tid & 7, rr = tid >> 3;  // column group of four, row of 32
+  const int c0 = blockIdx.x * 32, c = c0 + 4 * g;
+  const float *src = B + c;
+  auto rows = [&](float4 *v, int r0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int r = r0 + 32 * i + rr;
+      v[i] = load4(src + (size_t)r * ldb, r < k ? n - c : 0);
+    }
+  };
+  float4 v[4], w[4];
+  float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
+  rows(v, 0);
+  for (int r0 = 0; r0 < k; r0 += TR_K) {
+    rows(w, r0 + TR_K);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      mx.x = fmaxf(mx.x, fabsf(v[i].x)); mx.y = fmaxf(mx.y, fabsf(v[i].y));
+      mx.z = fmaxf(mx.z, fabsf(v[i].z)); mx.w = fmaxf(mx.w, fabsf(v[i].w));
+      if (k > TR_K) v[i] = w[i];
+    }
+  }
+  red[4 * g][rr] = mx.x; red[4 * g + 1][rr] = mx.y; red[4 * g + 2][rr] = mx.z; red[4 * g + 3][rr] = mx.w;
   __syncthreads();
-  if (ty == 0) {
-    for (int i = 1; i < 8; i++) mx = fmaxf(mx, red[i][tx]);
-    const float tc = f16_scale(__float_as_uint(mx));
-    sc[tx] = tc;
-    if (c < n) ics[c] = 1.f / tc;
+  {
+    float a = red[tid >> 3][tid & 7];
+#pragma unroll
+    for (int i = 1; i < 4; i++) a = fmaxf(a, red[tid >> 3][(tid & 7) + 8 * i]);
+    for (int o = 4; o > 0; o >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
+    if ((tid & 7) == 0) {
+      const float tc = f16_scale(__float_as_uint(a));
+      sc[tid >> 3] = tc;
+      if (c0 + (tid >> 3) < n) ics[c0 + (tid >> 3)] = 1.f / tc;
+    }
   }
   __syncthreads();
-  for (int r0 = 0; r0 < kp; r0 += 32) {
-    for (int i = ty; i < 32; i += 8) {
-      const int r = r0 + i;
-      t[i][tx] = (r < k && c < n) ? B[(size_t)r * ldb + c] : 0.f;
+  const float s0 = sc[4 * g], s1 = sc[4 * g + 1], s2 = sc[4 * g + 2], s3 = sc[4 * g + 3];
+  if (k > TR_K) rows(v, 0);
+  for (int r0 = 0, q = 0; r0 < kp; r0 += TR_K, q ^= 1) {
+    if (r0 + TR_K < kp) rows(w, r0 + TR_K);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int r = 32 * i + rr;
+      t[q][4 * g][r] = __float2half_rn(s0 * v[i].x);
+      t[q][4 * g + 1][r] = __float2half_rn(s1 * v[i].y);
+      t[q][4 * g + 2][r] = __float2half_rn(s2 * v[i].z);
+      t[q][4 * g + 3][r] = __float2half_rn(s3 * v[i].w);
     }
     __syncthreads();
-    for (int i = ty; i < 32; i += 8) {
-      const int cc = c0 + i, r = r0 + tx;
-      if (cc < n && r < kp) Bth[(size_t)cc * kp + r] = __float2half_rn(sc[i] * t[tx][i]);
+#pragma unroll
+    for (int e = tid; e < 32 * (TR_K / 8); e += 256) {  // 8 rows of a column
+      const int cc = e / (TR_K / 8), r = (e % (TR_K / 8)) * 8;
+      if (c0 + cc < n && r0 + r < kp)
+        *reinterpret_cast<uint4 *>(Bth + (size_t)(c0 + cc) * kp + r0 + r) = *reinterpret_cast<const uint4 *>(&t[q][cc][r]);
     }
-    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = w[i];
   }
 }
 
 // B^T scratch, [n x ldbt] floats, ldbt = k rounded up to 4; one per slot so
-// that updates on two streams (the LU's look-ahead) never share it
-static DBuf g_tc_bt_slots[2];
+// that updates on the LU's three streams never share it
+static DBuf g_tc_bt_slots[3];
 // FP16 path, per slot: A and B^T copies, the row and column factors
-static DBuf g_tc_ah_slots[2], g_tc_bh_slots[2], g_tc_rs_slots[2], g_tc_cs_slots[2];
+static DBuf g_tc_ah_slots[3], g_tc_bh_slots[3], g_tc_rs_slots[3], g_tc_cs_slots[3];
 
 // cudaFuncSetAttribute once per kernel and device (a driver call per launch
 // showed up in the LU's host enqueue time)
@@ -782,7 +849,7 @@ static int encode_map(CUtensorMap *map, const void *base, int rows, int cols, in
 static int launch_tc(float *C, int ldc, int m, int n, int k, float *A, int lda, const float *B, int ldb,
                      cudaStream_t st, int overwrite = 0, int max_ctas = 0, int use_tma = -1, int slot = 0)
 {
-  DBuf &g_tc_bt = g_tc_bt_slots[slot & 1];
+  DBuf &g_tc_bt = g_tc_bt_slots[slot];
   if (use_tma < 0) use_tma = g_tc_tma;
   long long tiles = (long long)((n + TC_BN - 1) / TC_BN) * ((m + TC_BM - 1) / TC_BM);
   if (tiles > (1ll << 30) || k < 1 || k > (1 << 20)) { set_error("tensor-core update shape out of range"); return RADB200_E_ARG; }
@@ -798,16 +865,15 @@ static int launch_tc(float *C, int ldc, int m, int n, int k, float *A, int lda, 
     // FP16 operands, each row of A and each column of B scaled by a power of
     // two into range (A and B are left as they are)
     const int kp = (k + 7) / 8 * 8;
-    DBuf &ah = g_tc_ah_slots[slot & 1], &bh = g_tc_bh_slots[slot & 1];
-    DBuf &rs = g_tc_rs_slots[slot & 1], &cs = g_tc_cs_slots[slot & 1];
+    DBuf &ah = g_tc_ah_slots[slot], &bh = g_tc_bh_slots[slot];
+    DBuf &rs = g_tc_rs_slots[slot], &cs = g_tc_cs_slots[slot];
     RB_TRY(ah.alloc((size_t)m * kp * sizeof(__half)));
     RB_TRY(bh.alloc((size_t)n * kp * sizeof(__half)));
     RB_TRY(rs.alloc((size_t)m * sizeof(float)));
     RB_TRY(cs.alloc((size_t)(n + 8) * sizeof(float)));  // the epilogue reads 4 at a time past a ragged end
-    const int nra = (int)std::min<int64_t>(((int64_t)m + 7) / 8, 148 * 16);
-    tc_f16_rows_kernel<<<std::max(nra, 1), 256, 0, st>>>(A, lda, m, k, ah.as<__half>(), kp, rs.as<float>());
+    tc_f16_rows_kernel<<<(m + 7) / 8, 256, 0, st>>>(A, lda, m, k, ah.as<__half>(), kp, rs.as<float>());
     RB_TRY(check_launch("tc_f16_rows_kernel"));
-    tc_f16_transpose_kernel<<<(n + 31) / 32, dim3(32, 8), 0, st>>>(B, ldb, k, n, bh.as<__half>(), kp, cs.as<float>());
+    tc_f16_transpose_kernel<<<(n + 31) / 32, 256, 0, st>>>(B, ldb, k, n, bh.as<__half>(), kp, cs.as<float>());
     RB_TRY(check_launch("tc_f16_transpose_kernel"));
     CUtensorMap ma, mb, mc;
     RB_TRY(encode_map(&mc, C, m, std::max(n & ~3, 4), ldc, 32));

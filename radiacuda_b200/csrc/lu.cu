@@ -8,7 +8,7 @@
 // positive semi-definite, so A is (close to) positive definite and needs no
 // row exchanges; a vanishing pivot is reported as RADB200_E_NUMERIC.
 //
-// Two levels: outer panels of 1024 columns (768 for the last 30,000 rows),
+// Two levels: outer panels of 1536 columns (768 for the last 20,000 rows),
 // 128-wide steps inside.  Step k
 // (width nb = 128) inside a panel:
 //   1. one CTA factors the diagonal block in shared memory (FP64) and writes
@@ -16,8 +16,10 @@
 //      (lu_diag.cuh);
 //   2. L21 = A21 U_kk^-1 and the panel's U12 = L_kk^-1 A12 as GEMMs (out of
 //      place, then copied back), so the triangular solves of the panel also
-//      run on the GEMM engine; a narrow update of the panel's other columns.
-// After the panel: its U block row by block forward substitution, then one
+//      run on the GEMM engine; a narrow update of the panel's other columns,
+//      its first 128 rows ahead of the others so that step k+1's diagonal block
+//      and U12 run beside them.
+// After the panel: its U block row by forward substitution in halves, then one
 // trailing update A22 -= L21 U12 with K = the panel width, split into the next panel's
 // columns (main stream) and the rest (a side stream, overlapping the next
 // panel's factorization).
@@ -176,13 +178,13 @@ static int copy2d(T *dst, int ldd, const T *src, int lds, int rows, int cols, cu
 
 template <typename T>
 static int gemm(T *C, int ldc, int m, int n, int k, T *A, int lda, const T *B, int ldb, int overwrite, cudaStream_t st,
-                int *tc_used)
+                int *tc_used, int slot = 0)
 {
   if (m <= 0 || n <= 0) return 0;
   LuHostSpan hs(0);
   if (sizeof(T) == 4) {
     int used = 0;
-    RB_TRY(tc_gemm_f32((float *)C, ldc, m, n, k, (float *)A, lda, (const float *)B, ldb, st, &used, overwrite));
+    RB_TRY(tc_gemm_f32((float *)C, ldc, m, n, k, (float *)A, lda, (const float *)B, ldb, st, &used, overwrite, slot));
     if (used) { *tc_used = 1; return 0; }
   }
   dim3 grid((n + 63) / 64, (m + 63) / 64);
@@ -196,16 +198,16 @@ static int gemm(T *C, int ldc, int m, int n, int k, T *A, int lda, const T *B, i
 // ldt) and copied back
 template <typename T>
 static int gemm_to(T *dst, int ldd, int m, int n, int k, T *A, int lda, const T *B, int ldb, bool c_is_a, T *tmp,
-                   int ldt, cudaStream_t st, int *tc_used)
+                   int ldt, cudaStream_t st, int *tc_used, int slot = 0)
 {
   if (m <= 0 || n <= 0) return 0;
   if (sizeof(T) == 4) {
     LuHostSpan hs(0);
     int used = 0;
-    RB_TRY(tc_gemm_f32_inplace((float *)dst, ldd, m, n, k, (float *)A, lda, (const float *)B, ldb, st, &used, c_is_a));
+    RB_TRY(tc_gemm_f32_inplace((float *)dst, ldd, m, n, k, (float *)A, lda, (const float *)B, ldb, st, &used, c_is_a, slot));
     if (used) { *tc_used = 1; return 0; }
   }
-  RB_TRY(gemm<T>(tmp, ldt, m, n, k, A, lda, B, ldb, 1, st, tc_used));
+  RB_TRY(gemm<T>(tmp, ldt, m, n, k, A, lda, B, ldb, 1, st, tc_used, slot));
   return copy2d<T>(dst, ldd, tmp, ldt, m, n, st);
 }
 
@@ -238,14 +240,15 @@ static double g_upd_bytes = 0.0, g_upd_flops = 0.0;
 // forward substitution over its 128-row sub-blocks, and the trailing matrix
 // receives ONE update with K = LU_OUTER: the C traffic of the dominant GEMM
 // drops by LU_OUTER / 128 against 128-wide steps.
-// Outer panel widths: 1024 columns while at least LU_LATE_AT_DEFAULT rows
-// remain, then 768.  The trailing GEMMs dominate the early panels (a wider K
-// raises their rate: 489 -> 533 TFLOP/s), the main stream's panel chain the
-// late ones.  Swept on the 60,000^2 factorization (solve, s): 768 throughout
-// 0.494; 1024 then 768 below 20,000 / 30,000 / 40,000 rows 0.482 / 0.481 /
-// 0.482; 1280 then 768 0.482; 1536 then 768 0.487; 1024 then 512 0.495;
-// 1024 then 640 0.493; 1280 then 1024 0.497.
-constexpr int LU_OUTER_DEFAULT = 1024, LU_OUTER_LATE_DEFAULT = 768, LU_LATE_AT_DEFAULT = 30000;
+// Outer panel widths: 1536 columns while at least LU_LATE_AT_DEFAULT rows
+// remain, then 768.  The trailing GEMMs dominate the early panels (up to K of
+// about 1024 they are bound by the traffic of C: 660, 705 and 730 TFLOP/s at
+// 1024, 1280 and 1536 columns), the main stream's panel chain the late ones.
+// Direct solve of the 60,000^2 system, ms: 1536 then 768 below 20,000 rows 394;
+// 1280 then 768 399; 1024 then 768 409 (below 30,000 rows 411); 1536 then 1024
+// 400; 1024 throughout 420.
+constexpr int LU_WIDEST = 2048;  // of all panels
+constexpr int LU_OUTER_DEFAULT = 1536, LU_OUTER_LATE_DEFAULT = 768, LU_LATE_AT_DEFAULT = 20000;
 // the outer panel width: LU_OUTER_DEFAULT, or RADB200_LU_OUTER (a multiple of
 // 128 from 256 to 2048) for tuning; RADB200_LU_OUTER_LATE (same range) is the
 // width once fewer than RADB200_LU_LATE_AT rows remain (tuning: the trailing
@@ -254,7 +257,7 @@ static int lu_width_env(const char *name, int dflt)
 {
   const char *e = getenv(name);
   int v = e ? atoi(e) : dflt;
-  return (v >= 256 && v <= 2048 && v % LU_NB == 0) ? v : dflt;
+  return (v >= 256 && v <= LU_WIDEST && v % LU_NB == 0) ? v : dflt;
 }
 static int lu_outer()
 {
@@ -281,18 +284,24 @@ static int lu_outer_at(int remaining)
 // The main stream waits for the side stream before the U block row of step
 // k+1, the only later work that reads or writes the columns the side stream
 // updates.  Events order the two streams; nothing waits on the device.
-constexpr int LU_SIDE_FREE_SMS = 12;  // swept 4-74 on the 60,000^2 factorization: 12 was fastest;
-                                       // with the 1024/768 panels: 6 +9 ms, 20 within 2 ms
+// Inside a panel the first 128 rows of an update go first (rows_first): the
+// next diagonal block and its U12 then run on a third stream of high priority
+// beside the update of the other rows (the diagonal block is one CTA for 97 us,
+// 45 ms of the main stream's chain over the 60,000^2 factorization; 14 left).
+constexpr int LU_SIDE_FREE_SMS = 12;  // 60,000^2 direct solve: 8 411, 12 409, 20 407 ms; 28 and 40 slower
 
 struct LuStreams {
-  cudaStream_t main = nullptr, side = nullptr;
-  cudaEvent_t in = nullptr, upd = nullptr, side_done = nullptr, out = nullptr;
+  cudaStream_t main = nullptr, side = nullptr, diag = nullptr;
+  cudaEvent_t in = nullptr, upd = nullptr, side_done = nullptr, out = nullptr, row = nullptr, diag_done = nullptr;
   int init()
   {
     if (main) return 0;
     RB_CUDA(cudaStreamCreateWithFlags(&main, cudaStreamNonBlocking));
     RB_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-    for (cudaEvent_t *e : {&in, &upd, &side_done, &out}) RB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    int lo = 0, hi = 0;  // the diagonal block's launches take the next free SM
+    RB_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    RB_CUDA(cudaStreamCreateWithPriority(&diag, cudaStreamNonBlocking, hi));
+    for (cudaEvent_t *e : {&in, &upd, &side_done, &out, &row, &diag_done}) RB_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     return 0;
   }
 };
@@ -302,6 +311,7 @@ template <typename T>
 static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, double tiny, cudaStream_t st, int *tc_used)
 {
   const int n3 = I.n3, ld = I.ld;
+  T *tmp_row = tmp + std::max((size_t)n3 * LU_NB, (size_t)LU_NB * ld);
   RB_CUDA(cudaFuncSetAttribute(diag_factor_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
   // RADB200_LU_TIMING=1 prints the time of each phase (synchronizes per phase);
   // RADB200_LU_TIMING=2 prints the host's time to enqueue the factorization
@@ -363,7 +373,7 @@ static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, doubl
     mk_cat.push_back(cat);
     return 0;
   };
-  bool side_pending = false;
+  bool side_pending = false, ahead = false;
   auto at = [&](int r, int c) { return A + (size_t)r * ld + c; };
   // C[m x n] -= A B with the update's timing events on stream q
   auto update = [&](T *C, int m, int n, int k, T *Ap, const T *Bp, cudaStream_t q, int slot, int cap) -> int {
@@ -390,34 +400,74 @@ static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, doubl
     }
     return 0;
   };
+  auto diag = [&](int j0, int jb, cudaStream_t q) -> int {
+    LuHostSpan hs(2);
+    diag_factor_kernel<T><<<1, DG_T, DG_SMEM, q>>>(A, ld, j0, jb, Linv, Uinv, d_err, tiny);
+    return check_launch("diag_factor_kernel");
+  };
+  // U12 of step j0 inside its panel: L_jj^-1 A12 (out of place: tmp_row)
+  auto u12 = [&](int j0, int pend, cudaStream_t q, int slot) -> int {
+    const int jb = std::min(LU_NB, pend - j0), rest = j0 + jb, w = pend - rest;
+    return w <= 0 ? 0
+                  : gemm_to<T>(at(j0, rest), ld, jb, w, jb, Linv + (size_t)j0 * LU_NB, LU_NB, at(j0, rest), ld, false,
+                               tmp_row, LU_WIDEST, q, tc_used, slot);
+  };
+  // An update of the rows from r0 on of a panel that ends at column pend:
+  // run(r, rows) first for the next step's 128 rows, whose diagonal block and
+  // U12 then go on beside run() of the others
+  auto rows_first = [&](int r0, int pend, auto run) -> int {
+    const int rows = n3 - r0, first = std::min(LU_NB, rows);
+    if (!lookahead) return run(r0, rows);
+    RB_TRY(run(r0, first));
+    RB_CUDA(cudaEventRecord(g_lu_streams.row, sm));
+    RB_CUDA(cudaStreamWaitEvent(g_lu_streams.diag, g_lu_streams.row, 0));
+    RB_TRY(diag(r0, std::min(LU_NB, pend - r0), g_lu_streams.diag));
+    RB_TRY(u12(r0, pend, g_lu_streams.diag, 2));
+    RB_CUDA(cudaEventRecord(g_lu_streams.diag_done, g_lu_streams.diag));
+    ahead = true;
+    return rows > first ? run(r0 + first, rows - first) : 0;
+  };
+  // U rows r0 .. r1 of the n columns from c0 on by halves: the upper half, its
+  // product off the lower half, the lower half.  Every level reads and
+  // converts half of the rows once (row by row of blocks, the rows above were
+  // converted again for each: 3,584 instead of 1,536 rows per 1024).
+  auto urows = [&](auto self, int r0, int r1, int c0, int n) -> int {
+    const int blocks = (r1 - r0 + LU_NB - 1) / LU_NB, mid = std::min(r1, r0 + (blocks + 1) / 2 * LU_NB);
+    if (blocks == 1)
+      return gemm_to<T>(at(r0, c0), ld, r1 - r0, n, r1 - r0, Linv + (size_t)r0 * LU_NB, LU_NB, at(r0, c0), ld, false, tmp, ld,
+                        sm, tc_used);
+    RB_TRY(self(self, r0, mid, c0, n));
+    RB_TRY(gemm<T>(at(mid, c0), ld, r1 - mid, n, mid - r0, at(mid, r0), ld, at(r0, c0), ld, 0, sm, tc_used));
+    return self(self, mid, r1, c0, n);
+  };
   for (int K0 = 0, NBe = 0; K0 < n3; K0 += NBe) {
     NBe = std::min(lu_outer_at(n3 - K0), n3 - K0);
     const int pend = K0 + NBe;  // end of the panel's columns
     // ---- factor the panel columns [K0, pend) over rows [K0, n3) (main stream;
     // the previous step updated these columns there first)
     for (int j0 = K0; j0 < pend; j0 += LU_NB) {
-      const int jb = std::min(LU_NB, pend - j0);
-      {
-        LuHostSpan hs(2);
-        diag_factor_kernel<T><<<1, DG_T, DG_SMEM, sm>>>(A, ld, j0, jb, Linv, Uinv, d_err, tiny);
-        RB_TRY(check_launch("diag_factor_kernel"));
+      const int jb = std::min(LU_NB, pend - j0), rest = j0 + jb, m = n3 - rest, w = pend - rest;
+      const bool done = ahead;  // the diagonal block and the panel's U12 of this step
+      if (ahead) {
+        RB_CUDA(cudaStreamWaitEvent(sm, g_lu_streams.diag_done, 0));
+        ahead = false;
+      } else {
+        RB_TRY(diag(j0, jb, sm));
       }
       RB_TRY(mark(0));
       RB_TRY(phase(0));
-      const int rest = j0 + jb, m = n3 - rest;
       if (m <= 0) break;
       // L21 = A21 U_jj^-1   (tmp: m x LU_NB)
       RB_TRY(gemm_to<T>(at(rest, j0), ld, m, jb, jb, at(rest, j0), ld, Uinv + (size_t)j0 * LU_NB, LU_NB, true, tmp, LU_NB,
                         sm, tc_used));
       RB_TRY(mark(1));
-      const int w = pend - rest;  // panel columns right of this step
       if (w > 0) {
-        // U12 inside the panel = L_jj^-1 A12   (tmp: jb x w)
-        RB_TRY(gemm_to<T>(at(j0, rest), ld, jb, w, jb, Linv + (size_t)j0 * LU_NB, LU_NB, at(j0, rest), ld, false, tmp, ld,
-                          sm, tc_used));
+        if (!done) RB_TRY(u12(j0, pend, sm, 0));
         RB_TRY(mark(2));
         // narrow update of the panel: A[rest:, rest:pend] -= L21 U12
-        RB_TRY(gemm<T>(at(rest, rest), ld, m, w, jb, at(rest, j0), ld, at(j0, rest), ld, 0, sm, tc_used));
+        RB_TRY(rows_first(rest, pend, [&](int r, int mr) -> int {
+          return gemm<T>(at(r, rest), ld, mr, w, jb, at(r, j0), ld, at(j0, rest), ld, 0, sm, tc_used);
+        }));
         RB_TRY(mark(3));
       }
       RB_TRY(phase(1));
@@ -432,19 +482,16 @@ static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, doubl
     }
     RB_TRY(mark(4));
     // ---- U block row of the trailing columns: forward substitution with the
-    // panel's unit-lower diagonal block, 128 rows at a time
-    for (int j0 = K0; j0 < pend; j0 += LU_NB) {
-      const int jb = std::min(LU_NB, pend - j0);
-      if (j0 > K0) RB_TRY(gemm<T>(at(j0, T0), ld, jb, mT, j0 - K0, at(j0, K0), ld, at(K0, T0), ld, 0, sm, tc_used));
-      RB_TRY(gemm_to<T>(at(j0, T0), ld, jb, mT, jb, Linv + (size_t)j0 * LU_NB, LU_NB, at(j0, T0), ld, false, tmp, ld, sm,
-                        tc_used));
-    }
+    // panel's unit-lower diagonal block
+    RB_TRY(urows(urows, K0, pend, T0, mT));
     RB_TRY(mark(5));
     RB_TRY(phase(2));
     // ---- trailing update A22 -= L21 U12 with K = NBe: the next panel's
     // columns on the main stream, the rest on the side stream
     const int nxt = lookahead ? std::min(lu_outer_at(mT), mT) : mT;  // the next panel's width
-    RB_TRY(update(at(T0, T0), mT, nxt, NBe, at(T0, K0), at(K0, T0), sm, 0, 0));
+    RB_TRY(rows_first(T0, T0 + nxt, [&](int r, int mr) -> int {
+      return update(at(r, T0), mr, nxt, NBe, at(r, K0), at(K0, T0), sm, 0, 0);
+    }));
     RB_TRY(mark(6));
     if (mT > nxt) {
       RB_CUDA(cudaEventRecord(g_lu_streams.upd, sm));
@@ -455,6 +502,7 @@ static int lu_factor(Intrc &I, T *A, T *Linv, T *Uinv, T *tmp, int *d_err, doubl
     RB_TRY(phase(3));
   }
   if (lookahead) {
+    if (ahead) RB_CUDA(cudaStreamWaitEvent(sm, g_lu_streams.diag_done, 0));
     RB_CUDA(cudaEventRecord(g_lu_streams.side_done, ss));
     RB_CUDA(cudaStreamWaitEvent(sm, g_lu_streams.side_done, 0));
     RB_CUDA(cudaEventRecord(g_lu_streams.out, sm));
@@ -695,7 +743,7 @@ int lu_build_x(Intrc &I, int mode, const double *X, int of_d, double *factor_sec
   int tc_used = 0;
   size_t es = (mode == RADB200_LU_F64) ? sizeof(double) : sizeof(float);
   RB_TRY(I.LUinv.alloc(2 * (size_t)n3 * LU_NB * es));
-  RB_TRY(I.lu_scratch.alloc((size_t)std::max((size_t)n3 * LU_NB, (size_t)LU_NB * ld) * es));
+  RB_TRY(I.lu_scratch.alloc((std::max((size_t)n3 * LU_NB, (size_t)LU_NB * ld) + LU_NB * LU_WIDEST) * es));
   if (mode == RADB200_LU_F64) {
     I.LU32.release();
     RB_TRY(I.LU64.alloc((size_t)n3 * ld * sizeof(double)));

@@ -650,13 +650,11 @@ TC_TRAFFIC_OVER_ALGORITHMIC = {"tf32": 0.92, "f16": 0.92}
 FIELD_OPS_PER_TET = 4 * 16 + 6 * 5 + 6 * 40 + 4 * 51 + 3
 
 # Instructions the FP32 field kernel issues per (point, tetrahedron) pair,
-# from ncu's smsp__inst_executed.sum x 32 / pairs on the 20,000-point,
-# 20,000-tetrahedron case (tests/profile_cases.py field --precision single), and
-# their split over the pipes.  The kernel is issue-bound: its roofline is the
-# SMs' issue rate, 4 warp-instructions (128 thread-instructions) per clock
-# per SM, divided by these instructions per pair.
-FIELD_INST_PER_PAIR = 793
-FIELD_INST_MIX = {"fma": 329, "alu": 157, "fp64": 81, "lsu": 60, "xu": 50}
+# from ncu's smsp__inst_executed.sum x 32 / pairs on 8,000 tetrahedra and 1e6
+# points (9.65e10 warp-instructions).  The kernel is issue-bound: its roofline
+# is the SMs' issue rate, 4 warp-instructions (128 thread-instructions) per
+# clock per SM, divided by these instructions per pair.
+FIELD_INST_PER_PAIR = 386
 B200_SMS = 148
 
 
@@ -664,12 +662,11 @@ def field_roofline(pairs_per_s, op_tflops, fp32_peak, clk):
     mhz = (clk or {}).get("sm_mhz") or 1965.0
     peak = B200_SMS * mhz * 1e6 * 128 / 1e12  # thread-instructions issued per second, 1e12
     ach = pairs_per_s * FIELD_INST_PER_PAIR / 1e12
-    return {"kernel": "field_tet_kernel<float> (FP32 terms)", "bound": "issue",
+    return {"kernel": "field_tet32_kernel (FP32 terms)", "bound": "issue",
             "achieved": round(ach, 3), "peak": round(peak, 3), "unit": "T instructions/s", "frac": round(ach / peak, 4),
             "peak_source": f"{B200_SMS} SMs x 128 thread-instructions per clock at the median SM clock sampled "
                            f"during the timed steps ({mhz:.0f} MHz)",
-            "algorithmic": f"{FIELD_INST_PER_PAIR} instructions per (point, tetrahedron), ncu-counted "
-                           f"(per pipe: {FIELD_INST_MIX})",
+            "algorithmic": f"{FIELD_INST_PER_PAIR} instructions per (point, tetrahedron), ncu-counted",
             "pairs_per_s": round(pairs_per_s, 1),
             "op_model": {"achieved_tflops": round(op_tflops, 3), "fp32_fma_peak_tflops": round(fp32_peak, 3),
                          "frac": round(op_tflops / fp32_peak, 4),

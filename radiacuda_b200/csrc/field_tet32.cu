@@ -4,13 +4,15 @@
 // FP64 and rounded to FP32; distances, edge integrals and solid angles in
 // FP32; weights and sums in FP64.  Bound by instruction issue: the library's
 // log1pf, atan2f, division and square root made 793 thread-instructions a
-// pair.  Most pairs are distant, and there each element is short:
+// pair, this form 386 (8,000 tetrahedra, 1e6 points: 223 ms before, 126 ms).
+// Most pairs are distant, and there each element is short:
 //   L / 2 = artanh(x),   x = l / (Ra + Rb) <= 1/6:    a quotient, 3 terms;
 //   half solid angle = arctan(num / den) <= 0.025:     a quotient, 2 terms,
 // when the point is at least 4 times the longest edge from vertex 0 (every
-// distance is then at least 3 of them).  This L has less error than the
-// log1pf form (2-norm of B against FP64 on 3,000 tetrahedra 1.9e-7 against
-// 2.6e-7): it takes the exact length and two distances, no dot product.
+// distance is then at least 3 of them).  The quotients' corrections, and what
+// rounding took from Ra + Rb, go into the last addition of each: 2-norm of B
+// against FP64 on 20,000 / 3,000 tetrahedra 1.9e-7 / 2.2e-7 (the library's form
+// 2.6e-7 / 2.3e-7; without these corrections 2.4e-7 / 2.5e-7 and 118 ms).
 // Nearer pairs take the log1pf and atan2f forms.  A warp pays for the longer
 // path when any of its lanes needs it, so larger point sets are first put in
 // Morton order; each point's sum runs over the tetrahedra in their own order
@@ -37,11 +39,14 @@ __device__ __forceinline__ float rcp32(float d)
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
   return y;
 }
-// n / d by the approximate reciprocal and one Newton correction of the quotient
-__device__ __forceinline__ float quot32(float n, float d)
+// n / d = q + c: the product with the approximate reciprocal and its Newton
+// correction, which the caller adds last, in the same rounding as its series;
+// t is what d is short of its unrounded value by
+__device__ __forceinline__ float quot32(float n, float d, float t, float &c)
 {
   const float y = rcp32(d), q = n * y;
-  return fmaf(fmaf(-d, q, n), y, q);
+  c = fmaf(-q, t, fmaf(-d, q, n)) * y;
+  return q;
 }
 // sqrt by the approximate reciprocal root and one Newton correction
 __device__ __forceinline__ float root32(float s)
@@ -106,19 +111,22 @@ __device__ __forceinline__ void tet32_pair(const double *__restrict__ sd, const 
     for (int k = 0; k < 4; k++) R[k] = root32(R[k]);
 #pragma unroll
     for (int e = 0; e < 6; e++) {
-      const float x = quot32(sf[e], R[tet_edge_a(e)] + R[tet_edge_b(e)]), z = x * x;
+      const float ra = R[tet_edge_a(e)], rb = R[tet_edge_b(e)], s = ra + rb;
+      float c;  // ra and rb differ by less than a factor 2: (ra - s) + rb is exact
+      const float x = quot32(sf[e], s, (ra - s) + rb, c), z = x * x;
       // artanh(x) = x (1 + z p(z)), least maximum error 2.3e-9 for z <= 1/36
       const float p = fmaf(fmaf(0.1477081972f, z, 0.1999480270f), z, 0.3333334154f);
-      edge_add(e, fmaf(x * z, p, x));
+      edge_add(e, x + fmaf(x * z, p, c));
     }
 #pragma unroll
     for (int f = 0; f < 4; f++) {
       const int a = tet_face_a(f), b = tet_face_b(f), c = tet_face_c(f);
       const float num = fmaf(rx[a], sf[6 + 3 * f], fmaf(ry[a], sf[7 + 3 * f], rz[a] * sf[8 + 3 * f]));
       const float den = fmaf(fmaf(R[a], R[b], d[tet_pair(a, b)]), R[c], fmaf(d[tet_pair(a, c)], R[b], d[tet_pair(b, c)] * R[a]));
-      const float w = quot32(-num, den), u = w * w;
+      float cw;
+      const float w = quot32(-num, den, 0.f, cw), u = w * w;
       // arctan(w) = w (1 + u p(u)), least maximum error 3e-11 for u <= 0.0012
-      face_add(f, fmaf(w * u, fmaf(0.1998287159f, u, -0.3333333076f), w));
+      face_add(f, w + fmaf(w * u, fmaf(0.1998287159f, u, -0.3333333076f), cw));
     }
   } else {
 #pragma unroll

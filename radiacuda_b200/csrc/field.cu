@@ -673,6 +673,8 @@ __global__ void __launch_bounds__(TRJ_THREADS) trajectory_kernel(GeomView g, Trj
   double x = a.y0, hmin = 1e-10 * a.step;
   int rc = 0;
   long long ne = 0;
+  // every CTA of the cluster has started before any writes to another's sums
+  cooperative_groups::this_cluster().sync();
   for (int i = 0; i < a.np; i++) {
     if (!a.adaptive) trj_eqs(g, a, x, Y, dY, c, ne);
     if (writer) {

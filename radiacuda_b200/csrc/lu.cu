@@ -640,6 +640,8 @@ template <typename T> static int sweeps(Intrc &I, const T *A, int transposed, do
   RB_CUDA(cudaGetDevice(&dev));
   RB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int grid = std::min(nblk, nsm);
+  const char *e = getenv("RADB200_SWEEP_SPIN");
+  const int spin = e ? std::min(std::max(atoi(e), 0), SWEEP_SPIN) : SWEEP_SPIN;
   auto run = [&](auto kernel, int blocks, auto... args) -> int {
     const size_t smem = sweep_smem<T>(blocks);
     RB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -647,13 +649,13 @@ template <typename T> static int sweeps(Intrc &I, const T *A, int transposed, do
     return check_launch("sweep_kernel");
   };
   if (transposed) {
-    RB_TRY(run(sweep_t_kernel<T, false>, 1, A, ld, U, n3, x, y, count, err));
-    RB_TRY(run(sweep_t_kernel<T, true>, 1, A, ld, L, n3, y, z, count + 1, err));
+    RB_TRY(run(sweep_t_kernel<T, false>, 1, A, ld, U, n3, x, y, count, err, spin));
+    RB_TRY(run(sweep_t_kernel<T, true>, 1, A, ld, L, n3, y, z, count + 1, err, spin));
   } else {
     // (FP64 factors: no coupling blocks)
     const T *Mf = sizeof(T) == 4 ? I.sweep_m.as<T>() : nullptr, *Mb = Mf ? Mf + (size_t)nblk * LU_NB * LU_NB : nullptr;
-    RB_TRY(run(sweep_kernel<T, false>, Mf ? 2 : 1, A, ld, L, n3, x, y, count, err, Mf));
-    RB_TRY(run(sweep_kernel<T, true>, Mf ? 2 : 1, A, ld, U, n3, y, z, count + 1, err, Mb));
+    RB_TRY(run(sweep_kernel<T, false>, Mf ? 2 : 1, A, ld, L, n3, x, y, count, err, spin, Mf));
+    RB_TRY(run(sweep_kernel<T, true>, Mf ? 2 : 1, A, ld, U, n3, y, z, count + 1, err, spin, Mb));
   }
   RB_CUDA(cudaMemcpyAsync(x, z, (size_t)n3 * sizeof(double), cudaMemcpyDeviceToDevice, st));
   return 0;

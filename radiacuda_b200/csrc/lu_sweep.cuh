@@ -23,14 +23,14 @@
 //     the inverse beforehand, M_k waits in registers in FP64, and after the
 //     neighbour's values arrive only x_k = y_k - M_k x_j remains.
 // A CTA waits only on blocks taken before its own by CTAs that are running, so
-// every wait ends; each is also bounded by SWEEP_SPIN polls, after which the
-// launch records an error in *err and every CTA returns.
+// every wait ends; each is also bounded by `spin` polls, after which the launch
+// records an error in *err and every CTA waits for its own copies and returns.
 #pragma once
 
 namespace rb {
 
 constexpr int SW_NB = 128, SW_T = 512, SW_W = SW_T / 32, SW_R = SW_NB / SW_W, SW_Q = SW_T / SW_NB, SW_C = SW_NB / SW_Q;
-constexpr int SWEEP_SPIN = 1 << 20;
+constexpr int SWEEP_SPIN = 1 << 20;  // RADB200_SWEEP_SPIN overrides it (0: a wait runs out at once)
 constexpr int SWEEP_NAP = 400, SWEEP_NAP_MAX = 8000;  // ns per block of distance
 constexpr unsigned long long SWEEP_EMPTY = ~0ull;
 
@@ -47,10 +47,10 @@ __device__ __forceinline__ unsigned long long sweep_peek(const double *p)
   return b;
 }
 // *p (last seen as b) once it is there; bad when the wait ran out
-__device__ __forceinline__ double sweep_get(const double *p, unsigned long long b, int dist, int *err, int *bad)
+__device__ __forceinline__ double sweep_get(const double *p, unsigned long long b, int dist, int spin, int *err, int *bad)
 {
   for (int it = 0; b == SWEEP_EMPTY; it++) {
-    if (it > SWEEP_SPIN || ((it & 255) == 255 && *(volatile int *)err != 0)) {
+    if (it > spin || ((it & 255) == 255 && *(volatile int *)err != 0)) {
       atomicExch(err, 1);
       *bad = 1;
       return 0.0;
@@ -99,7 +99,7 @@ __device__ __forceinline__ void sweep_staged() { asm volatile("cp.async.wait_all
 template <typename T, bool UPPER>
 __global__ void __launch_bounds__(SW_T, 1) sweep_kernel(const T *__restrict__ A, int ld, const T *__restrict__ Inv, int n3,
                                                         const double *__restrict__ b, double *x, int *counter, int *err,
-                                                        const T *__restrict__ M)
+                                                        int spin, const T *__restrict__ M)
 {
   constexpr int NR = sweep_rows<T>(), NS = SW_R / NR, P = sweep_pitch<T>();
   extern __shared__ __align__(16) unsigned char sweep_dyn[];
@@ -138,8 +138,9 @@ __global__ void __launch_bounds__(SW_T, 1) sweep_kernel(const T *__restrict__ A,
     };
     // x_j of tile s into xs[s & 1]; false when a wait ran out
     auto arrive = [&](int s) -> bool {
-      if (tid < SW_NB) xs[s & 1][tid] = col0(s) + tid < n3 ? sweep_get(x + col0(s) + tid, seen, t - s, err, &s_bad) : 0.0;
+      if (tid < SW_NB) xs[s & 1][tid] = col0(s) + tid < n3 ? sweep_get(x + col0(s) + tid, seen, t - s, spin, err, &s_bad) : 0.0;
       __syncthreads();
+      if (s_bad) sweep_staged();  // the launch ends: no copy into shared memory outlives its CTA
       return s_bad == 0;
     };
     double acc[SW_R];
@@ -217,7 +218,8 @@ __global__ void __launch_bounds__(SW_T, 1) sweep_kernel(const T *__restrict__ A,
 // LOWER: L^T (backward), else U^T (forward)
 template <typename T, bool LOWER>
 __global__ void __launch_bounds__(SW_T, 1) sweep_t_kernel(const T *__restrict__ A, int ld, const T *__restrict__ Inv, int n3,
-                                                          const double *__restrict__ b, double *x, int *counter, int *err)
+                                                          const double *__restrict__ b, double *x, int *counter, int *err,
+                                                          int spin)
 {
   constexpr int NR = sweep_rows<T>(), NS = SW_R / NR, P = sweep_pitch<T>();
   extern __shared__ __align__(16) unsigned char sweep_dyn[];
@@ -253,8 +255,9 @@ __global__ void __launch_bounds__(SW_T, 1) sweep_t_kernel(const T *__restrict__ 
       if (tid < SW_NB && s < t && row0(s) + tid < n3) seen = sweep_peek(x + row0(s) + tid);
     };
     auto arrive = [&](int s) -> bool {
-      if (tid < SW_NB) xs[s & 1][tid] = row0(s) + tid < n3 ? sweep_get(x + row0(s) + tid, seen, t - s, err, &s_bad) : 0.0;
+      if (tid < SW_NB) xs[s & 1][tid] = row0(s) + tid < n3 ? sweep_get(x + row0(s) + tid, seen, t - s, spin, err, &s_bad) : 0.0;
       __syncthreads();
+      if (s_bad) sweep_staged();  // the launch ends: no copy into shared memory outlives its CTA
       return s_bad == 0;
     };
     double acc[4] = {0.0, 0.0, 0.0, 0.0};

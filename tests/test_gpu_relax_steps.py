@@ -116,3 +116,24 @@ def test_triangular_sweeps(cuda, rad, n, mode):
     finally:
         again.free()
     assert np.array_equal(lam2, lam)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("n", [86, 171, 300])
+def test_a_sweep_whose_wait_runs_out_ends(cuda, rad, n, mode, monkeypatch):
+    """RADB200_SWEEP_SPIN=0: blocks after the first give up at once, with the
+    copies of their inverses under way.  The solve fails, the device goes on."""
+    h = _blocks(rad, n)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    nat = _native.NativeInteraction(pack, 1)
+    try:
+        monkeypatch.setenv("RADB200_SWEEP_SPIN", "0")
+        with pytest.raises(Exception):
+            nat.direct(mode, 1e-13, 60)
+    finally:
+        monkeypatch.undo()
+        nat.free()
+    P = np.array([[0.317, 5.071, 0.233]])
+    g = model.pack_sources(rad._objs, h, tuple(rad._rand))
+    assert rel_err(_native.field(g, P, 0), O.field(g, P, 0)) < 1e-9

@@ -484,10 +484,12 @@ int adjoint_solve(Intrc &I, const double *dLdM, double rtol, int max_iter, doubl
   AdjOp op(I, coef.as<double>(), t, part, use_lu);
   double relres = 0.0;
   int its = 0;
-  RB_TRY(gmres(op, n3, ld, g, x, rtol, max_iter, 60, &relres, &its, 0));
+  const int rc = gmres(op, n3, ld, g, x, rtol, max_iter, 60, &relres, &its, 0);
+  // a sweep that gave up leaves NaN, so its flag is read (and cleared) whatever gmres said
   int tri_err = 0;
   if (use_lu) RB_TRY(tri_sweep_error(&tri_err));
   if (tri_err) { set_error("adjoint solve: a triangular sweep timed out waiting for a block"); return RADB200_E_TIMEOUT; }
+  RB_TRY(rc);
   if (!use_lu) {  // lambda = P^-T z
     adj_block_kernel<<<nb, 128>>>(coef.as<double>(), 1, n, x, t);
     RB_TRY(check_launch("adj_block_kernel"));

@@ -835,15 +835,17 @@ int direct_solve(Intrc &I, int mode, double rtol, int max_iter, double *status)
   LinOp op(I, tmp);
   double relres = 0.0;
   int its = 0;
-  RB_TRY(gmres(op, n3, ld, b, I.M.as<double>(), rtol, max_iter, 30, &relres, &its, 0));
+  const int rc = gmres(op, n3, ld, b, I.M.as<double>(), rtol, max_iter, 30, &relres, &its, 0);
+  // a sweep that gave up leaves NaN, so its flag is read (and cleared) whatever gmres said
+  int tri_err = 0;
+  RB_TRY(tri_sweep_error(&tri_err));
+  if (tri_err) { set_error("direct solve: a triangular sweep timed out waiting for a block"); return RADB200_E_TIMEOUT; }
+  RB_TRY(rc);
   RB_CUDA(cudaDeviceSynchronize());
   if (timing_on())
     fprintf(stderr, "RADB200_TIMING solve: refinement, %d its: products %.3f ms, sweeps %.3f ms\n", its, 1e3 * op.t_mv,
             1e3 * op.t_pc);
   pc.mark("solve: refinement");
-  int tri_err = 0;
-  RB_TRY(tri_sweep_error(&tri_err));
-  if (tri_err) { set_error("direct solve: a triangular sweep timed out waiting for a block"); return RADB200_E_TIMEOUT; }
   status[0] = relres;
   status[1] = its;
   status[2] = tf;

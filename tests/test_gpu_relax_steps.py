@@ -137,3 +137,31 @@ def test_a_sweep_whose_wait_runs_out_ends(cuda, rad, n, mode, monkeypatch):
     P = np.array([[0.317, 5.071, 0.233]])
     g = model.pack_sources(rad._objs, h, tuple(rad._rand))
     assert rel_err(_native.field(g, P, 0), O.field(g, P, 0)) < 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1])
+def test_a_sweep_time_out_is_reported_and_forgotten(cuda, rad, mode, monkeypatch):
+    """The direct and the adjoint solve name the time-out, and the next solves,
+    on this interaction and on another, give what they gave before it."""
+    h = _blocks(rad, 171)
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    g = np.random.default_rng(3).normal(size=3 * 171)
+    nat, other = _native.NativeInteraction(pack, 1), _native.NativeInteraction(pack, 1)
+    try:
+        M = nat.direct(mode, 1e-13, 60)[0].copy()
+        lam = nat.adjoint_solve(g, 1e-13, 60)[0].copy()
+        for k in range(2):
+            monkeypatch.setenv("RADB200_SWEEP_SPIN", "0")
+            with pytest.raises(Exception, match="timed out"):
+                nat.adjoint_solve(g, 1e-13, 60)
+            if k:
+                with pytest.raises(Exception, match="timed out"):
+                    nat.direct(mode, 1e-13, 60)
+            monkeypatch.delenv("RADB200_SWEEP_SPIN")
+            assert np.array_equal(other.direct(mode, 1e-13, 60)[0], M)
+            assert np.array_equal(nat.direct(mode, 1e-13, 60)[0], M)
+            assert np.array_equal(nat.adjoint_solve(g, 1e-13, 60)[0], lam)
+    finally:
+        nat.free()
+        other.free()

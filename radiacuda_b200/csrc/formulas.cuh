@@ -393,15 +393,16 @@ __device__ __forceinline__ int polygon_S_terms(const VP *vtx, int nv, T coordz, 
 // against 2,500 issue slots.
 constexpr int EDGE_REC = 4;
 // of polygon vertex j: direction (2) and length of the edge to the next
-// vertex, twice the area of the fan triangle (0, j, j + 1)
+// vertex, twice the area of the fan triangle (0, j, j + 1).  An edge between
+// two equal vertices (a collapsed face) has direction zero and adds nothing.
 RB_HD void edge_record(const double *vtx, int nv, int j, double *e)
 {
   const int k = j + 1 < nv ? j + 1 : 0;
   const double ex = vtx[2 * k] - vtx[2 * j], ey = vtx[2 * k + 1] - vtx[2 * j + 1];
   const double l = sqrt(ex * ex + ey * ey);
   const double fx = vtx[2 * j] - vtx[0], fy = vtx[2 * j + 1] - vtx[1];
-  e[0] = ex / l;
-  e[1] = ey / l;
+  e[0] = l > 0.0 ? ex / l : 0.0;
+  e[1] = l > 0.0 ? ey / l : 0.0;
   e[2] = l;
   e[3] = fx * ey - fy * ex;
 }

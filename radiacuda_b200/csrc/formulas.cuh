@@ -245,11 +245,14 @@ RB_HD double cuboid_edge_L(double b0, double b1, double rho2, bool mixed, bool n
 // the elements of cuboid_TS, 12 logarithms and 6 arctangents without quotients.
 __device__ __forceinline__ V3<double> cuboid_J(V3<double> q, V3<double> hd, V3<double> J, const Guard &g)
 {
-  double x0 = -q.x - hd.x, x1 = -q.x + hd.x, y0 = -q.y - hd.y, y1 = -q.y + hd.y, z0 = -q.z - hd.z, z1 = -q.z + hd.z;
+  // the signs of the widths, if negative, turn the field (cuboid_TS)
+  const int ws = hi32(hd.x) ^ hi32(hd.y) ^ hi32(hd.z);
+  const double hx = fabs(hd.x), hy = fabs(hd.y), hz = fabs(hd.z);
+  double x0 = -q.x - hx, x1 = -q.x + hx, y0 = -q.y - hy, y1 = -q.y + hy, z0 = -q.z - hz, z1 = -q.z + hz;
   int nan = 0;
-  if (x0 == 0. || x1 == 0.) { const double r = abs_rand(g, hd.x); if (x0 == 0.) x0 = r; if (x1 == 0.) x1 = r; nan |= r == 0.; }
-  if (y0 == 0. || y1 == 0.) { const double r = abs_rand(g, hd.y); if (y0 == 0.) y0 = r; if (y1 == 0.) y1 = r; nan |= (r == 0.) << 1; }
-  if (z0 == 0. || z1 == 0.) { const double r = abs_rand(g, hd.z); if (z0 == 0.) z0 = r; if (z1 == 0.) z1 = r; nan |= (r == 0.) << 2; }
+  if (x0 == 0. || x1 == 0.) { const double r = abs_rand(g, hx); if (x0 == 0.) x0 = r; if (x1 == 0.) x1 = r; nan |= r == 0.; }
+  if (y0 == 0. || y1 == 0.) { const double r = abs_rand(g, hy); if (y0 == 0.) y0 = r; if (y1 == 0.) y1 = r; nan |= (r == 0.) << 1; }
+  if (z0 == 0. || z1 == 0.) { const double r = abs_rand(g, hz); if (z0 == 0.) z0 = r; if (z1 == 0.) z1 = r; nan |= (r == 0.) << 2; }
   const bool mx = (hi32(x0) & ~hi32(x1)) < 0, my = (hi32(y0) & ~hi32(y1)) < 0, mz = (hi32(z0) & ~hi32(z1)) < 0;
   const bool nx = hi32(x0) < 0, ny = hi32(y0) < 0, nz = hi32(z0) < 0;
   const double xx0 = x0 * x0, xx1 = x1 * x1, yy0 = y0 * y0, yy1 = y1 * y1, zz0 = z0 * z0, zz1 = z1 * z1;
@@ -279,7 +282,7 @@ __device__ __forceinline__ V3<double> cuboid_J(V3<double> q, V3<double> hd, V3<d
     if (nan & 2) bv.y = bad;
     if (nan & 4) bv.z = bad;
   }
-  const double c = 0.0001;
+  const double c = flip_sign(0.0001, ws);
   return mk3<double>(c * (J.y * bv.z - J.z * bv.y), c * (J.z * bv.x - J.x * bv.z), c * (J.x * bv.y - J.y * bv.x));
 }
 

@@ -73,3 +73,28 @@ def test_collapsed_faces(cuda, rad, guards, ends):
     row = np.array(rad.FldPtcTrj(obj, 0.05, init, [-5, 5.3], 7))
     exp = trajectory(lambda q: O.field(b, q[None], 0)[0], 0.05, init, -5, 5.3, 7)
     assert np.abs(row - exp).max() <= 1e-12
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("current", [False, True])
+@pytest.mark.parametrize("sign", [(-1, 1, 1), (1, -1, 1), (1, 1, -1), (-1, -1, 1), (-1, 1, -1), (-1, -1, -1)])
+def test_negative_widths(cuda, rad, guards, sign, current):
+    """The C-ABI takes cuboids of negative width: each turns the field's sign,
+    as in the reference's formulas, outside and inside.  A current block
+    against the positive one to the bit; against the oracle to the rounding of
+    its corner terms (some 10 ulp of terms up to 4 pi |M|, and of 1e-4 times
+    lengths of some 10)."""
+    make = rad.ObjRecCur if current else rad.ObjRecMag
+    a = _arrays(rad, make([0.1, -0.2, 0.3], [4.0, 6.0, 8.0], [0.3, -0.7, 1.1]))
+    b = {k: v.copy() for k, v in a.items()}
+    b["rec"][0, 3:6] *= sign
+    rng = np.random.default_rng(8)
+    P = np.concatenate([rng.uniform(-9, 9, size=(60, 3)), rng.uniform(-1.5, 1.5, size=(10, 3))])
+    s = np.prod(sign)
+    for what in (0, 1):
+        got, exp = _native.field(b, P, what), O.field(b, P, what)
+        if current:
+            assert np.array_equal(got, s * _native.field(a, P, what))
+        bound = 1e-14 if current else 1e-13
+        assert np.abs(got - exp).max() <= bound
+        assert np.abs(_noalloc(cuda, b, P, what) - exp).max() <= bound

@@ -260,9 +260,10 @@ int launch_tri_records(const GeomView &g, int n_poly, double *tri, cudaStream_t 
 // vertices) and waits on it: FP64 pipe 25% busy, 6e7 tetrahedron pairs in 8.4
 // ms.  Here a block stages the records of up to TRI_TILE faces of up to 16
 // units in shared memory: FP64 pipe 62% busy, 3.7 ms (1.6e10 pairs/s); the
-// reference's polygon formula took 28 ms.
+// reference's polygon formula took 28 ms.  5 CTAs per SM: without the bound the
+// rarely called poly_special would set the kernel's registers (158; 6% slower).
 constexpr int TRI_UNITS = 16;
-__global__ void __launch_bounds__(128) field_tri_kernel(GeomView g, const double *__restrict__ pts, int64_t npts, int what,
+__global__ void __launch_bounds__(128, 5) field_tri_kernel(GeomView g, const double *__restrict__ pts, int64_t npts, int what,
                                                         double *__restrict__ out, int ub, int ue, int chunk, int accumulate)
 {
   __shared__ double sf[TRI_TILE * TRI_REC];
@@ -317,19 +318,38 @@ __global__ void __launch_bounds__(128) field_tri_kernel(GeomView g, const double
                      : __ldg(g.poly + (size_t)s_unit[k] * RADB200_POLY_STRIDE + 3 + (f - 21));
     }
     __syncthreads();
-    for (int k = 0; k < nu; k++) {
-      const double *Tr = su + 24 * k, *F = Tr + 12, *M = Tr + 21;
+    unsigned special = 0;  // units whose short form has no value at this point
+    auto point = [&](const double *Tr) {
       const double dx = P.x - Tr[9], dy = P.y - Tr[10], dz = P.z - Tr[11];
-      const V3<double> q = mk3<double>(Tr[0] * dx + Tr[1] * dy + Tr[2] * dz, Tr[3] * dx + Tr[4] * dy + Tr[5] * dz,
-                                       Tr[6] * dx + Tr[7] * dy + Tr[8] * dz);
+      return mk3<double>(Tr[0] * dx + Tr[1] * dy + Tr[2] * dz, Tr[3] * dx + Tr[4] * dy + Tr[5] * dz,
+                         Tr[6] * dx + Tr[7] * dy + Tr[8] * dz);
+    };
+    auto add = [&](const double *F, double hx, double hy, double hz) {
+      acc[0] += F[0] * hx + F[1] * hy + F[2] * hz;
+      acc[1] += F[3] * hx + F[4] * hy + F[5] * hz;
+      acc[2] += F[6] * hx + F[7] * hy + F[8] * hz;
+    };
+    for (int k = 0; k < nu; k++) {
+      const double *Tr = su + 24 * k, *M = Tr + 21;
+      const V3<double> q = point(Tr);
       double h[3] = {0, 0, 0};
       int inside = 1;
       for (int f = s_end[k]; f < s_end[k + 1]; f++) inside &= tri_face(sf + f * TRI_REC, q, h);
       if (what == 2) h[0] = h[1] = h[2] = 0.0;
+      if (not_finite(h[0])) {
+        special |= 1u << k;
+        continue;
+      }
       if (what != 1 && inside) { h[0] += M[0]; h[1] += M[1]; h[2] += M[2]; }
-      acc[0] += F[0] * h[0] + F[1] * h[1] + F[2] * h[2];
-      acc[1] += F[3] * h[0] + F[4] * h[1] + F[5] * h[2];
-      acc[2] += F[6] * h[0] + F[7] * h[1] + F[8] * h[2];
+      add(Tr + 12, h[0], h[1], h[2]);
+    }
+    for (; special; special &= special - 1) {
+      const int k = __ffs(special) - 1;
+      const double *Tr = su + 24 * k, *M = Tr + 21;
+      PolygonTerms t = poly_special(g.face, g.face_vtx, g.vtx2d, s_face[k], s_end[k + 1] - s_end[k],
+                                    mk3<double>(M[0], M[1], M[2]), point(Tr), g.g);
+      if (what == 0 && t.in) { t.x += M[0]; t.y += M[1]; t.z += M[2]; }
+      add(Tr + 12, t.x, t.y, t.z);
     }
     base += nu;
   }

@@ -419,17 +419,47 @@ __device__ __forceinline__ double half_solid_angle(double z, double zz, double a
   return atan2_64(z * a2, fma(fma(R0, R1, d01), R2, fma(d02, R1, d12 * R0)));
 }
 
+// polygon_S_terms as a call, for the points where the short form has no value
+// or not the reference's: S (3) and the inner-side flag
+struct PolygonTerms {
+  double x, y, z;
+  int in;
+};
+__device__ __noinline__ static PolygonTerms polygon_special(const double *vtx, int nv, double coordz, V3<double> P, Guard g)
+{
+  double cx = 0, cy = 0;
+  for (int k = 0; k < nv; k++) { cx += vtx[2 * k]; cy += vtx[2 * k + 1]; }
+  PolygonTerms t;
+  t.in = polygon_S_terms<double, double>(vtx, nv, coordz, cx / nv, cy / nv, P, g, t.x, t.y, t.z);
+  return t;
+}
+// D of an edge's ends (edge_D64), NaN for a point within twice the guard's step
+// of the edge or an end (without guards, on it): there the integrals are what
+// the reference's own steps leave of infinite ones
+__device__ __noinline__ static double edge_D64_off(double ax, double ay, double az, double Ra, double bx, double by, double bz,
+                                                   double Rb, double l, double step)
+{
+  const double cx = ay * bz - az * by, cy = az * bx - ax * bz, cz = ax * by - ay * bx, r = 2.0 * step;
+  if (fmin(Ra, Rb) <= r || cx * cx + cy * cy + cz * cz <= (r * l) * (r * l)) return __longlong_as_double(0x7ff8000000000000LL);
+  return edge_D64(ax, ay, az, Ra, bx, by, bz, Rb);
+}
+RB_HD bool not_finite(double x) { return (hi32(x) & 0x7ff00000) == 0x7ff00000; }
+
 // vtx: nv counter-clockwise vertices in the face frame; er: their edge records
-// (null: formed here); z == 0 steps off the plane by the length guard.
-// Returns 1 when the point is on the inner side of the face plane (z > 0).
+// (null: formed here).  A point with z == 0 steps off the plane by the length
+// guard; without guards it is on the outer side (-0: the solid angle's limit
+// from there, which the flag and the M path agree with).  Boundary points, and
+// distances whose squares overflow, take the reference's terms.
 __device__ __forceinline__ int polygon_S(const double *vtx, const double *er, int nv, double coordz, V3<double> P,
                                          const Guard &g, double &Sx, double &Sy, double &Sz)
 {
   double z = coordz - P.z;
-  if (z == 0.0 && (g.absr != 0.0 || g.relr != 0.0 || g.zeror != 0.0)) {
+  double step = 0.0;
+  if (z == 0.0) {
     double cx = 0, cy = 0;
     for (int k = 0; k < nv; k++) { cx += vtx[2 * k]; cy += vtx[2 * k + 1]; }
-    z = fmax(abs_rand(g, coordz), fmax(abs_rand(g, vtx[0] - cx / nv), abs_rand(g, vtx[1] - cy / nv)));
+    step = fmax(abs_rand(g, coordz), fmax(abs_rand(g, vtx[0] - cx / nv), abs_rand(g, vtx[1] - cy / nv)));
+    z = step > 0.0 ? step : -0.0;
   }
   const double zz = z * z;
   auto edge = [&](int j, double *e) {
@@ -442,8 +472,14 @@ __device__ __forceinline__ int polygon_S(const double *vtx, const double *er, in
   auto edge_L = [&](double ax, double ay, double Ra, double bx, double by, double Rb, double l) {
     const double S = Ra + Rb;
     double L;
-    edge_logs64<1>(&S, &l, &L, [&](int) { return edge_D64(ax, ay, z, Ra, bx, by, z, Rb); });
+    edge_logs64<1>(&S, &l, &L, [&](int) { return edge_D64_off(ax, ay, z, Ra, bx, by, z, Rb, l, step); });
     return L;
+  };
+  auto finish = [&]() -> int {
+    if (!not_finite(Sx)) return z > 0.0;
+    const PolygonTerms t = polygon_special(vtx, nv, coordz, P, g);
+    Sx = t.x; Sy = t.y; Sz = t.z;
+    return t.in;
   };
   const double x0 = vtx[0] - P.x, y0 = vtx[1] - P.y, R0 = sqrt64(fma(x0, x0, fma(y0, y0, zz)));
   double e[EDGE_REC];
@@ -463,7 +499,7 @@ __device__ __forceinline__ int polygon_S(const double *vtx, const double *er, in
     Sx = fma(-e[1], L, Sx);
     Sy = fma(e[0], L, Sy);
     Sz = 2.0 * half_solid_angle(z, zz, e[3], x0, y0, R0, x1, y1, R1, x2, y2, R2);
-    return z > 0.0;
+    return finish();
   }
   double xp = x0, yp = y0, Rp = R0;
   Sx = Sy = Sz = 0.0;
@@ -481,7 +517,7 @@ __device__ __forceinline__ int polygon_S(const double *vtx, const double *er, in
     if (j > 0 && j + 1 < nv) Sz += 2.0 * half_solid_angle(z, zz, e[3], x0, y0, R0, xp, yp, Rp, xn, yn, Rn);
     xp = xn; yp = yn; Rp = Rn;
   }
-  return z > 0.0;
+  return finish();
 }
 
 // ---- triangle face in three dimensions -------------------------------------------
@@ -493,7 +529,9 @@ __device__ __forceinline__ int polygon_S(const double *vtx, const double *er, in
 // c = M.n / (4 pi) with the face form's pi, so that H += sum L c nu - half angle * 2 c n.
 constexpr int TRI_REC = 28;
 
-// adds the face's H to h; returns 1 when q is on the inner side
+// adds the face's H to h; returns 1 when q is on the inner side (polygon_S).
+// h[0] is not finite after a face at whose boundary points, or at whose
+// distance, only the reference's terms have a value: poly_special then.
 __device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double *h)
 {
   double x[3], y[3], z[3], R[3], S[3], L[3];
@@ -501,7 +539,8 @@ __device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double 
   for (int k = 0; k < 3; k++) { x[k] = rec[3 * k] - q.x; y[k] = rec[3 * k + 1] - q.y; z[k] = rec[3 * k + 2] - q.z; }
   const double m0 = rec[12], m1 = rec[13], m2 = rec[14];
   double num = fma(x[0], m0, fma(y[0], m1, z[0] * m2));
-  if (num == 0.0 && rec[27] > 0.0) {  // on the plane, guards on
+  if (num == 0.0 && !(rec[27] > 0.0)) num = -0.0;
+  else if (num == 0.0) {  // on the plane, guards on
     const double mm = sqrt64(fma(m0, m0, fma(m1, m1, m2 * m2))), s = rec[27] / mm;
     for (int k = 0; k < 3; k++) { x[k] += s * m0; y[k] += s * m1; z[k] += s * m2; }
     num = rec[27] * mm;
@@ -511,7 +550,7 @@ __device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double 
   S[0] = R[0] + R[1]; S[1] = R[1] + R[2]; S[2] = R[2] + R[0];
   edge_logs64<3>(S, rec + 9, L, [&](int e) {
     const int b = e == 2 ? 0 : e + 1;
-    return edge_D64(x[e], y[e], z[e], R[e], x[b], y[b], z[b], R[b]);
+    return edge_D64_off(x[e], y[e], z[e], R[e], x[b], y[b], z[b], R[b], rec[9 + e], rec[27]);
   });
   const double d01 = fma(x[0], x[1], fma(y[0], y[1], z[0] * z[1])), d12 = fma(x[1], x[2], fma(y[1], y[2], z[1] * z[2])),
                d02 = fma(x[0], x[2], fma(y[0], y[2], z[0] * z[2]));
@@ -520,6 +559,28 @@ __device__ __forceinline__ int tri_face(const double *rec, V3<double> q, double 
   for (int c = 0; c < 3; c++)
     h[c] += fma(L[0], rec[18 + c], fma(L[1], rec[21 + c], fma(L[2], rec[24 + c], w * rec[15 + c])));
   return num > 0.0;
+}
+
+// H of a polyhedron by the reference's terms, faces [f0, f0 + nf); in: 1 when q
+// is on the inner side of all
+__device__ __noinline__ static PolygonTerms poly_special(const double *face, const int *face_vtx, const double *vtx2d, int f0,
+                                                         int nf, V3<double> M, V3<double> q, Guard g)
+{
+  // the reference's polygon face form uses this 15-digit pi (radplnr2.cpp:32)
+  const double CH = 1.0 / (4.0 * 3.14159265358979);
+  PolygonTerms h{0.0, 0.0, 0.0, 1};
+  for (int f = f0; f < f0 + nf; f++) {
+    const double *R = face + (size_t)f * RADB200_FACE_STRIDE;
+    const V3<double> pl = mk3<double>(R[0] * q.x + R[1] * q.y + R[2] * q.z, R[3] * q.x + R[4] * q.y + R[5] * q.z,
+                                      R[6] * q.x + R[7] * q.y + R[8] * q.z);
+    const PolygonTerms s = polygon_special(vtx2d + 2 * (size_t)face_vtx[2 * f], face_vtx[2 * f + 1], R[9], pl, g);
+    const double w = -CH * (R[6] * M.x + R[7] * M.y + R[8] * M.z);
+    h.x += w * (R[0] * s.x + R[3] * s.y + R[6] * s.z);
+    h.y += w * (R[1] * s.x + R[4] * s.y + R[7] * s.z);
+    h.z += w * (R[2] * s.x + R[5] * s.y + R[8] * s.z);
+    h.in &= s.in;
+  }
+  return h;
 }
 
 // Arc current field at q (object frame), record a = [cx cy cz rmin rmax

@@ -98,3 +98,65 @@ def test_negative_widths(cuda, rad, guards, sign, current):
         bound = 1e-14 if current else 1e-13
         assert np.abs(got - exp).max() <= bound
         assert np.abs(_noalloc(cuda, b, P, what) - exp).max() <= bound
+
+
+CUBE = np.array([[x, y, z] for z in (0, 1) for y in (0, 1) for x in (0, 1)], float)
+BODIES = {
+    # axis-aligned faces meet these points exactly, so that all forms see them there
+    "box": (CUBE, [[1, 3, 4, 2], [5, 6, 8, 7], [1, 2, 6, 5], [2, 4, 8, 6], [4, 3, 7, 8], [3, 1, 5, 7]]),
+    "box of triangles": (CUBE, [[1, 3, 4], [1, 4, 2], [5, 6, 8], [5, 8, 7], [1, 2, 6], [1, 6, 5], [2, 4, 8], [2, 8, 6],
+                                [4, 3, 7], [4, 7, 8], [3, 1, 5], [3, 5, 7]]),
+    "corner": (np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]]), [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]]),
+}
+
+
+def _axis_points(name):
+    """Points of the body's faces in the coordinate planes: boundary (corners
+    and edges), interior, and the outward normal of each interior one."""
+    t = [0.25, 0.5, 0.375]
+    edge = [[0, 0, 0]] + [[a, 0, 0] for a in t] + [[0, a, 0] for a in t] + [[0, 0, a] for a in t]
+    face = [[0.25, 0.375, 0], [0.375, 0, 0.25], [0, 0.25, 0.375], [0.5, 0.125, 0]]
+    out = [[0, 0, -1], [0, -1, 0], [-1, 0, 0], [0, 0, -1]]
+    if name != "corner":
+        edge += [[1, 0, 0], [0, 1, 0], [0, 0, 1], [1, 1, 1], [1, 0, 1], [1, 1, 0.25], [0.375, 1, 1]]
+        face += [[1, 0.25, 0.625], [0.25, 0.625, 1], [0.25, 1, 0.625]]
+        out += [[1, 0, 0], [0, 0, 1], [0, 1, 0]]
+    return np.array(edge, float), np.array(face, float), np.array(out, float)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(BODIES))
+def test_points_on_polyhedra(cuda, rad, guards, name):
+    """With guards the reference's values, also on edges and corners, where they
+    are what its steps leave of infinite ones; next to an edge its terms lose
+    half of the digits: 1e-6.  Without guards a point of a face is on its outer
+    side, in B, H and M (the reference's angles cancel there: off by up to |M|,
+    and even outside the body in a face's plane), and edges and corners are
+    finite, as in the reference.  As one polyhedron and among others (17 units:
+    more than one tile), and by the no-alloc entry."""
+    V, F = BODIES[name]
+    one = rad.ObjPolyhdr(V, F, [0.3, -0.7, 1.1])
+    more = rad.ObjCnt([rad.ObjPolyhdr(V + [3.0 * k, 5.0, 7.0], F, [0.1, 0.2, 0.3]) for k in range(16)] +
+                      [rad.ObjPolyhdr(V, F, [0.3, -0.7, 1.1])])
+    edge, face, out = _axis_points(name)
+    for obj in (one, more):
+        arrs = _arrays(rad, obj)
+        for what in (0, 1, 2):
+            for run in (lambda P: _native.field(arrs, P, what), lambda P: _noalloc(cuda, arrs, P, what),
+                        lambda P: _native.field(arrs, np.tile(P, (30, 1)), what)[-len(P):]):
+                if guards == "on":
+                    for P in (edge, face):
+                        exp = O.field(arrs, P, what)
+                        assert np.all(np.abs(run(P) - exp) <= 1e-6 * np.abs(exp).max(axis=1, keepdims=True) + 1e-9)
+                else:
+                    assert np.all(np.isfinite(run(edge)))
+                    # 1e-9 off the plane the field has changed by 1e-9 of |M| / distance to an edge
+                    near = run(face + 1e-9 * out)
+                    assert np.abs(run(face) - near).max() <= 1e-7
+                    assert what != 2 or np.all(run(face) == 0.0)
+                    plane = np.array([[1.75, 0.3125, 0], [-0.5, 0.625, 0], [0, 1.375, 0.8125]])
+                    assert np.abs(run(plane) - run(plane + 1e-9)).max() <= 1e-7
+    # squares of these distances overflow
+    for scale in (1e155, 1e160, 1e200):
+        far = scale * np.array([[1.0, -0.4, 0.3]])
+        assert np.array_equal(_native.field(_arrays(rad, one), far, 1), np.zeros((1, 3)))

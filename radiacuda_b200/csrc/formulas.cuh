@@ -583,6 +583,23 @@ __device__ __noinline__ static PolygonTerms poly_special(const double *face, con
   return h;
 }
 
+// u + D of two legs of D, other legs' squares q; direct when D was raised to the
+// reference's least value (then q / (|u| + D) is another number)
+__device__ __forceinline__ double arc_sum(double u, double D, double q, bool raised)
+{
+  return u < 0.0 && !raised ? q / (fabs(u) + D) : u + D;
+}
+// The logarithms that take D11 and D21 (arc_node) within 1e-5 of the arc's lower
+// inner or outer corner edge, where the reference raises these to 1e-5
+__device__ __noinline__ static double2 arc_corner_logs(double r1, double r2, double z1, double z2, double h1, double h2, double zz1,
+                                                       double D11, double D12, double D21, double D22, double least)
+{
+  const bool c1 = h1 + z1 * z1 < least, c2 = h2 + z1 * z1 < least;
+  return make_double2(log(arc_sum(r1, D11, zz1, c1) / arc_sum(r2, D21, zz1, c2)),
+                      log(arc_sum(z1, D11, h1, c1) / arc_sum(z2, D12, h1, false)) -
+                          log(arc_sum(z1, D21, h2, c2) / arc_sum(z2, D22, h2, false)));
+}
+
 // Arc current field at q (object frame), record a = [cx cy cz rmin rmax
 // phimin phimax h j nseg]; trapezoid rule in phi with nseg sectors
 // (radTArcCur::B_compWithTrapeth, radarccu.cpp:30-236).
@@ -612,9 +629,14 @@ __device__ __forceinline__ V3<double> arc_node(const double *a, V3<double> P, in
   const double D21 = sqrt64(fmax(h2 + z1z1, ZeroTol)), D22 = sqrt64(fmax(h2 + z2z2, 1e-290));
   const double b1 = fabs(r1), b2 = fabs(r2), c1 = fabs(z1), c2 = fabs(z2);
   const bool mr = r1 < 0.0 && r2 > 0.0, nr = r1 < 0.0, mz = z1 < 0.0 && z2 > 0.0, nz = z1 < 0.0;
-  const double ln1 = cuboid_edge_L(b1 + D11, b2 + D21, zz1, mr, nr);   // log((r1 + D11) / (r2 + D21))
+  double ln1 = cuboid_edge_L(b1 + D11, b2 + D21, zz1, mr, nr);         // log((r1 + D11) / (r2 + D21))
   const double ln2 = -cuboid_edge_L(b1 + D12, b2 + D22, zz2, mr, nr);  // log((r2 + D22) / (r1 + D12))
-  const double lz = cuboid_edge_L(c1 + D11, c2 + D12, h1, mz, nz) - cuboid_edge_L(c1 + D21, c2 + D22, h2, mz, nz);
+  double lz = cuboid_edge_L(c1 + D11, c2 + D12, h1, mz, nz) - cuboid_edge_L(c1 + D21, c2 + D22, h2, mz, nz);
+  if (fmin(h1, h2) + z1z1 < ZeroTol) {
+    const double2 t = arc_corner_logs(r1, r2, z1, z2, h1, h2, zz1, D11, D12, D21, D22, ZeroTol);
+    ln1 = t.x;
+    lz = t.y;
+  }
   // arctan(z2 |r1| / (rs D12)) - arctan(z1 |r1| / (rs D11)), and the outer radius with the sign turned
   const double e1 = rs * D12, g1 = z2 * b1, e2 = rs * D11, g2 = z1 * b1;
   const double at1 = angle64(fma(g1, e2, -(e1 * g2)), fma(e1, e2, g1 * g2), 0);

@@ -160,3 +160,30 @@ def test_points_on_polyhedra(cuda, rad, guards, name):
     for scale in (1e155, 1e160, 1e200):
         far = scale * np.array([[1.0, -0.4, 0.3]])
         assert np.array_equal(_native.field(_arrays(rad, one), far, 1), np.zeros((1, 3)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("off", [0.0, 3e-6, -3e-6, 2e-5])
+def test_points_on_an_arcs_corner_edges(cuda, rad, guards, off):
+    """At a node of the arc's trapezoid rule the distances to its lower corner
+    edges are not below 1e-5 in the reference; its logarithms are of the
+    distances so raised.  (The upper ones it leaves as they come out of a
+    cancellation, so no value there is compared.)  The oracle forms the squared
+    distances by the law of cosines, 1e-15 of 1e-10: 1e-5 of a distance, in a
+    logarithm of some 12 half of them; elsewhere some ulp."""
+    arrs = _arrays(rad, rad.ObjArcCur([0, 0, 0], [2.0, 5.0], [0.0, 1.5], 3.0, 6, 1.7, "man", "z"))
+    phi = np.arange(7) * 0.25
+    P = np.array([[(r + off) * np.cos(f), (r + off) * np.sin(f), -1.5 + s * off] for r in (2.0, 5.0) for f in phi for s in (0, 1)])
+    exp = O.field(arrs, P, 0)
+    has = np.all(np.isfinite(exp), axis=1)   # just outside 1e-5 its sums u + D may cancel to zero
+    assert has.sum() >= 14
+    for got in (_native.field(arrs, P, 0), _noalloc(cuda, arrs, P, 0)):
+        assert np.all(np.isfinite(got))
+        assert np.abs(got - exp)[has].max() <= 1e-5 * np.abs(exp[has]).max()
+    if not has[2]:
+        return
+    init = np.array([P[2, 0], 1e-3, P[2, 2], -1e-3])   # a trajectory that starts there
+    row = np.array(rad.FldPtcTrj(rad.ObjArcCur([0, 0, 0], [2.0, 5.0], [0.0, 1.5], 3.0, 6, 1.7, "man", "z"), 0.05, init,
+                                 [P[2, 1], P[2, 1] + 1.0], 3))
+    ref = trajectory(lambda q: O.field(arrs, q[None], 0)[0], 0.05, init, P[2, 1], P[2, 1] + 1.0, 3)
+    assert np.abs(row - ref).max() <= 1e-5 * np.abs(exp[has]).max()

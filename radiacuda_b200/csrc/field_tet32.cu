@@ -347,7 +347,8 @@ int launch_tet32_field(const GeomView &g, const double *d_pts, int64_t npts, int
   const int nu = ue - ub;
   DBuf rec;
   RB_TRY(rec.alloc((size_t)nu * T32_REC));
-  tet32_record_kernel<<<std::min((nu * (T32_D + T32_F) + 255) / 256, 148 * 8), 256, 0, st>>>(g, ub, nu, rec.as<unsigned char>());
+  const int rblk = (int)std::min<int64_t>(((int64_t)nu * (T32_D + T32_F) + 255) / 256, 148 * 8);
+  tet32_record_kernel<<<rblk, 256, 0, st>>>(g, ub, nu, rec.as<unsigned char>());
   RB_TRY(check_launch("tet32_record_kernel"));
   // too few points for the GPU: split the tetrahedra as well
   const int64_t target = 148 * 8;

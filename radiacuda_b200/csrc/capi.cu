@@ -459,6 +459,7 @@ static void build_topo_range(const RadB200Geom *G, bool tensor, int pa, int pb, 
       }
       for (int j = 0; j < m; j++) {
         int a = L[j], b = L[(j + 1) % m];
+        if (a == b) continue;  // a collapsed face: no edge there
         int lo = std::min(a, b), hi = std::max(a, b);
         int ei = -1;
         for (size_t q = 0; q < edges.size(); q++)

@@ -76,6 +76,27 @@ def test_collapsed_faces(cuda, rad, guards, ends):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ends", [([1, 3, 3, 2], [4, 5, 6, 6]), ([1, 3, 2, 1], [4, 5, 5, 6])])
+def test_collapsed_faces_by_vertices_and_edges(cuda, rad, guards, ends):
+    """The vertex/edge form of the same wedge: its terms are the plain one's, so
+    FP64 agrees to rounding and FP32 terms to 8 units of 2^-24 of terms of
+    order |M|; the interaction assembled in that form too."""
+    mat = rad.MatLin([3.0, 3.0], [0.0, 0.0, 0.7])
+    plain, obj = (rad.ObjPolyhdr(PRISM, e + SIDES, [0.4, -0.6, 0.9]) for e in ([[1, 3, 2], [4, 5, 6]], list(ends)))
+    P = np.random.default_rng(6).uniform(1.5, 4, size=(50, 3))
+    for precision, tol in (("fast", 1e-14), ("single", 8 * 2.0 ** -24)):
+        assert np.abs(rad.Fld(obj, "b", P, precision=precision) - rad.Fld(plain, "b", P, precision=precision)).max() <= tol
+    M = []
+    for body in (plain, obj):
+        h = rad.ObjCnt([body, rad.ObjBckg([0.1, 0.2, 0.3])])
+        rad.MatApl(body, mat)
+        im = rad.RlxPre(h, fast=True)
+        rad.RlxAuto(im, 1e-12, 200, 4)
+        M.append(np.array(rad.ObjM(body)).ravel()[-3:])
+    assert np.abs(M[0] - M[1]).max() <= 1e-7 and np.abs(M[0]).max() > 0.1   # the matrix is held in FP32
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("current", [False, True])
 @pytest.mark.parametrize("sign", [(-1, 1, 1), (1, -1, 1), (1, 1, -1), (-1, -1, 1), (-1, 1, -1), (-1, -1, -1)])
 def test_negative_widths(cuda, rad, guards, sign, current):

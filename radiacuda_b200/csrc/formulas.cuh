@@ -24,8 +24,6 @@ struct Guard { double absr, relr, zeror; };
 template <typename T> __device__ __forceinline__ T fabsT(T x) { return x < T(0) ? -x : x; }
 __device__ __forceinline__ double logT(double x) { return log(x); }
 __device__ __forceinline__ float logT(float x) { return logf(x); }
-__device__ __forceinline__ double atanT(double x) { return atan(x); }
-__device__ __forceinline__ float atanT(float x) { return atanf(x); }
 __device__ __forceinline__ double atan2T(double y, double x) { return atan2(y, x); }
 __device__ __forceinline__ float atan2T(float y, float x) { return atan2f(y, x); }
 __device__ __forceinline__ double sqrtT(double x) { return sqrt(x); }
@@ -38,15 +36,6 @@ template <typename T> __device__ __forceinline__ T abs_rand(const Guard &g, T A)
   T fromrel = T(g.relr) * A;
   T amax = (fromrel < T(g.absr)) ? T(g.absr) : fromrel;
   return (A != T(0)) ? amax : ((amax < T(g.zeror)) ? T(g.zeror) : amax);
-}
-
-// radTg3d::TransAtans (radg3d.h:938-946)
-template <typename T> __device__ __forceinline__ T trans_atans(T x, T y, T &pimult)
-{
-  T buf = T(1) - x * y;
-  if (buf == T(0)) buf = sizeof(T) == 8 ? T(1e-50) : T(1e-30);
-  pimult = ((buf > T(0)) ? T(0) : T(1)) * ((x < T(0)) ? T(-1) : T(1));
-  return (x + y) / buf;
 }
 
 // ---- cuboid -------------------------------------------------------------------

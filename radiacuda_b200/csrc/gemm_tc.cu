@@ -387,8 +387,8 @@ constexpr int TM_THREADS = 320;  // warps 0-7: epilogue; warp 8: TMA loads; warp
 // engine (one rounding, as before).  Holding all 4 slices ahead spilled (1.8
 // ms).  The TMA and MMA lanes are two because the divisions and waits of one
 // lane doing both were serial with every chunk.
-// F16: the operands are FP16 copies scaled by powers of two (*scale holds
-// 1 / (sA sB), applied to the accumulator in the epilogue): kind::f16 MMAs of
+// F16: the operands are FP16 copies scaled by powers of two (row_scale and
+// col_scale hold their inverses, applied in the epilogue): kind::f16 MMAs of
 // K = 16 (32 bytes of a 128-byte row, as the TF32 K = 8 step), 64 elements
 // per stage row instead of 32, so a stage feeds twice the flops.
 template <bool F16>

@@ -13,6 +13,7 @@ import numpy as np
 import pytest
 
 import oracle.oracle as O
+from oracle.trajectory_oracle import trajectory
 from radiacuda_b200 import _native, model
 
 LD = np.longdouble
@@ -266,9 +267,35 @@ def test_trajectories_do_not_depend_on_their_number(cuda, rad, n):
     obj = rad.ObjCnt([yoke, tet, rad.ObjRaceTrk([0.1, 0.2, 30.3], [2, 22], [60, 80], 30, 6, 15.0, "man", "z")])
     init = rng.uniform([-3, -2e-3, -3, -2e-3], [3, 2e-3, 3, 2e-3], size=(n, 4))
     batch = rad.FldPtcTrj(obj, 0.3, init, [-60, 59.5], 12)
+    arrs = model.pack_sources(rad._objs, obj, tuple(rad._rand))
     for k in (0, n - 1):
         assert np.array_equal(batch[k], np.array(rad.FldPtcTrj(obj, 0.3, init[k], [-60, 59.5], 12)))
-    # the same field as the field kernels', through one slope
-    P = np.array([init[0, 0], -60.0, init[0, 2]])
-    assert np.abs(np.array(rad.Fld(obj, "b", P.tolist())) - O.field(model.pack_sources(rad._objs, obj, tuple(rad._rand)),
-                                                                   P[None], 0)[0]).max() < 1e-10
+        # and the rows that the integrator makes of the oracle's field (B to 1e-10
+        # of its scale, over 120 mm at 1e-3 / (T mm) of curvature)
+        exp = trajectory(lambda q: O.field(arrs, q[None], 0)[0], 0.3, init[k], -60, 59.5, 12)
+        assert np.abs(batch[k] - exp).max() <= 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 37])
+def test_trajectory_items_two_to_a_lane(cuda, rad, n):
+    """Arcs of 6,000 nodes, current blocks, cuboids with images and a
+    polyhedron: more than 32 * 512 work items, so that lanes take several."""
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    rng = np.random.default_rng(2)
+    coils = [rad.ObjArcCur([0.3 * k, 0.1, 25.0 + 9 * k], [3.0, 20.0], [0.2, 0.2 + 1.1 * (k + 1)], 7.0, 6000, 12.0, "man", "z")
+             for k in range(3)]
+    blocks = rad.ObjCnt([rad.ObjRecMag([4.0 * i - 20, 0.3, -22.0 - i], [3.0, 30.0, 5.0], rng.normal(size=3).tolist())
+                         for i in range(11)])
+    rad.TrfZerPara(blocks, [0, 0, 0], [0, 0, 1])
+    rest = [rad.ObjRecCur([30.2, 0.4, 18.3], [4.0, 40.0, 6.0], [0.0, 9.0, 0.0]),
+            rad.ObjPolyhdr([[70, 0, 5], [75, 1, 5], [71, 6, 5], [72, 2, 11]], [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]],
+                           [0.2, 0.3, 0.9]), rad.ObjBckg([0.01, -0.02, 0.03])]
+    obj = rad.ObjCnt(coils + [blocks] + rest)
+    arrs = model.pack_sources(rad._objs, obj, tuple(rad._rand))
+    init = rng.uniform([-3, -2e-3, -3, -2e-3], [3, 2e-3, 3, 2e-3], size=(n, 4))
+    got = np.asarray(rad.FldPtcTrj(obj, 0.3, init, [-60, 59.5], 6))
+    for k in (0, n - 1):
+        exp = trajectory(lambda q: O.field(arrs, q[None], 0)[0], 0.3, init[k], -60, 59.5, 6)
+        assert np.abs(got[k] - exp).max() <= 1e-9

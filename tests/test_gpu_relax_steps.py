@@ -66,10 +66,39 @@ def test_saturating_methods_agree(cuda, rad, n):
 
 
 @pytest.mark.gpu
-def test_adjoint_gmres_restarts(cuda, rad):
-    """More Krylov vectors than one cycle holds: the restarted iteration still
-    reaches the tolerance on a strongly coupled system without a preconditioner
-    that would end it at once."""
+@pytest.mark.parametrize("restart", [1, 2, 3, 7, 20])
+@pytest.mark.parametrize("n", [86, 171])
+def test_gmres_restarts(cuda, rad, n, restart, monkeypatch):
+    """Newton's inner solves to 1e-10 of a strongly coupled linear system in
+    cycles of a few vectors (RADB200_NK): about 35 vectors each in one cycle of
+    200.  The same solution, with more products than one cycle takes, which
+    only restarts add."""
+    MD.reset(rad)
+    rng = np.random.default_rng(n)
+    hs = []
+    for k in range(n):
+        m = rng.normal(size=3).tolist()
+        hs.append(rad.ObjRecMag([2.1 * (k % 5), 2.1 * ((k // 5) % 5), 2.1 * (k // 25)], [2.0, 2.0, 2.0], m))
+        rad.MatApl(hs[-1], rad.MatLin([30.0, 18.0], m))
+    h = rad.ObjCnt(hs + [rad.ObjBckg([0.02, -0.01, 0.05])])
+    pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
+    exp = O.linear_direct(pack, O.assemble(pack), O.extfield(pack))
+    nat = _native.NativeInteraction(pack, 1)
+    products = {}
+    try:
+        for r in (200, restart):
+            monkeypatch.setenv("RADB200_NK", f"1e-10,0.01,{r},5000")
+            M, _, st = nat.relax(1, 1e-12, 20000, True, 1.0, np.zeros(3 * n))
+            products[r] = st[3]
+            assert st[0] <= 1e-12 and rel_err(M, exp) < 1e-11
+    finally:
+        nat.free()
+    assert products[restart] > products[200] > 40
+
+
+@pytest.mark.gpu
+def test_newton_on_a_strongly_coupled_mesh(cuda, rad):
+    """Tetrahedra of chi = 1000: several Newton steps of many vectors each."""
     h, body = MD.tet_mesh(rad, ncell=3, n_tets=100, chi=1000.0)
     pack = model.pack_interaction(rad._objs, h, 0, tuple(rad._rand))
     n = pack.elem_src.shape[0]

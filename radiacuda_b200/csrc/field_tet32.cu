@@ -4,15 +4,20 @@
 // FP64 and rounded to FP32; distances, edge integrals and solid angles in
 // FP32; weights and sums in FP64.  Bound by instruction issue: the library's
 // log1pf, atan2f, division and square root made 793 thread-instructions a
-// pair, this form 386 (8,000 tetrahedra, 1e6 points: 223 ms before, 126 ms).
+// pair, this form 377 (8,000 tetrahedra, 1e6 points: 223 ms before, 126 ms).
 // Most pairs are distant, and there each element is short:
 //   L / 2 = artanh(x),   x = l / (Ra + Rb) <= 1/6:    a quotient, 3 terms;
 //   half solid angle = arctan(num / den) <= 0.025:     a quotient, 2 terms,
 // when the point is at least 4 times the longest edge from vertex 0 (every
 // distance is then at least 3 of them).  The quotients' corrections, and what
-// rounding took from Ra + Rb, go into the last addition of each: 2-norm of B
-// against FP64 on 20,000 / 3,000 tetrahedra 1.9e-7 / 2.2e-7 (the library's form
-// 2.6e-7 / 2.3e-7; without these corrections 2.4e-7 / 2.5e-7 and 118 ms).
+// rounding took from Ra + Rb, go into the last addition of each.
+// In a smooth body the terms of an inner edge cancel among its tetrahedra, if
+// all take the same value for it.  So an edge distant by itself (Ra + Rb >= 6 l)
+// takes the distant form in every tetrahedron, also in those that are not.
+// 2-norm and largest error at a point of B against FP64, the body of chi = 1000
+// relaxed, 20,000 tetrahedra, 1e6 points: 3.2e-8, 6.2e-7 (the library's form
+// 4.0e-8, 7.6e-7; by whole tetrahedra, without this rule, 6.9e-8, 2.1e-6);
+// 3,000 tetrahedra 3.4e-8 (3.8e-8; 6.4e-8).
 // Nearer pairs take the log1pf and atan2f forms.  A warp pays for the longer
 // path when any of its lanes needs it, so larger point sets are first put in
 // Morton order; each point's sum runs over the tetrahedra in their own order
@@ -55,6 +60,17 @@ __device__ __forceinline__ float root32(float s)
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
   const float g = s * y;
   return fmaf(0.5f * y, fmaf(-g, g, s), g);
+}
+
+// half the edge integral, artanh(l / (Ra + Rb)), for Ra + Rb >= 6 l
+__device__ __forceinline__ float far_half_L(float ra, float rb, float l)
+{
+  const float s = ra + rb;
+  float c;  // ra and rb differ by less than a factor 2: (ra - s) + rb is exact
+  const float x = quot32(l, s, (ra - s) + rb, c), z = x * x;
+  // artanh(x) = x (1 + z p(z)), least maximum error 2.3e-9 for z <= 1/36
+  const float p = fmaf(fmaf(0.1477081972f, z, 0.1999480270f), z, 0.3333334154f);
+  return x + fmaf(x * z, p, c);
 }
 
 struct D3 {
@@ -110,14 +126,7 @@ __device__ __forceinline__ void tet32_pair(const double *__restrict__ sd, const 
 #pragma unroll
     for (int k = 0; k < 4; k++) R[k] = root32(R[k]);
 #pragma unroll
-    for (int e = 0; e < 6; e++) {
-      const float ra = R[tet_edge_a(e)], rb = R[tet_edge_b(e)], s = ra + rb;
-      float c;  // ra and rb differ by less than a factor 2: (ra - s) + rb is exact
-      const float x = quot32(sf[e], s, (ra - s) + rb, c), z = x * x;
-      // artanh(x) = x (1 + z p(z)), least maximum error 2.3e-9 for z <= 1/36
-      const float p = fmaf(fmaf(0.1477081972f, z, 0.1999480270f), z, 0.3333334154f);
-      edge_add(e, x + fmaf(x * z, p, c));
-    }
+    for (int e = 0; e < 6; e++) edge_add(e, far_half_L(R[tet_edge_a(e)], R[tet_edge_b(e)], sf[e]));
 #pragma unroll
     for (int f = 0; f < 4; f++) {
       const int a = tet_face_a(f), b = tet_face_b(f), c = tet_face_c(f);
@@ -129,12 +138,19 @@ __device__ __forceinline__ void tet32_pair(const double *__restrict__ sd, const 
       face_add(f, w + fmaf(w * u, fmaf(0.1998287159f, u, -0.3333333076f), cw));
     }
   } else {
+    float Q[4];  // the distances as the distant form takes them
 #pragma unroll
-    for (int k = 0; k < 4; k++) R[k] = sqrtf(R[k]);
+    for (int k = 0; k < 4; k++) {
+      Q[k] = root32(R[k]);
+      R[k] = sqrtf(R[k]);
+    }
 #pragma unroll
     for (int e = 0; e < 6; e++) {
       const int a = tet_edge_a(e), b = tet_edge_b(e);
-      edge_add(e, 0.5f * edge_L(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b], d[e], sf[e]));
+      const float l = sf[e];
+      // an edge distant by itself takes the form that it takes in every other tetrahedron
+      if (Q[a] + Q[b] >= 6.f * l) edge_add(e, far_half_L(Q[a], Q[b], l));
+      else edge_add(e, 0.5f * edge_L(rx[a], ry[a], rz[a], R[a], rx[b], ry[b], rz[b], R[b], d[e], l));
     }
     double total = 0.0;
 #pragma unroll

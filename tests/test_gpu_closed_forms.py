@@ -250,6 +250,36 @@ def test_tetrahedra_with_fp32_terms(cuda, rad, ntets, npts):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [4, 8, 12])
+def test_fp32_terms_cancel_inside_a_mesh(cuda, rad, n):
+    """A uniformly magnetized mesh of n^3 cubes of six tetrahedra: inner edges
+    and faces carry no field, and their terms cancel to the bit only if every
+    tetrahedron around an edge takes the same value for it, near and distant
+    ones.  What is left are the errors of the surface's 18 n^2 edges of length
+    1 at distances around n: each rounded to 2^-24 (2^-25 / 1.7 in the mean) of
+    L = 1 / n, with weights up to 1.4 |M| / (4 pi) and |M| = 1.34, twice that
+    with the distances' rounding: 4.2 * 2^-25 * 1.9 / (4 pi) * 0.58 = 1.1e-8,
+    whatever n is."""
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    rng = np.random.default_rng(0)
+    cube = [[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0], [0, 0, 1], [1, 0, 1], [1, 1, 1], [0, 1, 1]]
+    kuhn = [[0, 1, 2, 6], [0, 2, 3, 6], [0, 3, 7, 6], [0, 7, 4, 6], [0, 4, 5, 6], [0, 5, 1, 6]]
+    V = np.stack([a.ravel() for a in np.meshgrid(*[np.arange(n + 1.0)] * 3, indexing="ij")], 1)
+    V += rng.uniform(-0.02, 0.02, V.shape)
+    tets = []
+    for c in np.ndindex(n, n, n):
+        at = [((c[0] + a) * (n + 1) + c[1] + b) * (n + 1) + c[2] + d for a, b, d in cube]
+        tets += [rad.ObjPolyhdr(V[[at[i] for i in t]], [[1, 2, 3], [1, 4, 2], [2, 4, 3], [3, 4, 1]], [0.3, -0.7, 1.1])
+                 for t in kuhn]
+    obj = rad.ObjCnt(tets)
+    P = rng.uniform(-4, n + 4, size=(20000, 3))
+    P = np.ascontiguousarray(P[~np.all((P > -1) & (P < n + 1), axis=1)])
+    d = rad.Fld(obj, "b", P, precision="single") - rad.Fld(obj, "b", P, precision="fast")
+    assert np.sqrt((d * d).sum(axis=1).mean()) <= 1.1e-8
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [2, 18, 19, 37, 74, 149])
 def test_trajectories_do_not_depend_on_their_number(cuda, rad, n):
     """Clusters of 8, 4, 2 and 1 CTAs by the number of trajectories: the same

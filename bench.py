@@ -282,11 +282,11 @@ def run_ours(args, rank, world):
     upd_tflops = upd_f.value / max(upd_s.value, 1e-30) / 1e12
     upd_gbs = upd_b.value / max(upd_s.value, 1e-30) / 1e9
     upd_bytes_per_launch = upd_b.value / max(upd_n.value, 1)
-    roof_upd = {"kernel": ("tc_update_tma_kernel<FP16 operands> (LU trailing update A22 -= L21 U12, K = 1024, "
-                           "then 768 for the last 30,000 rows; operands scaled per row and column by powers of two, "
+    roof_upd = {"kernel": ("tc_update_tma_kernel<FP16 operands> (LU trailing update A22 -= L21 U12, K = 1536, "
+                           "then 768 for the last 20,000 rows; operands scaled per row and column by powers of two, "
                            "FP32 accumulation)" if f16_ops else
-                           "tc_update_tma_kernel<TF32 operands> (LU trailing update A22 -= L21 U12, K = 1024, "
-                           "then 768 for the last 30,000 rows)"),
+                           "tc_update_tma_kernel<TF32 operands> (LU trailing update A22 -= L21 U12, K = 1536, "
+                           "then 768 for the last 20,000 rows)"),
                 "bound": "tensor",
                 "achieved": round(upd_tflops, 1), "peak": round(tf32_peak, 1), "unit": "TFLOP/s",
                 "frac": round(upd_tflops / tf32_peak, 4),
@@ -296,7 +296,7 @@ def run_ours(args, rank, world):
                 "frac_of_burst": round(upd_tflops / (float(peaks.get("bf16_tflops", 1590.0)) / div), 4),
                 "hbm_achieved_gbs": round(upd_gbs, 1), "hbm_peak_gbs": hbm, "hbm_frac": round(upd_gbs / hbm, 4),
                 "traffic": round(TC_TRAFFIC_OVER_ALGORITHMIC["f16" if f16_ops else "tf32"] * upd_bytes_per_launch),
-                "traffic_note": "ncu dram bytes / algorithmic bytes (0.92) of the same kernel on a 9,000^2 LU, "
+                "traffic_note": "ncu dram bytes / algorithmic bytes (0.91; 0.93 with TF32 operands) of the same kernel on a 9,000^2 LU, "
                                 "times the algorithmic bytes per launch",
                 "launches_per_step": int(upd_n.value // max(args.steps, 1)),
                 "seconds_per_step": round(upd_s.value / max(args.steps, 1), 4),
@@ -594,7 +594,7 @@ def trajectory_timing(reps=3):
     relaxed iron dipole (about 360 saturating cuboids with 4 images each, a
     racetrack coil): one 0.3 GeV trajectory through the gap over +-200 mm at
     401 points (default fixed-step Runge-Kutta: 1,600 field evaluations in
-    sequence), and a batch of 1,024 trajectories (one CTA each).  Median wall
+    sequence), and a batch of 1,024 trajectories (one cluster each).  Median wall
     time of `reps` after one warm-up; the reference CPU module's FldPtcTrj on
     the same relaxed model beside it, with the largest difference."""
     import torch
@@ -636,9 +636,9 @@ def trajectory_timing(reps=3):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum over the algorithmic bytes of the
-# trailing-update kernel, from ncu captures of a 9,000^2 LU: 561 MB / 611 MB with
-# TF32 operands, 475 MB / 515.7 MB with FP16 operands
-TC_TRAFFIC_OVER_ALGORITHMIC = {"tf32": 0.92, "f16": 0.92}
+# trailing-update kernel, from ncu captures of a 9,000^2 LU: 504 MB / 539.8 MB with
+# TF32 operands, 469 MB / 515.7 MB with FP16 operands
+TC_TRAFFIC_OVER_ALGORITHMIC = {"tf32": 0.93, "f16": 0.91}
 
 
 # FP64 operations of one (point, tetrahedron) term of the vertex/edge form
@@ -651,10 +651,10 @@ FIELD_OPS_PER_TET = 4 * 16 + 6 * 5 + 6 * 40 + 4 * 51 + 3
 
 # Instructions the FP32 field kernel issues per (point, tetrahedron) pair,
 # from ncu's smsp__inst_executed.sum x 32 / pairs on 8,000 tetrahedra and 1e6
-# points (9.65e10 warp-instructions).  The kernel is issue-bound: its roofline
+# points (9.41e10 warp-instructions).  The kernel is issue-bound: its roofline
 # is the SMs' issue rate, 4 warp-instructions (128 thread-instructions) per
 # clock per SM, divided by these instructions per pair.
-FIELD_INST_PER_PAIR = 386
+FIELD_INST_PER_PAIR = 377
 B200_SMS = 148
 
 

@@ -86,7 +86,7 @@ RB_HD double sqrt64(double s)
   return fma(g * e, fma(0.375, e, 0.5), g);
 }
 
-// arctan(r) for |r| <= tan(pi/8): relative error of the polynomial 1.3e-18
+// arctan(r) for |r| <= tan(pi/8): relative error of the polynomial 4.5e-18
 RB_HD double atan_poly(double r)
 {
   const double z = r * r;
@@ -124,7 +124,7 @@ RB_HD double angle64(double y, double x, int turns)
 }
 
 // 2 artanh(s) = log((1 + s) / (1 - s)) for |s| <= 0.203: relative error of the
-// polynomial 1.8e-17
+// polynomial 3.6e-17
 RB_HD double artanh2_poly(double s)
 {
   const double z = s * s;

@@ -246,7 +246,8 @@ static double g_upd_bytes = 0.0, g_upd_flops = 0.0;
 // 1024, 1280 and 1536 columns), the main stream's panel chain the late ones.
 // Direct solve of the 60,000^2 system, ms: 1536 then 768 below 20,000 rows 394;
 // 1280 then 768 399; 1024 then 768 409 (below 30,000 rows 411); 1536 then 1024
-// 400; 1024 throughout 420.
+// 400; 1024 throughout 420.  The same rule on 45,000 / 37,500 / 30,000 rows: 157 /
+// 108 / 74 (1024 first: 162 / 109 / 74; 768 throughout: 166 / 111 / 74).
 constexpr int LU_WIDEST = 2048;  // of all panels
 constexpr int LU_OUTER_DEFAULT = 1536, LU_OUTER_LATE_DEFAULT = 768, LU_LATE_AT_DEFAULT = 20000;
 // the outer panel width: LU_OUTER_DEFAULT, or RADB200_LU_OUTER (a multiple of
@@ -286,8 +287,9 @@ static int lu_outer_at(int remaining)
 // updates.  Events order the two streams; nothing waits on the device.
 // Inside a panel the first 128 rows of an update go first (rows_first): the
 // next diagonal block and its U12 then run on a third stream of high priority
-// beside the update of the other rows (the diagonal block is one CTA for 97 us,
-// 45 ms of the main stream's chain over the 60,000^2 factorization; 14 left).
+// beside the update of the other rows (the diagonal block is one CTA for 80 us,
+// 97 with its launch: 45 ms of the main stream's chain over the 60,000^2
+// factorization; 14 left).
 constexpr int LU_SIDE_FREE_SMS = 12;  // 60,000^2 direct solve: 8 411, 12 409, 20 407 ms; 28 and 40 slower
 
 struct LuStreams {

@@ -1031,7 +1031,7 @@ def FldPtcTrj(obj: int, E: float, init, lims, np_: int):
     PrcAngle set positive (FldCmpCrt / FldCmpPrc) every interval is
     integrated with step-doubling control, else with one fourth-order
     Runge-Kutta step, as in the reference.  An extension: init given as an
-    [n, 4] array runs n trajectories at once (one CTA each) and returns an
+    [n, 4] array runs n trajectories at once (one cluster each) and returns an
     [n, np_, 5] array."""
     ini = np.asarray(init, dtype=np.float64)
     lim = np.asarray(lims, dtype=np.float64).reshape(-1)

@@ -5,6 +5,8 @@
     python tests/profile_cases.py lu       [--tets N] [--mode 0|1]
     python tests/profile_cases.py relax    [--blocks N]
     python tests/profile_cases.py adjoint  [--pairs N] [--points P]
+    python tests/profile_cases.py cuboids  [--blocks N] [--points P]   (field of an iron dipole of N cuboids, 4 images)
+    python tests/profile_cases.py trajectory [--blocks N]              (one, 101 points, in the same dipole)
 
 Each case builds a seeded model of the benchmark's shapes (tetrahedral mesh
 of chi = 1000 material, magnet array) at a size that keeps one launch of the
@@ -30,7 +32,7 @@ import models as MD  # noqa: E402
 
 def main(argv=None):
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["field", "assemble", "lu", "relax", "adjoint"])
+    ap.add_argument("case", choices=["field", "assemble", "lu", "relax", "adjoint", "cuboids", "trajectory"])
     ap.add_argument("--pairs", type=int, default=20)
     ap.add_argument("--tets", type=int, default=20000)
     ap.add_argument("--points", type=int, default=20000)
@@ -68,6 +70,18 @@ def main(argv=None):
         t0 = time.perf_counter()
         prob.backward(np.random.default_rng(1).normal(size=P.shape))
         print("adjoint", prob.n, "elements", P.shape[0], "points", time.perf_counter() - t0, "s", prob.last_timing)
+    elif a.case in ("cuboids", "trajectory"):
+        h = MD.iron_dipole(rad, n_target=a.blocks)
+        rng = np.random.default_rng(0)
+        for lf in model.collect_leaves(rad._objs, h):
+            if hasattr(lf.obj, "m"):
+                lf.obj.m = rng.normal(size=3)
+        t0 = time.perf_counter()
+        if a.case == "cuboids":
+            B = rad.Fld(h, "b", rng.uniform([-45, -1, -18], [45, 1, 18], size=(a.points, 3)))
+        else:
+            B = np.array(rad.FldPtcTrj(h, 0.3, [0.3, 0.0, 0.7, 0.0], [-120.0, 119.7], 101))
+        print(a.case, time.perf_counter() - t0, "s", float(np.abs(B).max()))
     else:
         h = MD.magnet_array(rad, nside=int(np.sqrt(a.blocks)), div=3)
         im = rad.RlxPre(h)

@@ -5,7 +5,7 @@ integration and with the step-doubling control.
 
 CPU tests pin the oracle's restatement of the integrator
 (oracle/trajectory_oracle.py) on the oracle field; GPU tests run the device
-kernel (one CTA per trajectory) through rad.FldPtcTrj.
+kernel (one cluster of CTAs per trajectory) through rad.FldPtcTrj.
 """
 import json
 import os
@@ -103,7 +103,7 @@ def test_fldptctrj_matches_reference(rad, cuda, name, mode):
 
 @pytest.mark.gpu
 def test_batched_trajectories_equal_single_ones(rad, cuda):
-    """An [n, 4] batch runs n CTAs; each row equals the single-trajectory call."""
+    """An [n, 4] batch runs n clusters; each row equals the single-trajectory call."""
     h = BUILDERS["array_given"](rad)
     rng = np.random.default_rng(5)
     init = np.column_stack([rng.uniform(-20, 0, 24), rng.normal(0, 1e-3, 24), rng.uniform(6.5, 9.5, 24),

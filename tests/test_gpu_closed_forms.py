@@ -20,6 +20,12 @@ LD = np.longdouble
 EPS = 2.0 ** -52
 
 
+@pytest.fixture(autouse=True)
+def fixed_steps(rad):
+    """One Runge-Kutta step per interval, whatever a test before left set."""
+    rad.FldCmpPrc("PrcCoord->-1,PrcAngle->-1")
+
+
 def _tensor(q, d):
     """[n, 3, 3] in long double; q = point - centre, d the full widths."""
     h = LD(0.5) * np.asarray(d, LD)
@@ -329,3 +335,30 @@ def test_trajectory_items_two_to_a_lane(cuda, rad, n):
     for k in (0, n - 1):
         exp = trajectory(lambda q: O.field(arrs, q[None], 0)[0], 0.3, init[k], -60, 59.5, 6)
         assert np.abs(got[k] - exp).max() <= 1e-9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_traj", [1, 18, 37, 74, 149])
+@pytest.mark.parametrize("n_src", [1, 257, 513, 1025, 16385])
+def test_cluster_exchange_with_cheap_sources(cuda, rad, n_src, n_traj):
+    """Clusters of 1 to 8 CTAs on sources that cost almost nothing (uniform
+    fields), so that a CTA's first sums go to its cluster's other CTAs right
+    after the launch; 16,385 sources put two items on a lane.  The field is a
+    sum of n_src numbers: B is off by at most n_src eps sum|b|, the angles by
+    that times length / momentum, the positions by the length once more; the
+    integrator's own rounding is 64 ulp of the rows."""
+    rad.UtiDelAll()
+    rad.FldLenRndSw("off")
+    rng = np.random.default_rng(n_src)
+    b = rng.uniform(0.2, 1.0, size=(n_src, 3)) * [0.3, 0.5, -0.4] / n_src
+    obj = rad.ObjCnt([rad.ObjBckg(v.tolist()) for v in b])
+    init = rng.uniform([-3, -2e-3, -3, -2e-3], [3, 2e-3, 3, 2e-3], size=(n_traj, 4))
+    energy, lims, npts = 0.3, (-10.0, 9.5), 5
+    got = np.asarray(rad.FldPtcTrj(obj, energy, init, list(lims), npts))
+    B = b.sum(axis=0)
+    ang = n_src * 2.0 ** -53 * np.abs(b).sum() * 2.99792458e5 / (1e9 * energy) * (lims[1] - lims[0])
+    for k in (0, n_traj - 1):
+        exp = trajectory(lambda P: B, energy, init[k], *lims, npts)
+        bound = np.array([0.0, ang * 20.0, ang, ang * 20.0, ang]) + 64 * 2.0 ** -52 * np.abs(exp).max(axis=0)
+        assert np.all(np.abs(got[k] - exp) <= bound)
+    rad.FldLenRndSw("on")

@@ -15,6 +15,12 @@ from test_zz_no_alloc import _device_geom
 EPS = 2.0 ** -52
 
 
+@pytest.fixture(autouse=True)
+def fixed_steps(rad):
+    """One Runge-Kutta step per interval, whatever a test before left set."""
+    rad.FldCmpPrc("PrcCoord->-1,PrcAngle->-1")
+
+
 def _noalloc(cuda, arrs, P, what):
     import torch
 
